@@ -30,6 +30,13 @@ int gbcc_testing_gemm(int64_t M, int64_t N, int64_t K, const double* A, const do
 int gbcc_testing_gemm_ex(int64_t M, int64_t N, int64_t K, const double* A, const double* B, double* C,
                          int slices, int ksplit, int bn, int cta2, int chunk, int fold, int repeat, float* ms);
 
+/* The in-place FP64 kernel of small contractions: C = beta C + alpha A B^T.
+ * mode bit 0: A stored [K][M], bit 1: B stored [K][N], bit 2: alpha = -0.5 and
+ * beta = 1 on the C given (else alpha = 1, beta = 0), bit 3: A read as two
+ * terms, 2 A - 0.75 A.  *ms: the mean time of `repeat` launches. */
+int gbcc_testing_gemm_small(int64_t M, int64_t N, int64_t K, const double* A, const double* B, double* C, int mode,
+                            int repeat, float* ms);
+
 /* The BF16 split the packing kernels apply: x[0..n) (host) -> out[s*n + i]
  * (host), the bit patterns of slices s = 0..nslices-1 (nslices 1..3). */
 int gbcc_testing_split(const double* x, int64_t n, int nslices, uint16_t* out);

@@ -562,6 +562,8 @@ void calibrate_slices(gbcc_handle* h, const double* t1_in, const double* t2_in) 
   for (int k = 0; k < 3; ++k) {
     if (req[k] != 0) continue;
     h->slice_err[k] = 0.0;
+    // (a class whose contractions all run in FP64 has nothing to choose)
+    if (!h->eng->class_on_tensor_cores(static_cast<gbcc::TermClass>(k))) continue;
     for (int s = 2; s >= 1; --s) {
       int lim[3] = {0, 0, 0};
       lim[k] = s;

@@ -226,12 +226,25 @@ struct OperandPlan {
   unsigned* rowexp = nullptr;
 };
 
+// The in-place FP64 kernel (gemm_small.cu) takes a contraction whose estimated
+// time is at most this many microseconds: in the FP64 plan, where the panel
+// GEMM needs two packs first (500^3: 230 us, the panel GEMM alone 347 us;
+// 741^3: 711 against 780 us; beyond that each operand is read too many times);
+// in the mixed plan, where a tensor-core launch costs 15-30 us and its packs
+// 5-10 us each however small the product; in the FP64_TC plan, with six
+// slices to pack.
+constexpr double kSmallUs = 800.0;
+constexpr double kSmallUsMixed = 20.0;
+constexpr double kSmallUsFixed = 80.0;
+
 // slice pairs of a plan: 3 slices give 6, the fixed-point split's 6 slices 21
 constexpr int kMaxPlanPairs = 36;
 
 struct GemmPlan {
   bool use_tc = false;
   bool smallk = false;     // mixed precision, K <= kSmallK: FP32 CUDA-core kernel on FP64 panels
+  bool small = false;      // FP64, operands read in place (gemm_small.cu)
+  GemmSmallArgs sg{};
   bool a_is_first = true;  // GEMM M side is the call's A operand
   int64_t M = 0, N = 0, K = 0;
   OperandPlan P[2];        // [0] = M side, [1] = N side
@@ -339,6 +352,12 @@ std::vector<SiteStat> Engine::site_stats(int precision) {
   return out;
 }
 
+bool Engine::class_on_tensor_cores(TermClass cls) const {
+  for (const auto& sp : sites_)
+    if (sp->kind == 1 && sp->cls == cls && sp->plan[1].use_tc) return true;
+  return false;
+}
+
 Engine::Engine() = default;
 
 Engine::~Engine() {
@@ -349,6 +368,7 @@ Engine::~Engine() {
   dev_free(wbfa_);
   dev_free(wbfb_);
   dev_free(wpart_);
+  dev_free(wcount_);
 }
 
 Tensor& Engine::tensor(const std::string& name, std::initializer_list<int64_t> dims, bool constant) {
@@ -402,8 +422,11 @@ void Engine::reset_plans() {
   sites_.clear();
   for (void* p : owned_) dev_free(p);
   owned_.clear();
+  tables_.clear();
   planned_ = false;
-  ws64_a_ = ws64_b_ = wsbf_a_ = wsbf_b_ = wspart_ = 0;
+  ws64_a_ = ws64_b_ = wsbf_a_ = wsbf_b_ = wspart_ = wscount_ = 0;
+  dev_free(wcount_);
+  wcount_ = nullptr;
   dev_free(wpart_);
   wpart_ = nullptr;
   dev_free(w64a_);
@@ -442,20 +465,30 @@ Site& Engine::site() {
   return *sites_[cursor_++];
 }
 
+// Offset tables are small and many (several per operand and plan): they share
+// chunks of device memory, filled on the host while planning and copied once
+// each in finalize().
 DevTable Engine::upload(const std::vector<int64_t>& v) {
+  constexpr size_t kChunk = 1 << 17, kAlign = 32;  // elements; 256-byte aligned tables
+  const size_t need = (std::max<size_t>(v.size(), 1) + kAlign - 1) / kAlign * kAlign;
+  if (tables_.empty() || tables_.back().host.size() + need > tables_.back().cap) {
+    TableChunk c;
+    c.cap = std::max(need, kChunk);
+    c.d = static_cast<int64_t*>(dev_alloc(c.cap * sizeof(int64_t)));
+    owned_.push_back(c.d);
+    bytes_ += c.cap * sizeof(int64_t);
+    tables_.push_back(std::move(c));
+  }
+  TableChunk& c = tables_.back();
   DevTable t;
   t.n = static_cast<int64_t>(v.size());
-  const size_t bytes = std::max<size_t>(v.size(), 1) * sizeof(int64_t);
-  t.d = static_cast<int64_t*>(dev_alloc(bytes));
-  owned_.push_back(t.d);
-  bytes_ += bytes;
-  if (!v.empty()) GBCC_CK(cudaMemcpy(t.d, v.data(), v.size() * sizeof(int64_t), cudaMemcpyHostToDevice));
+  t.d = c.d + c.host.size();
+  c.host.insert(c.host.end(), v.begin(), v.end());
+  c.host.resize(static_cast<size_t>(t.d - c.d) + need, 0);
   return t;
 }
 
-int Engine::slices_for(TermClass cls, double flops) const {
-  // contractions this small are cheaper in FP64 than a tensor-core launch
-  if (flops < 1.0e6) return 0;
+int Engine::slices_for(TermClass cls) const {
   return slices_[cls];
 }
 
@@ -760,6 +793,13 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
         const GemmTcArgs t = tc_args(p, cls, panel);
         launch_tc(p, t);
       }
+    } else if (p.small) {
+      GemmSmallArgs g = p.sg;
+      g.partial = wpart_;
+      g.count = wcount_;
+      prof_gemm(s);
+      launch_gemm_small(g, stream_);
+      ++n_launch_;
     } else {
       const double* panel[2];
       for (int side = 0; side < 2; ++side) {
@@ -855,7 +895,11 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
     p = GemmPlan{};
     p.flops = flops;
     const bool emu = pm == 2;
-    int slices = pm == 1 ? slices_for(cls, flops) : (emu && slices_for(cls, flops) > 0 ? kFixedSlices : 0);
+    p.sg.M = std::max(rowsA, rowsB);
+    p.sg.N = std::min(rowsA, rowsB);
+    p.sg.K = K;
+    p.small = plan_gemm_small(p.sg) <= (pm == 0 ? kSmallUs : (emu ? kSmallUsFixed : kSmallUsMixed));
+    int slices = p.small || pm == 0 ? 0 : (emu ? kFixedSlices : slices_for(cls));
     // a short contraction into a large output is memory-bound: CUDA cores
     // (measured faster for N > 32; the tensor-core kernel wins below).  The
     // FP64-grade plan keeps such contractions on the FP64 kernel.
@@ -894,7 +938,10 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
     // contracted-index order
     const Ix& bigM = Ms[0].x;
     const Ix& bigN = Ns[0].x;
-    if (!p.use_tc) {
+    if (p.small) {
+      const Ix& ref = bigM.t->size() >= bigN.t->size() ? bigM : bigN;
+      PM.kord = order_by(kset, ref.lab);
+    } else if (!p.use_tc) {
       const bool dM = Ms.size() == 1 && !Ms[0].y.t && storage_is_panel(bigM, mext);
       const bool dN = Ns.size() == 1 && !Ns[0].y.t && storage_is_panel(bigN, next);
       if (dM && (!dN || bigM.t->size() >= bigN.t->size())) {
@@ -957,7 +1004,7 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
       gather_finish(g);
       g.R = op.rows;
       g.C = op.K;
-      if (!p.use_tc) {
+      if (!p.use_tc && !p.small) {
         g.Rpad = op.rows;
         g.Cpad = op.K;
         g.ldo = op.K;
@@ -983,7 +1030,19 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
     if (p.smallk && !p.P[0].direct && p.P[0].gather.plain && p.P[0].gather.transpose &&
         smallk_streams(p.N, K, p.m_major))
       p.P[0].inplace = true;
-    if (!p.use_tc && !p.smallk) {
+    if (p.small) {
+      GemmSmallArgs& g = p.sg;
+      g.a = p.P[0].gather;
+      g.b = p.P[1].gather;
+      g.C = p.C;
+      g.cm = p.cm;
+      g.cn = p.cn;
+      g.alpha = p.alpha;
+      g.beta = p.beta;
+      p.ksplit = g.ksplit;
+      wspart_ = std::max(wspart_, g.partial_elems);
+      if (g.ksplit > 1) wscount_ = std::max(wscount_, static_cast<size_t>(g.tiles));
+    } else if (!p.use_tc && !p.smallk) {
       // fewer 64 x 64 output tiles than two per SM: split K over blocks (one SM
       // runs FP64 at ~1/150 of the GPU's already low FP64 rate, so even a
       // 1 MFLOP contraction is slow on a single block)
@@ -1135,11 +1194,14 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
 
 void Engine::finalize() {
   if (!planned_) throw Error(GBCC_ERR_STATE, "engine: finalize before PLAN");
+  for (const TableChunk& c : tables_)
+    GBCC_CK(cudaMemcpy(c.d, c.host.data(), c.host.size() * sizeof(int64_t), cudaMemcpyHostToDevice));
+  tables_.clear();
   // every old workspace is released and its pointer cleared before the first
   // new allocation: one that fails leaves no pointer to freed memory behind
   for (void** p : {reinterpret_cast<void**>(&w64a_), reinterpret_cast<void**>(&w64b_),
                    reinterpret_cast<void**>(&wbfa_), reinterpret_cast<void**>(&wbfb_),
-                   reinterpret_cast<void**>(&wpart_)}) {
+                   reinterpret_cast<void**>(&wpart_), reinterpret_cast<void**>(&wcount_)}) {
     dev_free(*p);
     *p = nullptr;
   }
@@ -1148,7 +1210,9 @@ void Engine::finalize() {
   wbfa_ = static_cast<__nv_bfloat16*>(dev_alloc(wsbf_a_ * sizeof(__nv_bfloat16)));
   wbfb_ = static_cast<__nv_bfloat16*>(dev_alloc(wsbf_b_ * sizeof(__nv_bfloat16)));
   wpart_ = static_cast<double*>(dev_alloc(wspart_ * sizeof(double)));
-  bytes_ += (ws64_a_ + ws64_b_ + wspart_) * sizeof(double) + (wsbf_a_ + wsbf_b_) * sizeof(__nv_bfloat16);
+  wcount_ = static_cast<unsigned*>(dev_alloc(wscount_ * sizeof(unsigned)));
+  GBCC_CK(cudaMemsetAsync(wcount_, 0, std::max<size_t>(wscount_, 1) * sizeof(unsigned), stream_));
+  bytes_ += wscount_ * sizeof(unsigned) + (ws64_a_ + ws64_b_ + wspart_) * sizeof(double) + (wsbf_a_ + wsbf_b_) * sizeof(__nv_bfloat16);
   // packs shared by several contractions of a residual get their own buffer
   for (auto& kv : pack_uses_) {
     if (kv.second.size() < 2) continue;

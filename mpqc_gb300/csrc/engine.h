@@ -169,6 +169,8 @@ class Engine {
   // packs of them can be shared between contractions.
   void set_frozen(std::initializer_list<const Tensor*> ts) { frozen_ = std::unordered_set<const Tensor*>(ts); }
   std::vector<SiteStat> site_stats(int precision);
+  // whether the mixed plan has a tensor-core contraction of this class
+  bool class_on_tensor_cores(TermClass cls) const;
 
   // Persistent device tensor owned by the engine (allocated on first request).
   Tensor& tensor(const std::string& name, std::initializer_list<int64_t> dims, bool constant = false);
@@ -224,7 +226,7 @@ class Engine {
   void launch_tc_classes(const GemmPlan& p, TermClass cls, __nv_bfloat16* const panel[2]);
   GemmTcArgs tc_args(const GemmPlan& p, TermClass cls, __nv_bfloat16* const panel[2]) const;
   void launch_tc(const GemmPlan& p, const GemmTcArgs& t);
-  int slices_for(TermClass cls, double flops) const;
+  int slices_for(TermClass cls) const;
 
   cudaStream_t stream_ = nullptr;
   Mode mode_ = Mode::kPlan;
@@ -236,9 +238,16 @@ class Engine {
   std::vector<std::unique_ptr<Site>> sites_;
   std::unordered_map<std::string, std::unique_ptr<Tensor>> tensors_;
   std::vector<void*> owned_;  // tables and constant-pack buffers
+  struct TableChunk {  // offset tables waiting for finalize()
+    int64_t* d = nullptr;
+    size_t cap = 0;
+    std::vector<int64_t> host;
+  };
+  std::vector<TableChunk> tables_;
   // shared workspaces (sized during PLAN)
-  size_t ws64_a_ = 0, ws64_b_ = 0, wsbf_a_ = 0, wsbf_b_ = 0, wspart_ = 0;
+  size_t ws64_a_ = 0, ws64_b_ = 0, wsbf_a_ = 0, wsbf_b_ = 0, wspart_ = 0, wscount_ = 0;
   double* wpart_ = nullptr;  // K-split partial tiles
+  unsigned* wcount_ = nullptr;  // finished splits of each tile (gemm_small.cu), zero between launches
   double* w64a_ = nullptr;
   double* w64b_ = nullptr;
   __nv_bfloat16* wbfa_ = nullptr;

@@ -167,6 +167,28 @@ struct GemmF64Args {
 };
 void launch_gemm_f64(const GemmF64Args& g, cudaStream_t st);
 
+// Small FP64 contractions, operands read in place through their gather terms
+// (gemm_small.cu); same C, cm, cn, alpha, beta as GemmF64Args.
+struct GemmSmallArgs {
+  int64_t M, N, K;
+  // operand terms (t, nterms, plain, transpose of GatherArgs are used)
+  GatherArgs a, b;
+  double* C;
+  const int64_t* cm;
+  const int64_t* cn;
+  double alpha, beta;
+  // set by plan_gemm_small: output tile, tiles along N and in all, K split
+  int tm, tn, ntn, ksplit, kps;
+  int64_t tiles;
+  size_t partial_elems;
+  // partial tiles (partial_elems) and one zeroed counter per tile (ksplit > 1)
+  double* partial;
+  unsigned* count;
+};
+// Chooses the tile and the K split for M, N, K; returns the estimated time in us.
+double plan_gemm_small(GemmSmallArgs& g);
+void launch_gemm_small(const GemmSmallArgs& g, cudaStream_t st);
+
 // Short contractions (K <= kSmallK) with large outputs on CUDA cores: FP64
 // panels rounded to FP32, FP32 products and sums, one FP64 FMA per output.
 // Memory-bound on the FP64 read-modify-write of C; used in mixed precision

@@ -198,6 +198,75 @@ extern "C" int gbcc_testing_gemm_ex3(int64_t M, int64_t N, int64_t K, const doub
   return status;
 }
 
+extern "C" int gbcc_testing_gemm_small(int64_t M, int64_t N, int64_t K, const double* A, const double* B,
+                                       double* Cout, int mode, int repeat, float* ms) {
+  using namespace gbcc;
+  if (M < 1 || N < 1 || K < 1 || !A || !B || !Cout || mode < 0 || mode > 15 || repeat < 1) return GBCC_ERR_INVALID_ARG;
+  std::vector<void*> owned;
+  auto alloc = [&](size_t bytes) {
+    void* p = dev_alloc(bytes);
+    owned.push_back(p);
+    return p;
+  };
+  int status = GBCC_OK;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  try {
+    auto upload = [&](const void* src, size_t bytes) {
+      void* p = alloc(bytes);
+      GBCC_CK(cudaMemcpy(p, src, bytes, cudaMemcpyDefault));
+      return p;
+    };
+    auto table = [&](int64_t n, int64_t stride) {
+      std::vector<int64_t> h(n);
+      for (int64_t i = 0; i < n; ++i) h[i] = i * stride;
+      return static_cast<int64_t*>(upload(h.data(), n * sizeof(int64_t)));
+    };
+    GemmSmallArgs g{};
+    g.M = M; g.N = N; g.K = K;
+    auto operand = [&](GatherArgs& x, const double* src, int64_t rows, bool k_major, bool two) {
+      x.nterms = two ? 2 : 1;
+      x.plain = two ? 0 : 1;
+      x.transpose = k_major ? 1 : 0;
+      gather_set_coef(x.t[0], two ? 2.0 : 1.0);
+      x.t[0].a = static_cast<const double*>(upload(src, rows * K * sizeof(double)));
+      x.t[0].ra = table(rows, k_major ? 1 : K);
+      x.t[0].ca = table(K, k_major ? rows : 1);
+      x.t[1] = x.t[0];
+      gather_set_coef(x.t[1], -0.75);
+    };
+    operand(g.a, A, M, (mode & 1) != 0, (mode & 8) != 0);
+    operand(g.b, B, N, (mode & 2) != 0, false);
+    g.C = static_cast<double*>(upload(Cout, M * N * sizeof(double)));
+    g.cm = table(M, N);
+    g.cn = table(N, 1);
+    g.alpha = (mode & 4) ? -0.5 : 1.0;
+    g.beta = (mode & 4) ? 1.0 : 0.0;
+    plan_gemm_small(g);
+    g.partial = static_cast<double*>(alloc(std::max<size_t>(g.partial_elems, 1) * sizeof(double)));
+    g.count = static_cast<unsigned*>(alloc(g.tiles * sizeof(unsigned)));
+    GBCC_CK(cudaMemset(g.count, 0, g.tiles * sizeof(unsigned)));
+    launch_gemm_small(g, nullptr);
+    GBCC_CK(cudaDeviceSynchronize());
+    GBCC_CK(cudaMemcpy(Cout, g.C, M * N * sizeof(double), cudaMemcpyDefault));
+    GBCC_CK(cudaEventCreate(&e0));
+    GBCC_CK(cudaEventCreate(&e1));
+    GBCC_CK(cudaEventRecord(e0, nullptr));
+    for (int r = 0; r < repeat; ++r) launch_gemm_small(g, nullptr);
+    GBCC_CK(cudaEventRecord(e1, nullptr));
+    GBCC_CK(cudaEventSynchronize(e1));
+    float t = 0.f;
+    GBCC_CK(cudaEventElapsedTime(&t, e0, e1));
+    if (ms) *ms = t / repeat;
+  } catch (const Error& e) {
+    cudaGetLastError();
+    status = e.status;
+  }
+  if (e0) cudaEventDestroy(e0);
+  if (e1) cudaEventDestroy(e1);
+  for (void* p : owned) dev_free(p);
+  return status;
+}
+
 extern "C" int gbcc_testing_split(const double* x, int64_t n, int nslices, uint16_t* out) {
   using namespace gbcc;
   if (!x || !out || n < 0 || nslices < 1 || nslices > 3) return GBCC_ERR_INVALID_ARG;
