@@ -237,9 +237,6 @@ constexpr double kSmallUs = 800.0;
 constexpr double kSmallUsMixed = 20.0;
 constexpr double kSmallUsFixed = 80.0;
 
-// slice pairs of a plan: 3 slices give 6, the fixed-point split's 6 slices 21
-constexpr int kMaxPlanPairs = 36;
-
 struct GemmPlan {
   bool use_tc = false;
   bool smallk = false;     // mixed precision, K <= kSmallK: FP32 CUDA-core kernel on FP64 panels
@@ -253,11 +250,11 @@ struct GemmPlan {
   double alpha = 1.0, beta = 0.0;
   double* C = nullptr;
   int slices = 0, npairs = 0, bn = 0;
-  bool emu = false;        // FP64_TC: pairs ordered by weight class, one launch per class
+  bool emu = false;        // FP64_TC: fixed-point slices (gemm_multi.cu)
   int ksplit = 1;         // K split over CTAs (deterministic two-pass reduction)
   bool m_major = false;   // C unit-stride along M
-  int64_t k_per_split = 0;  // FP64: K elements per split; tensor cores: k-blocks per split
-  int pa[kMaxPlanPairs] = {}, pb[kMaxPlanPairs] = {};
+  int64_t k_per_split = 0;  // FP64: K elements per split; tensor cores: k-blocks (FP64_TC: halves of them) per split
+  int pa[kMaxPairs] = {}, pb[kMaxPairs] = {};
   double flops = 0.0;
   int sps = 1;             // tensor cores: slices per pipeline stage (2: both slices of a k-block)
   int group = 1;           // tensor cores: M tiles per band of the tile order (1: rows)
@@ -334,7 +331,6 @@ std::vector<SiteStat> Engine::site_stats(int precision) {
       const GemmPlan& p = sp->plan[plan_index(precision)];
       st.flops = p.flops;
       st.pairs = p.use_tc ? p.npairs : 0;
-      st.classes = p.use_tc && p.emu ? p.slices : 0;
       st.cls = sp->cls;
       st.M = p.M;
       st.N = p.N;
@@ -617,12 +613,10 @@ GemmTcArgs Engine::tc_args(const GemmPlan& p, TermClass cls, __nv_bfloat16* cons
   t.b_slices = p.slices;
   // a slice limit below the packed count keeps the pairs p + q < limit: the
   // split is sequential, so these are exactly the products of a
-  // limit-slice split (used to measure the error of fewer slices); it
-  // applies to the mixed plan only
-  const int lim = p.emu ? 0 : slice_limit_[cls];
+  // limit-slice split (used to measure the error of fewer slices)
+  const int lim = slice_limit_[cls];
   t.npairs = 0;
-  // FP64_TC: the pairs of each weight class are set per launch (launch_tc_classes)
-  for (int q = 0; q < (p.emu ? 0 : p.npairs); ++q) {
+  for (int q = 0; q < p.npairs; ++q) {
     if (lim > 0 && p.pa[q] + p.pb[q] >= lim) continue;
     t.pa[t.npairs] = p.pa[q];
     t.pb[t.npairs] = p.pb[q];
@@ -638,12 +632,6 @@ GemmTcArgs Engine::tc_args(const GemmPlan& p, TermClass cls, __nv_bfloat16* cons
   // under a slice limit measures the error the smaller plan will have)
   const int eff_slices = (lim > 0 && lim < p.slices) ? lim : p.slices;
   t.chunk = eff_slices >= 3 ? chunk_ : chunk_lo_;
-  if (p.emu) {
-    // exact FP32 chunk sums: 4 steps of 64 products below 2^14 units each,
-    // two chunks per FP32 register sum before the float-float fold
-    t.chunk = kFixedChunk;
-    t.fold = kFixedFold;
-  }
   t.err = err_;
   t.ksplit = p.ksplit;
   t.kb_per_split = static_cast<int>(p.k_per_split);
@@ -667,14 +655,36 @@ void Engine::launch_tc(const GemmPlan& p, const GemmTcArgs& t) {
   }
 }
 
-// FP64_TC: one launch per weight class w = p + q, the classes of the smallest
-// weight first; the first applies the call's beta, the rest accumulate.
-void Engine::launch_tc_classes(const GemmPlan& p, TermClass cls, __nv_bfloat16* const panel[2]) {
-  GemmTcArgs t = tc_args(p, cls, panel);
-  for (int w = p.slices - 1; w >= 0; --w) {
-    t.npairs = fixed_class_pairs(p.slices, w, t.pa, t.pb);
-    t.beta = w == p.slices - 1 ? p.beta : 1.0;
-    launch_tc(p, t);
+// FP64_TC: every weight class in one launch (gemm_multi.cu)
+void Engine::launch_fixed(const GemmPlan& p, __nv_bfloat16* const panel[2]) {
+  GemmMultiArgs t{};
+  t.M = p.M;
+  t.N = p.N;
+  t.K = p.K;
+  t.kblocks = p.P[0].Kpad / kTcBK;
+  t.A = panel[0];
+  t.a_rows = p.P[0].rows_pad;
+  t.B = panel[1];
+  t.b_rows = p.P[1].rows_pad;
+  t.bn = p.bn;
+  t.C = p.C;
+  t.cm = p.cm;
+  t.cn = p.cn;
+  t.alpha = p.alpha;
+  t.beta = p.beta;
+  t.m_major = p.m_major ? 1 : 0;
+  t.ksplit = p.ksplit;
+  t.hb_per_split = static_cast<int>(p.k_per_split);
+  t.partial = wpart_;
+  t.err = err_;
+  if (!launch_gemm_fixed(t, stream_)) throw Error(GBCC_ERR_CUDA, "tcgen05 GEMM launch rejected (tensor map or size)");
+  ++n_tc_;
+  ++tc_total_;
+  ++n_launch_;
+  if (p.ksplit > 1) {
+    launch_splitk_reduce(p.M, p.N, p.ksplit, wpart_, round_up(p.M, kTcBM), round_up(p.N, p.bn), p.C, p.cm, p.cn,
+                         p.alpha, p.beta, stream_);
+    ++n_launch_;
   }
 }
 
@@ -788,7 +798,7 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
       for (int side = 0; side < 2; ++side) panel[side] = tc_panel(p.P[side], side);
       prof_gemm(s);
       if (p.emu) {
-        launch_tc_classes(p, cls, panel);
+        launch_fixed(p, panel);
       } else {
         const GemmTcArgs t = tc_args(p, cls, panel);
         launch_tc(p, t);
@@ -1066,14 +1076,15 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
       // the ladder and ring contractions take the faster 192/256-wide tiles
       // (not FP64_TC: its chunk sums need the float-float fold of tiles up to 128)
       const bool wide = !emu && (cls == kClassLadder || cls == kClassRing);
-      p.bn = gemm_tc_pick_bn(p.N, wide);
       int bns[4];
-      const int nbn = gemm_tc_bn_candidates(p.N, wide, bns);
+      int nbn = 1;
+      if (emu) bns[0] = gemm_multi_bn(p.N);
+      else nbn = gemm_tc_bn_candidates(p.N, wide, bns);
       int64_t npanel = 0;  // N-side panel rows: room for every candidate tile width
       for (int c = 0; c < nbn; ++c) npanel = std::max<int64_t>(npanel, round_up(p.N, bns[c]));
       p.npairs = 0;
       if (emu) {
-        for (int w = 0; w < slices; ++w) p.npairs += fixed_class_pairs(slices, w, p.pa + p.npairs, p.pb + p.npairs);
+        p.npairs = slices * (slices + 1) / 2;
       } else {
         for (int a = 0; a < slices; ++a)
           for (int b = 0; b < slices; ++b)
@@ -1088,7 +1099,8 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
         OperandPlan& op = p.P[side];
         op.slices = slices;
         op.Kpad = Kpad;
-        op.rows_pad = side == 0 ? round_up(op.rows, kTcBM) : npanel;
+        // (the FP64_TC kernel's tensor maps end at the last row)
+        op.rows_pad = emu ? op.rows : (side == 0 ? round_up(op.rows, kTcBM) : npanel);
         GatherArgs& g = op.gather;
         g.Rpad = op.rows_pad;
         g.Cpad = Kpad;
@@ -1136,6 +1148,22 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
       const int64_t kblocks = Kpad / kTcBK;
       const int64_t sms = num_sms();
       p.ncand = 0;
+      if (emu) {
+        // fewer tiles than SMs: splits of at least 10 stages (two chunks), as
+        // many as fill the chip
+        p.bn = bns[0];
+        const int64_t hbs = (K + 31) / 32;
+        const int64_t tiles = ((p.M + kTcBM - 1) / kTcBM) * ((p.N + p.bn - 1) / p.bn);
+        int64_t ks = tiles < sms ? std::min<int64_t>(sms / tiles, hbs / 10) : 1;
+        if (ks > 1) {
+          p.k_per_split = (hbs + ks - 1) / ks;
+          ks = (hbs + p.k_per_split - 1) / p.k_per_split;
+        }
+        p.ksplit = static_cast<int>(std::max<int64_t>(ks, 1));
+        if (p.ksplit > 1)
+          wspart_ = std::max(wspart_, static_cast<size_t>(ks * round_up(p.M, kTcBM) * round_up(p.N, p.bn)));
+        continue;
+      }
       for (int c = 0; c < nbn; ++c) {
         const int64_t npad = round_up(p.N, bns[c]);
         const int64_t tiles = (p.P[0].rows_pad / kTcBM) * (npad / bns[c]);

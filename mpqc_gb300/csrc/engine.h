@@ -113,7 +113,6 @@ struct SiteStat {
   double gemm_ms = 0.0;  // of which the GEMM kernel
   double flops = 0.0;  // 2 M N K of a contraction, 0 for an assignment
   int pairs = 0;       // BF16 slice products on the tensor cores (0: FP64 / elementwise)
-  int classes = 0;     // FP64_TC: launches, one per weight class (0 otherwise)
   int cls = -1;        // TermClass of a contraction, -1 for an assignment
   int64_t M = 0, N = 0, K = 0;  // GEMM shape (assignment: rows, columns, 0)
   int bn = 0;          // tensor cores: N tile width; -1: the short-K CUDA-core kernel
@@ -160,7 +159,7 @@ class Engine {
     chunk_lo_ = fewer;
   }
   // Whether the next PLAN also builds the FP64-grade tensor-core plan
-  // (GBCC_PREC_FP64_TC: fixed-point slices, one launch per weight class)
+  // (GBCC_PREC_FP64_TC: fixed-point slices)
   void set_emulation(bool on) { emu_ = on; }
   bool emulation() const { return emu_; }
   // Record CUDA events around every operation of EXEC passes.
@@ -223,7 +222,7 @@ class Engine {
   DevTable upload(const std::vector<int64_t>& v);
   __nv_bfloat16* tc_panel(OperandPlan& op, int side);
   void pack_panel(const OperandPlan& op, __nv_bfloat16* out);
-  void launch_tc_classes(const GemmPlan& p, TermClass cls, __nv_bfloat16* const panel[2]);
+  void launch_fixed(const GemmPlan& p, __nv_bfloat16* const panel[2]);
   GemmTcArgs tc_args(const GemmPlan& p, TermClass cls, __nv_bfloat16* const panel[2]) const;
   void launch_tc(const GemmPlan& p, const GemmTcArgs& t);
   int slices_for(TermClass cls) const;

@@ -26,8 +26,10 @@
 //
 // Persistent kernel: one CTA per SM walks the 128 x BN output tiles
 // (N-tile index fastest, so CTAs running together share the A panel in L2).
-//   warp 0     : TMA producer (one thread), STAGES-deep smem ring
-//   warp 1     : TMEM allocator + MMA issuer (one thread), kind::f16
+//   warp 0     : TMA producer, STAGES-deep smem ring
+//   warp 1     : TMEM allocator + MMA issuer, kind::f16 (both warps run their
+//                loops with all lanes, one lane elected per instruction:
+//                tc_common.cuh)
 //   warps 4..11: epilogue; warp w reads TMEM lanes 32*(w%4).. and the column
 //                half (w-4)/4 of the tile (warps 2 and 3 only pad the
 //                block to three warps per scheduler, which leaves 168
@@ -36,266 +38,18 @@
 // Every mbarrier wait is bounded: on timeout the kernel records kDevTimeout in
 // *err, drains its own copies in flight, waits for its MMAs, frees its TMEM
 // and returns.
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
 #include <cstdio>
 #include <cstring>
-#include <mutex>
 
 #include "fp_bits.cuh"
 #include "kernels.h"
+#include "tc_common.cuh"
 
 namespace gbcc {
 namespace {
 
 constexpr int BM = kTcBM;   // 128
 constexpr int BK = kTcBK;   // 64 bf16 = 128 bytes = one swizzle row
-constexpr uint64_t kWaitNs = 2000000000ull;  // 2 s per wait
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ uint64_t globaltimer() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait for the phase of `parity` to complete.  Gives up (false) after
-// limit_ns, or early once any CTA has recorded an error.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const int* err,
-                                          uint64_t limit_ns = kWaitNs) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer();
-  for (uint32_t it = 1;; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 255u) == 0) {
-      if (globaltimer() - t0 > limit_ns) return false;
-      if (*reinterpret_cast<const volatile int*>(err) != kDevOk) return false;
-    }
-  }
-}
-
-// Bounded wait that ignores the error word (teardown paths).
-__device__ __forceinline__ void mbar_wait_teardown(uint64_t* bar, uint32_t parity) {
-  const uint64_t t0 = globaltimer();
-  while (!mbar_try_wait(bar, parity) && globaltimer() - t0 < kWaitNs) {
-  }
-}
-
-__device__ __forceinline__ void record_error(int* err, int code) { atomicCAS(err, kDevOk, code); }
-
-__device__ __forceinline__ void fence_barrier_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-__device__ __forceinline__ void tma_load_3d(const CUtensorMap* map, uint64_t* bar, void* dst, int c0,
-                                            int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
-
-__device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
-  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
-               "r"(ncols)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
-               : "memory");
-}
-
-// Shared-memory matrix descriptor: K-major tile, 128-byte swizzle, 8-row
-// groups 1024 bytes apart (SBO), descriptor version 1, base offset 0 (tiles
-// are 1024-byte aligned).
-__device__ __forceinline__ uint64_t sdesc_sw128(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>(16u >> 4) << 16;    // leading byte offset (unused for SW128 K-major)
-  d |= static_cast<uint64_t>(1024u >> 4) << 32;  // stride byte offset
-  d |= static_cast<uint64_t>(1) << 46;           // descriptor version
-  d |= static_cast<uint64_t>(2) << 61;           // 128-byte swizzle
-  return d;
-}
-
-// Instruction descriptor, kind::f16: D = F32, A = B = BF16, both K-major.
-__host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
-         (static_cast<uint32_t>(m >> 4) << 24);
-}
-
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          smem_u32(bar))
-      : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-}
-
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// ---- CTA-pair (cta_group::2) helpers
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-
-// shared::cluster address of the same shared variable in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t map_to_rank(const void* p, uint32_t rank) {
-  uint32_t out;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(smem_u32(p)), "r"(rank));
-  return out;
-}
-
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_alloc2(uint32_t* slot, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
-               "r"(ncols)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-
-// TMA load into this CTA's shared memory, completion counted on the mbarrier
-// at cluster address `bar` (the pair leader's barrier).
-__device__ __forceinline__ void tma_load_3d_pair(const CUtensorMap* map, uint32_t bar, void* dst, int c0, int c1,
-                                                 int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_bf16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// Arrive on the mbarrier at the same shared offset in every CTA of `mask`
-// once the MMAs issued so far have completed.
-__device__ __forceinline__ void mma_commit_pair(uint64_t* bar, uint16_t mask) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-          smem_u32(bar)),
-      "h"(mask)
-      : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Knuth's TwoSum: hi + lo += x with the rounding error of hi + x kept in lo.
-__device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float x) {
-  const float s = __fadd_rn(hi, x);
-  const float v = __fsub_rn(s, hi);
-  const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, v)), __fsub_rn(x, v));
-  hi = s;
-  lo = __fadd_rn(lo, e);
-}
-
 constexpr int kStgLd = 17;  // padded row of the per-warp output staging tile (8-byte words)
 
 // SPS: slices per pipeline stage.  1: a stage holds one (A slice, B slice)
@@ -428,77 +182,79 @@ __global__ void __launch_bounds__(TcCfg<BN, CTA2, SPS>::kThreads, 1)
   // wait limit of the pipeline's barriers (a test hook may shorten it)
   const uint64_t wait_ns = g.wait_ns ? g.wait_ns : kWaitNs;
 
+  const uint32_t lead = elect_lead();  // the lane that issues for its warp (warps 0 and 1)
+
   if (warp == 0) {
     if (lane == 0) {
       prefetch_tmap(&tmA);
       prefetch_tmap(&tmB);
-      // first panel row of the operands (a window of a larger panel); rows
-      // past the panel's end load as zeros, rows past M or N are not stored
-      const int a_row0 = static_cast<int>(g.a_row0), b_row0 = static_cast<int>(g.b_row0);
-      uint32_t gi = 0;  // stage-use counter across tiles
-      bool ok = true;
-      // stage-ring position kept incrementally (no divisions in the loop)
-      int s = 0;
-      uint32_t ph = 0;
-      const uint32_t full0 = CTA2 ? map_to_rank(&full[0], 0) : 0;
-      for (int tile = unit; tile < ntiles && ok; tile += nunits) {
-        int m0, n0, kb0, n_iter, split;
-        decode(tile, m0, n0, kb0, n_iter, split);
-        const int nb0 = n0 + static_cast<int>(rank) * Cfg::kBRows;
-        int kb = kb0, pr = 0;
-        for (int it = 0; it < n_iter; ++it, ++gi) {
-          if (!mbar_wait(&empty[s], ph ^ 1, g.err, wait_ns)) {
-            record_error(g.err, kDevTimeout);
-            ok = false;
-            break;
+    }
+    __syncwarp();
+    // first panel row of the operands (a window of a larger panel); rows
+    // past the panel's end load as zeros, rows past M or N are not stored
+    const int a_row0 = static_cast<int>(g.a_row0), b_row0 = static_cast<int>(g.b_row0);
+    const uint32_t sA0 = smem_u32(sA), sB0 = smem_u32(sB);
+    uint32_t gi = 0;  // stage-use counter across tiles
+    bool ok = true;
+    // stage-ring position kept incrementally (no divisions in the loop)
+    int s = 0;
+    uint32_t ph = 0;
+    const uint32_t full0 = CTA2 ? map_to_rank(&full[0], 0) : 0;
+    for (int tile = unit; tile < ntiles && ok; tile += nunits) {
+      int m0, n0, kb0, n_iter, split;
+      decode(tile, m0, n0, kb0, n_iter, split);
+      const int nb0 = n0 + static_cast<int>(rank) * Cfg::kBRows;
+      int kb = kb0, pr = 0;
+      for (int it = 0; it < n_iter; ++it, ++gi) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&empty[s], ph ^ 1, g.err, wait_ns));
+        if (!ok) {
+          record_error(g.err, kDevTimeout);
+          break;
+        }
+        const uint32_t dA = sA0 + s * Cfg::kAStage, dB = sB0 + s * Cfg::kBStage;
+        if constexpr (CTA2) {
+          // the leader's full barrier counts the bytes of both CTAs
+          const uint32_t bar = full0 + static_cast<uint32_t>(s) * 8u;
+          if (leader) mbar_expect_tx(lead, &full[s], 2 * Cfg::kStageBytes);
+          tma_load_3d_pair(lead, &tmA, bar, dA, 0, m0 + a_row0, g.pa[pr] * kblocks + kb);
+          tma_load_3d_pair(lead, &tmB, bar, dB, 0, nb0 + b_row0, g.pb[pr] * kblocks + kb);
+        } else if constexpr (SPS == 1) {
+          // test hook (gbcc_testing_gemm_timeout): leave one stage unloaded,
+          // so that its consumer's bounded wait runs out
+          if (g.skip_stage1 == 0 || static_cast<int64_t>(gi) + 1 != g.skip_stage1) {
+            mbar_expect_tx(lead, &full[s], Cfg::kStageBytes);
+            tma_load_3d(lead, &tmA, &full[s], dA, 0, m0 + a_row0, g.pa[pr] * kblocks + kb);
+            tma_load_3d(lead, &tmB, &full[s], dB, 0, nb0 + b_row0, g.pb[pr] * kblocks + kb);
           }
-          if constexpr (CTA2) {
-            // the leader's full barrier counts the bytes of both CTAs
-            const uint32_t bar = full0 + static_cast<uint32_t>(s) * 8u;
-            if (leader) mbar_expect_tx(&full[s], 2 * Cfg::kStageBytes);
-            tma_load_3d_pair(&tmA, bar, sA + s * Cfg::kAStage, 0, m0 + a_row0, g.pa[pr] * kblocks + kb);
-            tma_load_3d_pair(&tmB, bar, sB + s * Cfg::kBStage, 0, nb0 + b_row0, g.pb[pr] * kblocks + kb);
-          } else if constexpr (SPS == 1) {
-            // test hook (gbcc_testing_gemm_timeout): leave one stage unloaded,
-            // so that its consumer's bounded wait runs out
-            if (g.skip_stage1 == 0 || static_cast<int64_t>(gi) + 1 != g.skip_stage1) {
-              mbar_expect_tx(&full[s], Cfg::kStageBytes);
-              tma_load_3d(&tmA, &full[s], sA + s * Cfg::kAStage, 0, m0 + a_row0, g.pa[pr] * kblocks + kb);
-              tma_load_3d(&tmB, &full[s], sB + s * Cfg::kBStage, 0, nb0 + b_row0, g.pb[pr] * kblocks + kb);
-            }
-          } else {
-            // every slice of A and B of this k-block
-            mbar_expect_tx(&full[s], Cfg::kStageBytes);
+        } else {
+          // every slice of A and B of this k-block
+          mbar_expect_tx(lead, &full[s], Cfg::kStageBytes);
 #pragma unroll
-            for (int j = 0; j < SPS; ++j) {
-              tma_load_3d(&tmA, &full[s], sA + s * Cfg::kAStage + j * Cfg::kABytes, 0, m0 + a_row0,
-                          j * kblocks + kb);
-              tma_load_3d(&tmB, &full[s], sB + s * Cfg::kBStage + j * Cfg::kBBytes, 0, nb0 + b_row0,
-                          j * kblocks + kb);
-            }
-          }
-          if (SPS > 1 || ++pr == g.npairs) {
-            pr = 0;
-            ++kb;
-          }
-          if (++s == S) {
-            s = 0;
-            ph ^= 1;
+          for (int j = 0; j < SPS; ++j) {
+            tma_load_3d(lead, &tmA, &full[s], dA + j * Cfg::kABytes, 0, m0 + a_row0, j * kblocks + kb);
+            tma_load_3d(lead, &tmB, &full[s], dB + j * Cfg::kBBytes, 0, nb0 + b_row0, j * kblocks + kb);
           }
         }
-      }
-      // every copy issued here has landed before the CTA can exit: the
-      // leader's full barriers count them; the partner sees them consumed
-      const uint32_t first = gi > static_cast<uint32_t>(S) ? gi - S : 0;
-      for (uint32_t u = first; u < gi; ++u) {
-        if (leader) mbar_wait_teardown(&full[u % S], (u / S) & 1);
-        else mbar_wait_teardown(&empty[u % S], (u / S) & 1);
+        if (SPS > 1 || ++pr == g.npairs) {
+          pr = 0;
+          ++kb;
+        }
+        if (++s == S) {
+          s = 0;
+          ph ^= 1;
+        }
       }
     }
+    // every copy issued here has landed before the CTA can exit: the
+    // leader's full barriers count them; the partner sees them consumed
+    const uint32_t first = gi > static_cast<uint32_t>(S) ? gi - S : 0;
+    for (uint32_t u = first; u < gi; ++u) {
+      if (leader) mbar_wait_teardown(&full[u % S], (u / S) & 1);
+      else mbar_wait_teardown(&empty[u % S], (u / S) & 1);
+    }
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (leader) {
       constexpr uint32_t idesc = idesc_bf16(BMP, BN);
-      uint32_t gi = 0;  // stage-use counter
       uint32_t c = 0;   // chunk counter
       bool ok = true;
       // shared-memory descriptors: built once, advanced by adding encoded
@@ -511,60 +267,54 @@ __global__ void __launch_bounds__(TcCfg<BN, CTA2, SPS>::kThreads, 1)
         int m0, n0, kb0, n_iter, split;
         decode(tile, m0, n0, kb0, n_iter, split);
         int pos = 0;
-        for (int it = 0; it < n_iter; ++it, ++gi) {
+        for (int it = 0; it < n_iter; ++it) {
           const uint32_t b = c & 1;
-          if (pos == 0 && !mbar_wait(&acc_empty[b], ((c >> 1) & 1) ^ 1, g.err, wait_ns)) {
+          if (pos == 0) ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[b], ((c >> 1) & 1) ^ 1, g.err, wait_ns));
+          if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&full[s], ph, g.err, wait_ns));
+          if (!ok) {
             record_error(g.err, kDevTimeout);
-            ok = false;
-            break;
-          }
-          if (!mbar_wait(&full[s], ph, g.err, wait_ns)) {
-            record_error(g.err, kDevTimeout);
-            ok = false;
             break;
           }
           tc_fence_after();
           const uint32_t d = tmem + b * BN;
           if constexpr (SPS == 1) {
-            const uint64_t ad = adesc0 + ((static_cast<uint64_t>(s) * Cfg::kAStage) >> 4);
-            const uint64_t bd = bdesc0 + ((static_cast<uint64_t>(s) * Cfg::kBStage) >> 4);
+            const uint64_t ad = adesc0 + static_cast<uint64_t>(s * (Cfg::kAStage >> 4));
+            const uint64_t bd = bdesc0 + static_cast<uint64_t>(s * (Cfg::kBStage >> 4));
 #pragma unroll
             for (int k = 0; k < BK / 16; ++k) {
               const uint32_t acc = (pos > 0 || k > 0) ? 1u : 0u;
-              if constexpr (CTA2) mma_bf16_pair(d, ad + 2 * k, bd + 2 * k, idesc, acc);
-              else mma_bf16(d, ad + 2 * k, bd + 2 * k, idesc, acc);
+              if constexpr (CTA2) mma_bf16_pair(lead, d, ad + 2 * k, bd + 2 * k, idesc, acc);
+              else mma_bf16(lead, d, ad + 2 * k, bd + 2 * k, idesc, acc);
             }
           } else {
             // all slice pairs of the k-block from the one stage
             for (int q = 0; q < g.npairs; ++q) {
-              const uint64_t ad = adesc0 + ((static_cast<uint64_t>(s) * Cfg::kAStage +
-                                             static_cast<uint64_t>(g.pa[q]) * Cfg::kABytes) >> 4);
-              const uint64_t bd = bdesc0 + ((static_cast<uint64_t>(s) * Cfg::kBStage +
-                                             static_cast<uint64_t>(g.pb[q]) * Cfg::kBBytes) >> 4);
+              const uint64_t ad = adesc0 + static_cast<uint64_t>(s * (Cfg::kAStage >> 4) + g.pa[q] * (Cfg::kABytes >> 4));
+              const uint64_t bd = bdesc0 + static_cast<uint64_t>(s * (Cfg::kBStage >> 4) + g.pb[q] * (Cfg::kBBytes >> 4));
 #pragma unroll
               for (int k = 0; k < BK / 16; ++k) {
                 const uint32_t acc = (pos > 0 || q > 0 || k > 0) ? 1u : 0u;
-                mma_bf16(d, ad + 2 * k, bd + 2 * k, idesc, acc);
+                mma_bf16(lead, d, ad + 2 * k, bd + 2 * k, idesc, acc);
               }
             }
           }
-          if constexpr (CTA2) mma_commit_pair(&empty[s], 0x3);
-          else mma_commit(&empty[s]);
+          if constexpr (CTA2) mma_commit_pair(lead, &empty[s], 0x3);
+          else mma_commit(lead, &empty[s]);
           if (++s == S) {
             s = 0;
             ph ^= 1;
           }
           if (++pos == chunk || it == n_iter - 1) {
-            if constexpr (CTA2) mma_commit_pair(&acc_full[b], 0x3);
-            else mma_commit(&acc_full[b]);
+            if constexpr (CTA2) mma_commit_pair(lead, &acc_full[b], 0x3);
+            else mma_commit(lead, &acc_full[b]);
             ++c;
             pos = 0;
           }
         }
       }
       // TMEM is freed below only after every MMA issued here has completed
-      if constexpr (CTA2) mma_commit_pair(done, 0x1);
-      else mma_commit(done);
+      if constexpr (CTA2) mma_commit_pair(lead, done, 0x1);
+      else mma_commit(lead, done);
       mbar_wait_teardown(done, 0);
     }
   } else if (warp >= kEpiWarp0) {
@@ -832,20 +582,6 @@ __global__ void __launch_bounds__(TcCfg<BN, CTA2, SPS>::kThreads, 1)
     if constexpr (CTA2) tmem_dealloc2(tmem, Cfg::kTmemCols);
     else tmem_dealloc(tmem, Cfg::kTmemCols);
   }
-}
-
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-            cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-  });
-  return fn;
 }
 
 // Operand panels are k-block major per slice, [Kpad/64][rows][64] BF16, so a

@@ -268,6 +268,44 @@ constexpr int kTcBM = 128;
 constexpr int kTcBK = 64;
 
 // ---------------------------------------------------------------------------
+// Tensor-core products with every slice of a K block staged once (gemm_multi.cu).
+// Panels are slice panels as above, [slices][kblocks][rows][64].
+// ---------------------------------------------------------------------------
+struct GemmMultiArgs {
+  int64_t M, N, K;
+  int64_t kblocks;                  // Kpad / 64
+  const __nv_bfloat16* A;
+  const __nv_bfloat16* A2;          // (T): the second segment's A panel
+  const __nv_bfloat16* B;
+  int64_t a_rows, b_rows;           // rows per slice and k-block as stored
+  int bn;
+  // C[cm[m] + cn[n]] = beta C + alpha A B^T, or partial tiles [ksplit][Mpad][Npad]
+  double* C;
+  const int64_t* cm;
+  const int64_t* cn;
+  double alpha, beta;
+  int m_major;
+  int ksplit, hb_per_split;         // split of K over CTAs, in stages of 32 elements
+  double* partial;
+  int* err;
+  // (T): triples (i, j, k), their sums W[triple][3][v][v][v] (float2 high and
+  // low words with three slices, double with six)
+  const int4* triples;
+  int o, v;
+  double* W;
+  // set by the launchers
+  int hbs, last_k16, ntm, ntn, nts, ntf, tiles;
+  int64_t Mpad, Npad;
+};
+// FP64-grade product of fixed-point panels (kFixedSlices slices); bn 32 or 64
+// (gemm_multi_bn).  false: nothing launched (bad size or tensor map).
+bool launch_gemm_fixed(GemmMultiArgs g, cudaStream_t st);
+int gemm_multi_bn(int64_t N);
+// The three sums of two (T) permutation terms of each triple (triples.cu);
+// A, A2: rows (x, p, q) and (x, q, p) of o v^2, B: rows (y, z, r) of o^2 v
+bool launch_gemm_triples(GemmMultiArgs g, int slices, int ntriples, cudaStream_t st);
+
+// ---------------------------------------------------------------------------
 // Deterministic FP64 reductions for the residual-augmented energy and the
 // residual norm (two passes, fixed grid, fixed order).
 //   out[0] = sum r1^2, out[1] = sum r2^2,

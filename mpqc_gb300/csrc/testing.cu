@@ -446,7 +446,7 @@ extern "C" int gbcc_testing_gemm_fp64tc(int64_t M, int64_t N, int64_t K, const d
   try {
     cudaStream_t st = nullptr;
     const int nsl = kFixedSlices;
-    const int bn = bn_req ? bn_req : gemm_tc_pick_bn(N, false);
+    const int bn = bn_req ? bn_req : gemm_multi_bn(N);
     const int64_t Mpad = rup(M, cta2 ? 2 * kTcBM : kTcBM), Npad = rup(N, bn), Kpad = rup(K, kTcBK);
     double* dA = static_cast<double*>(alloc(M * K * sizeof(double)));
     double* dB = static_cast<double*>(alloc(N * K * sizeof(double)));
@@ -486,8 +486,28 @@ extern "C" int gbcc_testing_gemm_fp64tc(int64_t M, int64_t N, int64_t K, const d
       t.ksplit = static_cast<int>((kblocks + t.kb_per_split - 1) / t.kb_per_split);
       t.partial = static_cast<double*>(alloc(t.ksplit * Mpad * Npad * sizeof(double)));
     }
-    // one launch per weight class, smallest weight first, as the engine runs them
+    // tiles of 32 and 64 columns: the kernel the engine runs.  128 columns and
+    // CTA pairs: one launch of gemm_tc_kernel per weight class, smallest first.
+    const bool multi = bn_req != 128 && !cta2;
+    GemmMultiArgs u{};
+    if (multi) {
+      u.M = M; u.N = N; u.K = K; u.kblocks = Kpad / kTcBK;
+      u.A = sa; u.a_rows = Mpad; u.B = sb; u.b_rows = Npad;
+      u.bn = bn; u.C = dC; u.cm = cm; u.cn = cn; u.alpha = 1.0; u.err = err;
+      u.ksplit = 1;
+      if (ksplit > 1) {
+        const int64_t hbs = (K + 31) / 32;
+        u.hb_per_split = static_cast<int>((hbs + ksplit - 1) / ksplit);
+        u.ksplit = static_cast<int>((hbs + u.hb_per_split - 1) / u.hb_per_split);
+        u.partial = static_cast<double*>(alloc(u.ksplit * Mpad * Npad * sizeof(double)));
+      }
+    }
     auto run = [&]() {
+      if (multi) {
+        if (!launch_gemm_fixed(u, st)) throw Error(GBCC_ERR_CUDA, "tcgen05 launch rejected");
+        if (u.ksplit > 1) launch_splitk_reduce(M, N, u.ksplit, u.partial, Mpad, Npad, dC, cm, cn, 1.0, 0.0, st);
+        return;
+      }
       for (int w = nsl - 1; w >= 0; --w) {
         t.npairs = fixed_class_pairs(nsl, w, t.pa, t.pb);
         t.beta = w == nsl - 1 ? 0.0 : 1.0;

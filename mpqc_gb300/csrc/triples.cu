@@ -3,42 +3,47 @@
 // The reference's "straight" (T) (src/mpqc/chemistry/qc/lcao/cc/ccsd_t.h:
 // 1127-1167, denominators by CCSD_T_Reduce, :2274-2333) forms the connected
 // triples of all occupied triplets at once (o^3 v^3 elements).  Here the
-// triplets run in batches: for each pair i <= j, the triplets (i, j, k) with
-// k >= j (a triplet's abc sum is the same for every ordering of i, j, k, so it
-// counts once per distinct ordering).  A batch's
-//   W[k][a][b][c] = t3(a,b,c,i,j,k) = sum over the six simultaneous
+// triplets i <= j <= k run in batches (a triplet's abc sum is the same for
+// every ordering of i, j, k, so it counts once per distinct ordering):
+//   W[a][b][c] = t3(a,b,c,i,j,k) = sum over the six simultaneous
 //   permutations of (a,i),(b,j),(c,k) of
-//     X(a,b,c,i,j,k) = sum_d <id|ab> t2(d,c,j,k) - sum_l <jk|lc> t2(a,b,i,l)
-// is six GEMMs, one per permutation term, each over K = v + o (the d and l
-// sums concatenated along K), whose outputs are scattered into W through the
-// term's offset tables: each term keeps one of its operands fixed over the
-// batch and stacks the other over k, so every GEMM covers the whole batch,
-// and each writes along W's unit stride (c) in its epilogue's lane
-// direction.  The energy kernel then reads W at the six
-// virtual-index permutations that stand for t3's occupied-index permutations
-// (t3(abc,kij) = W[b][c][a], ...), adds the disconnected v3 from <ij|ab> and
-// t1, and divides by e_i + e_j + e_k - e_a - e_b - e_c.
-//
-// Operand panels (rows x K, K = v + o contiguous: columns d < v, then l),
-// packed once:
+//     X(a,b,c,i,j,k) = sum_d <id|ab> t2(d,c,j,k) - sum_l <jk|lc> t2(a,b,i,l),
+// each a product over K = v + o (the d and l sums concatenated along K) of the
+// panels (rows x K, columns d < v, then l)
 //   A  [(x,p,q)] = ( <xd|pq> = Giabc[x][d][p][q] , -t2(p,q,x,l) )
 //   At [(x,q,p)] = the same rows with p fastest
 //   B  [(y,z,c)] = ( t2(d,c,y,z) , <yz|lc> = Gijka[y][z][l][c] )
-//   B2 [(y,z,b)] = ( t2(b,d,y,z) = t2(d,b,z,y) , <zy|lb> = Gijka[z][y][l][b] )
-// in FP64 (precision FP64: the DFMA GEMM), three BF16 slices (MIXED) or six
-// fixed-point slices (FP64_TC, one launch per weight class).
+//
+// Tensor cores (MIXED: three BF16 slices, FP64_TC: six fixed-point ones).  The
+// six terms pair up by the output index that runs along B: with A for one and
+// At for the other, (i,j,k) and (j,i,k) share rows (a,b) and columns c, (i,k,j)
+// and (k,i,j) rows (a,c) and columns b, (j,k,i) and (k,j,i) rows (b,c) and
+// columns a.  Each pair is one product over 2 K (gemm_multi.cu), written once
+// to its own array, in its own order; the energy kernel adds the three as it
+// reads them.  (Six read-modify-write passes of W through scattered offsets, one
+// per term and pair i, j, took 112 ms at o = 20, v = 76; this takes 20 ms.)  A
+// batch is as many triplets as keep the three arrays in about 96 MB, most of
+// L2.  The energy kernel takes 8 x 8 x 8 blocks of a <= b <= c: all six
+// orderings of a set {a, b, c} are read once and give all six permuted W
+// (t3(abc,kij) = W[b][c][a], ...) that each of its terms needs, the disconnected
+// v3 from <ij|ab> and t1, and one denominator.
+//
+// FP64 runs the six terms as GEMMs over batches (i, j; k >= j), each keeping
+// one operand fixed over the batch, stacking the other over k and scattering
+// into W through its offset tables; its B2 [(y,z,b)] = B [(z,y,b)].
 #include <algorithm>
 #include <deque>
 #include <vector>
 
 #include "../../include/gbcc.h"
 #include "engine.h"
+#include "gather.cuh"
 #include "kernels.h"
 #include "triples.h"
 
 namespace gbcc {
 
-// test hook: triplets per batch (0: as many as keep the t3 slice in L2)
+// test hook: triplets per batch (0: the default)
 int64_t g_triples_chunk = 0;
 
 namespace {
@@ -59,11 +64,8 @@ __device__ __forceinline__ double block_sum_det(double v, double* sh) {
   return r;
 }
 
-// One batch (i, j; k = k0 + kk): block (a, kk) sums over (b, c) and writes the
-// weighted partial to partial[kk * v + a].  R: the arithmetic of the terms
-// (double for the FP64-grade precisions; float for MIXED, whose contractions
-// already carry ~1e-6 relative error), summed per thread in FP64.
-template <typename R>
+// One FP64 batch (i, j; k = k0 + kk): block (a, kk) sums over (b, c) and writes
+// the weighted partial to partial[kk * v + a].
 __global__ void __launch_bounds__(kThreads) triples_energy_kernel(
     const double* __restrict__ W, int64_t o, int64_t v, int i, int j, int k0, int nk, const double* __restrict__ Gijab,
     const double* __restrict__ t1, const double* __restrict__ eps_o, const double* __restrict__ eps_v,
@@ -76,23 +78,19 @@ __global__ void __launch_bounds__(kThreads) triples_energy_kernel(
   const double mult = (i < j && j < k) ? 6.0 : ((i == j && j == k) ? 1.0 : 3.0);
   const int64_t v2 = v * v;
   const double* __restrict__ Wk = W + static_cast<int64_t>(kk) * v2 * v;
-  const R base = static_cast<R>(eps_o[i] + eps_o[j] + eps_o[k] - eps_v[a]);
-  const R t1ai = static_cast<R>(t1[a * o + i]);
+  const double base = eps_o[i] + eps_o[j] + eps_o[k] - eps_v[a];
+  const double t1ai = t1[a * o + i];
   const double* __restrict__ g_ij = Gijab + (static_cast<int64_t>(i) * o + j) * v2;  // <ij|..>
   const double* __restrict__ g_jk = Gijab + (static_cast<int64_t>(j) * o + k) * v2;
   const double* __restrict__ g_ik = Gijab + (static_cast<int64_t>(i) * o + k) * v2;
   double acc = 0.0;
   for (int64_t e = threadIdx.x; e < v2; e += blockDim.x) {
     const int64_t b = e / v, c = e - b * v;
-    const R w = static_cast<R>(Wk[a * v2 + b * v + c]);
-    const R y = R(4) * w + static_cast<R>(Wk[b * v2 + c * v + a]) + static_cast<R>(Wk[c * v2 + a * v + b]) -
-                R(2) * (static_cast<R>(Wk[c * v2 + b * v + a]) + static_cast<R>(Wk[a * v2 + c * v + b]) +
-                        static_cast<R>(Wk[b * v2 + a * v + c]));
-    const R vv = static_cast<R>(g_ij[a * v + b]) * static_cast<R>(t1[c * o + k]) +
-                 static_cast<R>(g_jk[b * v + c]) * t1ai +
-                 static_cast<R>(g_ik[a * v + c]) * static_cast<R>(t1[b * o + j]);
-    const R d = base - static_cast<R>(eps_v[b]) - static_cast<R>(eps_v[c]);
-    acc += static_cast<double>((w + vv) * y / d);
+    const double w = Wk[a * v2 + b * v + c];
+    const double y = 4.0 * w + Wk[b * v2 + c * v + a] + Wk[c * v2 + a * v + b] -
+                     2.0 * (Wk[c * v2 + b * v + a] + Wk[a * v2 + c * v + b] + Wk[b * v2 + a * v + c]);
+    const double vv = g_ij[a * v + b] * t1[c * o + k] + g_jk[b * v + c] * t1ai + g_ik[a * v + c] * t1[b * o + j];
+    acc += (w + vv) * y / (base - eps_v[b] - eps_v[c]);
   }
   const double s = block_sum_det(acc, sh);
   if (threadIdx.x == 0) partial[static_cast<int64_t>(kk) * v + a] = mult * s;
@@ -107,22 +105,15 @@ __global__ void __launch_bounds__(kThreads) sum_kernel(const double* __restrict_
   if (threadIdx.x == 0) *out = scale * s;
 }
 
-int64_t rup(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
-
-// A packed operand: rows x K, FP64 rows (precision FP64) or a slice panel.
+// A packed operand of the FP64 path: rows x K.
 struct Panel {
-  int64_t rows = 0, K = 0, rows_pad = 0, Kpad = 0;
+  int64_t rows = 0, K = 0;
   double* f64 = nullptr;
-  __nv_bfloat16* bf = nullptr;
-  unsigned* rowexp = nullptr;
 };
 
 class Triples {
  public:
-  Triples(const TriplesInputs& in, int precision, cudaStream_t st, int* err)
-      : in_(in), prec_(precision), st_(st), err_(err) {
-    slices_ = precision == GBCC_PREC_MIXED ? 3 : (precision == GBCC_PREC_FP64_TC ? kFixedSlices : 0);
-  }
+  Triples(const TriplesInputs& in, cudaStream_t st) : in_(in), st_(st) {}
   ~Triples() {
     for (void* p : owned_) dev_free(p);
   }
@@ -150,13 +141,9 @@ class Triples {
             const int64_t* cn, bool m_major, double beta);
 
   TriplesInputs in_;
-  int prec_, slices_ = 0;
   cudaStream_t st_;
-  int* err_;
   std::vector<void*> owned_;
   std::deque<std::vector<int64_t>> tables_;  // stable addresses
-  double* partk_ = nullptr;  // K-split partial tiles
-  size_t partk_elems_ = 0;
   double* W_ = nullptr;      // t3 of one batch, [k - j][a][b][c]
   double* mask_ = nullptr;   // {0.0, 1.0}
 };
@@ -206,129 +193,37 @@ Panel Triples::pack(const double* src1, int64_t n1, const std::vector<int64_t>& 
   gather_finish(g);
   g.R = rows;
   g.C = K;
-  if (slices_ == 0) {
-    p.rows_pad = rows;
-    p.Kpad = K;
-    p.f64 = static_cast<double*>(alloc(static_cast<size_t>(rows) * K * sizeof(double)));
-    g.Rpad = rows;
-    g.Cpad = K;
-    g.ldo = K;
-    g.out = p.f64;
-    launch_gather(g, st_);
-    return p;
-  }
-  // rows padded for the widest tile (256): a window's tiles past the last
-  // row fall outside the tensor map and load as zeros
-  p.rows_pad = rup(rows, 256);
-  p.Kpad = rup(K, kTcBK);
-  p.bf = static_cast<__nv_bfloat16*>(alloc(static_cast<size_t>(slices_) * p.rows_pad * p.Kpad * sizeof(__nv_bfloat16)));
-  g.Rpad = p.rows_pad;
-  g.Cpad = p.Kpad;
-  g.ldo = p.Kpad;
-  g.outs = p.bf;
-  g.nslices = slices_;
-  g.slice_stride = p.rows_pad * p.Kpad;
-  if (prec_ == GBCC_PREC_FP64_TC) {
-    p.rowexp = static_cast<unsigned*>(alloc(static_cast<size_t>(p.rows_pad) * sizeof(unsigned)));
-    GBCC_CK(cudaMemsetAsync(p.rowexp, 0, static_cast<size_t>(p.rows_pad) * sizeof(unsigned), st_));
-    g.rowexp = p.rowexp;
-    g.fixed = 1;
-    launch_gather(g, st_);
-    g.fixed = 2;
-  }
+  p.f64 = static_cast<double*>(alloc(static_cast<size_t>(rows) * K * sizeof(double)));
+  g.Rpad = rows;
+  g.Cpad = K;
+  g.ldo = K;
+  g.out = p.f64;
   launch_gather(g, st_);
   return p;
 }
 
-// C[cm[m] + cn[n]] = beta C + alpha sum_k A[a0 + m][k] B[b0 + n][k], m < M, n < N
+// C[cm[m] + cn[n]] = beta C + sum_k A[a0 + m][k] B[b0 + n][k], m < M, n < N
 void Triples::gemm(const Panel& A, int64_t a0, int64_t M, const Panel& B, int64_t b0, int64_t N, const int64_t* cm,
                    const int64_t* cn, bool m_major, double beta) {
-  const double alpha = 1.0;
   if (M <= 0 || N <= 0) return;
   // the operand windows lie inside their panels (checked on the host)
   if (a0 < 0 || a0 + M > A.rows || b0 < 0 || b0 + N > B.rows || A.K != B.K)
     throw Error(GBCC_ERR_STATE, "(T): GEMM window outside its operand panel");
-  if (slices_ == 0) {
-    GemmF64Args f{};
-    f.M = M;
-    f.N = N;
-    f.K = A.K;
-    f.A = A.f64 + a0 * A.K;
-    f.lda = A.K;
-    f.B = B.f64 + b0 * B.K;
-    f.ldb = B.K;
-    f.C = W_;
-    f.cm = cm;
-    f.cn = cn;
-    f.alpha = alpha;
-    f.beta = beta;
-    f.m_major = m_major ? 1 : 0;
-    launch_gemm_f64(f, st_);
-    return;
-  }
-  const bool emu = prec_ == GBCC_PREC_FP64_TC;
-  GemmTcArgs t{};
-  t.M = M;
-  t.N = N;
-  t.bn = gemm_tc_pick_bn(N, !emu);
-  t.Mpad = rup(M, kTcBM);
-  t.Npad = rup(N, t.bn);
-  t.Kpad = A.Kpad;
-  t.A = A.bf;
-  t.a_slices = slices_;
-  t.a_rows = A.rows_pad;
-  t.a_row0 = a0;
-  t.B = B.bf;
-  t.b_slices = slices_;
-  t.b_rows = B.rows_pad;
-  t.b_row0 = b0;
-  t.C = W_;
-  t.cm = cm;
-  t.cn = cn;
-  t.alpha = alpha;
-  t.m_major = m_major ? 1 : 0;
-  t.err = err_;
-  t.sps = 1;
-  t.group = 1;
-  t.chunk = emu ? kFixedChunk : 4;
-  t.fold = emu ? kFixedFold : 0;
-  // fewer output tiles than SMs (the last batches): split K over CTAs
-  const int64_t tiles = (t.Mpad / kTcBM) * (t.Npad / t.bn), kblocks = t.Kpad / kTcBK;
-  const int64_t sms = num_sms();
-  if (tiles < sms && kblocks >= 4) {
-    int64_t ks = std::min<int64_t>((sms + tiles - 1) / tiles, kblocks / 2);
-    if (ks > 1) {
-      const int64_t kbps = (kblocks + ks - 1) / ks;
-      ks = (kblocks + kbps - 1) / kbps;
-      const size_t need = static_cast<size_t>(ks) * t.Mpad * t.Npad;
-      if (need > partk_elems_) throw Error(GBCC_ERR_STATE, "(T): K-split workspace too small");
-      t.ksplit = static_cast<int>(ks);
-      t.kb_per_split = static_cast<int>(kbps);
-      t.partial = partk_;
-    }
-  }
-  auto launch = [&](double b) {
-    t.beta = b;
-    if (!launch_gemm_tc(t, st_)) throw Error(GBCC_ERR_CUDA, "(T): tcgen05 GEMM launch rejected");
-    if (t.ksplit > 1)
-      launch_splitk_reduce(M, N, t.ksplit, partk_, t.Mpad, t.Npad, W_, cm, cn, alpha, b, st_);
-  };
-  if (!emu) {
-    t.npairs = 0;
-    for (int p = 0; p < slices_; ++p)
-      for (int q = 0; q < slices_; ++q)
-        if (p + q < slices_) {
-          t.pa[t.npairs] = p;
-          t.pb[t.npairs] = q;
-          ++t.npairs;
-        }
-    launch(beta);
-    return;
-  }
-  for (int w = slices_ - 1; w >= 0; --w) {
-    t.npairs = fixed_class_pairs(slices_, w, t.pa, t.pb);
-    launch(w == slices_ - 1 ? beta : 1.0);
-  }
+  GemmF64Args f{};
+  f.M = M;
+  f.N = N;
+  f.K = A.K;
+  f.A = A.f64 + a0 * A.K;
+  f.lda = A.K;
+  f.B = B.f64 + b0 * B.K;
+  f.ldb = B.K;
+  f.C = W_;
+  f.cm = cm;
+  f.cn = cn;
+  f.alpha = 1.0;
+  f.beta = beta;
+  f.m_major = m_major ? 1 : 0;
+  launch_gemm_f64(f, st_);
 }
 
 double Triples::run() {
@@ -429,16 +324,10 @@ double Triples::run() {
   const int64_t* cn5 = r_table(v);
   const int64_t* cn6 = r_table(v2);
 
-  // K-split workspace: a split happens only with fewer output tiles than
-  // SMs, ks <= ceil(SMs / tiles), so ks Mpad Npad < 2 SMs x one 128 x 256 tile
-  if (slices_ > 0) {
-    partk_elems_ = static_cast<size_t>(num_sms()) * 2 * kTcBM * 256;
-    partk_ = static_cast<double*>(alloc(partk_elems_ * sizeof(double)));
-  }
   // triplets per batch: all k >= j, unless their slice of t3 would pass
   // 8 GB (then chunks of k).  Chunks small enough to keep the slice in L2
-  // measured slower (the batches' GEMMs shrink and multiply: (H2O)10 mixed
-  // 18 s -> 28 s), so chunking only bounds memory.
+  // measured slower (the batches' GEMMs shrink and multiply), so chunking only
+  // bounds memory.
   int64_t kc = std::max<int64_t>(1, std::min<int64_t>(o, (static_cast<int64_t>(8) << 30) / (v3 * 8)));
   if (g_triples_chunk > 0) kc = std::min<int64_t>(o, g_triples_chunk);
   {
@@ -475,12 +364,8 @@ double Triples::run() {
         gemm(At, static_cast<int64_t>(k0) * v2, nk * v2, B2, pij, v, cm6, cn6, true, 1.0);
         const dim3 grid(static_cast<unsigned>(v), static_cast<unsigned>(nk));
         double* part = partial + slot * o * v + static_cast<int64_t>(k0 - j) * v;
-        if (prec_ == GBCC_PREC_MIXED)
-          triples_energy_kernel<float><<<grid, kThreads, 0, st_>>>(W_, o, v, i, j, k0, nk, in_.Gijab, in_.t1,
-                                                                    in_.eps_o, in_.eps_v, part);
-        else
-          triples_energy_kernel<double><<<grid, kThreads, 0, st_>>>(W_, o, v, i, j, k0, nk, in_.Gijab, in_.t1,
-                                                                     in_.eps_o, in_.eps_v, part);
+        triples_energy_kernel<<<grid, kThreads, 0, st_>>>(W_, o, v, i, j, k0, nk, in_.Gijab, in_.t1, in_.eps_o,
+                                                          in_.eps_v, part);
       }
     }
   }
@@ -492,10 +377,376 @@ double Triples::run() {
   return e;
 }
 
+// ---------------------------------------------------------------------------
+// tensor cores
+
+struct PackArgs {
+  int kind;                 // 0: A rows (x,p,q), 1: At rows (x,q,p), 2: B rows (y,z,c)
+  int64_t o, v, rows, K, kblocks;
+  const double* Giabc;
+  const double* Gijka;
+  const double* t2;
+  __nv_bfloat16* out;       // [slices][kblocks][rows][64]
+};
+
+// A block packs 32 rows: a thread takes 8 K elements of a row at a time, warp w
+// those at 8 w of each k-block, and stores 16 bytes a slice (the 8 warps fill
+// whole 128-byte lines).  Six slices need the row's largest exponent first.
+template <int SL>
+__global__ void __launch_bounds__(kThreads) triples_pack_kernel(PackArgs g) {
+  __shared__ unsigned ex[8][32];
+  const int lane = threadIdx.x % 32, w = threadIdx.x / 32;
+  const int64_t r = static_cast<int64_t>(blockIdx.x) * 32 + lane, v = g.v, o = g.o;
+  const double *s1 = nullptr, *s2 = nullptr;
+  int64_t st1 = 0, st2 = 0;
+  double coef = 1.0;
+  const bool in = r < g.rows;
+  if (in && g.kind < 2) {
+    const int64_t x = r / (v * v), rem = r - x * v * v, hi = rem / v, lo = rem - hi * v;
+    const int64_t pq = g.kind == 0 ? rem : lo * v + hi;
+    s1 = g.Giabc + x * v * v * v + pq;
+    st1 = v * v;
+    s2 = g.t2 + pq * o * o + x * o;
+    st2 = 1;
+    coef = -1.0;
+  } else if (in) {
+    const int64_t yz = r / v, c = r - yz * v;
+    s1 = g.t2 + c * o * o + yz;
+    st1 = v * o * o;
+    s2 = g.Gijka + yz * o * v + c;
+    st2 = v;
+  }
+  auto load8 = [&](int64_t k0, double x[8]) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int64_t k = k0 + j;
+      x[j] = !in || k >= g.K ? 0.0 : (k < v ? s1[k * st1] : flip_sign(s2[(k - v) * st2], coef < 0.0));
+    }
+  };
+  unsigned eb = 0;
+  if constexpr (SL != 3) {
+    for (int64_t kb = 0; kb < g.kblocks; ++kb) {
+      double x[8];
+      load8(kb * 64 + w * 8, x);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) eb = max(eb, exp_field(x[j]));
+    }
+    ex[w][lane] = eb;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) eb = max(eb, ex[q][lane]);
+  }
+  if (!in) return;
+  const int64_t slice = g.kblocks * g.rows * 64;
+  for (int64_t kb = 0; kb < g.kblocks; ++kb) {
+    double x[8];
+    load8(kb * 64 + w * 8, x);
+    unsigned short b[8][SL == 3 ? 3 : kFixedSlices];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if constexpr (SL == 3) split_bits(x[j], b[j], 3);
+      else fixed_split(x[j], eb, kFixedSlices, b[j]);
+    }
+    __nv_bfloat16* out = g.out + (kb * g.rows + r) * 64 + w * 8;
+#pragma unroll
+    for (int s = 0; s < SL; ++s) {
+      uint4 u;
+      u.x = b[0][s] | (static_cast<unsigned>(b[1][s]) << 16);
+      u.y = b[2][s] | (static_cast<unsigned>(b[3][s]) << 16);
+      u.z = b[4][s] | (static_cast<unsigned>(b[5][s]) << 16);
+      u.w = b[6][s] | (static_cast<unsigned>(b[7][s]) << 16);
+      *reinterpret_cast<uint4*>(out + s * slice) = u;
+    }
+  }
+}
+
+// orderings of three things (the even ones first), and for ordering m = (x,y,z)
+// the ordering (x,z,y) and the ordering (y,z,x)
+__device__ constexpr int kPerm[6][3] = {{0, 1, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}, {0, 2, 1}, {1, 0, 2}};
+__device__ constexpr int kSwap[6] = {4, 5, 3, 2, 0, 1};
+__device__ constexpr int kCycle[6] = {1, 2, 0, 5, 3, 4};
+
+constexpr int kB = 8;                 // virtual block
+constexpr int kRowLd = 9, kSlabLd = 73;  // padded strides: reads along any index hit different banks
+constexpr int kCube = kB * kSlabLd;
+
+template <typename R>
+struct EnergySmem {
+  double W[3][6][kCube];              // float2 (three slices) or double words
+  R G[3][9][kB * kRowLd];             // <ij|, <jk|, <ik| over ordered block pairs
+  R t1[3][3][kB];                     // t1 of i, j, k over the blocks
+  R ev[3][kB];
+  double red[kThreads];
+};
+
+struct EnergyArgs {
+  int o, v;
+  const int4* triples;                // this batch's
+  const unsigned* blocks;             // block triples A <= B <= C, 10 bits each
+  int nblocks;
+  const double* W;                    // [triple][3][v][v][v]
+  const double* Gijab;
+  const double* t1;
+  const double* eps_o;
+  const double* eps_v;
+  double* partial;                    // [triple][gridDim.x]
+};
+
+// hi + lo += x (TwoSum), for sums of many FP32 terms
+__device__ __forceinline__ void add_ff(float& hi, float& lo, float x) {
+  const float s = __fadd_rn(hi, x), b = __fsub_rn(s, hi);
+  lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b)));
+  hi = s;
+}
+
+__device__ __forceinline__ void copy8_async(double* dst, const double* src, bool in) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst)), n = in ? 8u : 0u;  // 0 source bytes: zeros
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+
+// Block (bx, t): the block triples bx, bx + gridDim.x, ... of triplet t.  R: the
+// arithmetic of the terms (double for FP64_TC; float for MIXED, whose products
+// carry ~1e-6, with W and the sums as float-float pairs).
+//
+// Bound by instructions and by the latency of one block triple's loads (two
+// blocks of 96 KB an SM), not by L2: so the 18 cubes come by asynchronous copies,
+// all in flight at once, and a thread keeps one (a, b) for two values of c --
+// every cube of ordering m is read at F[m], the same six offsets for all three
+// arrays.
+template <typename R>
+__global__ void __launch_bounds__(kThreads, 2) triples_blocks_kernel(EnergyArgs g) {
+  extern __shared__ double smem_d[];
+  auto& S = *reinterpret_cast<EnergySmem<R>*>(smem_d);
+  constexpr bool kPair = sizeof(R) == 4;
+  const int tid = threadIdx.x;
+  const int v = g.v, o = g.o, v2 = v * v;
+  const int64_t v3 = static_cast<int64_t>(v2) * v;
+  const int4 ijk = g.triples[blockIdx.y];
+  const int i = ijk.x, j = ijk.y, k = ijk.z;
+  const double mult = (i < j && j < k) ? 6.0 : ((i == j && j == k) ? 1.0 : 3.0);
+  const double* __restrict__ W = g.W + static_cast<int64_t>(blockIdx.y) * 3 * v3;
+  const double* __restrict__ Gp[3] = {g.Gijab + (static_cast<int64_t>(i) * o + j) * v2,
+                                      g.Gijab + (static_cast<int64_t>(j) * o + k) * v2,
+                                      g.Gijab + (static_cast<int64_t>(i) * o + k) * v2};
+  const R eijk = static_cast<R>(g.eps_o[i] + g.eps_o[j] + g.eps_o[k]);
+  const int l2 = tid & 7, l1 = (tid >> 3) & 7, l0 = tid >> 6;  // copies: l0 and l0 + 4
+  const int la = l1, lb = l2, lc0 = 2 * l0;                    // terms: (a, b) and c0, c0 + 1
+  double acc = 0.0;
+  float ahi = 0.f, alo = 0.f;
+  for (int bt = blockIdx.x; bt < g.nblocks; bt += gridDim.x) {
+    const unsigned code = g.blocks[bt];
+    const int A = static_cast<int>(code & 1023u) * kB, B = static_cast<int>((code >> 10) & 1023u) * kB,
+              C = static_cast<int>(code >> 20) * kB;
+    auto start = [&](int q) { return q == 0 ? A : (q == 1 ? B : C); };
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      const int gf = start(kPerm[m][1]) + l1, gr = start(kPerm[m][2]) + l2;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int s = l0 + 4 * h, gs = start(kPerm[m][0]) + s;
+        const bool in = gs < v && gf < v && gr < v;  // zeros past v
+        const double* src = W + (in ? static_cast<int64_t>(gs * v + gf) * v + gr : 0);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) copy8_async(&S.W[p][m][s * kSlabLd + l1 * kRowLd + l2], src + p * v3, in);
+      }
+    }
+    // <ij|, <jk|, <ik| over the six ordered block pairs: 64 elements by 64 threads each
+#pragma unroll
+    for (int u = 0; u < 5; ++u) {
+      const int q = l0 + 4 * u;  // pair (q % 6) of array (q / 6)
+      if (q < 18) {
+        const int p = q / 6, m = q % 6;
+        const int bs = m < 2 ? 0 : (m < 4 ? 1 : 2), bf = m == 0 ? 1 : (m == 1 ? 2 : (m == 2 ? 0 : (m == 3 ? 2 : (m == 4 ? 0 : 1))));
+        const int gs = start(bs) + l1, gf = start(bf) + l2;
+        const double* gp = p == 0 ? Gp[0] : (p == 1 ? Gp[1] : Gp[2]);
+        S.G[p][bs * 3 + bf][l1 * kRowLd + l2] = (gs < v && gf < v) ? static_cast<R>(gp[gs * v + gf]) : R(0);
+      }
+    }
+    if (tid < 72) {
+      const int x = tid & 7, blk = (tid >> 3) % 3, p = (tid >> 3) / 3;
+      const int gx = start(blk) + x, occ = p == 0 ? i : (p == 1 ? j : k);
+      S.t1[p][blk][x] = gx < v ? static_cast<R>(g.t1[gx * o + occ]) : R(0);
+      if (p == 0) S.ev[blk][x] = gx < v ? static_cast<R>(g.eps_v[gx]) : R(0);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const int a = A + la, b = B + lb;
+    if (a > b) continue;
+    // offsets of (l[P0], l[P1], l[P2]) in a cube, c = c0, and what one more c adds
+    constexpr int kStep[6] = {1, kRowLd, kSlabLd, kSlabLd, kRowLd, 1};
+    int F[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      auto l = [&](int q) { return q == 0 ? la : (q == 1 ? lb : lc0); };
+      F[m] = l(kPerm[m][0]) * kSlabLd + l(kPerm[m][1]) * kRowLd + l(kPerm[m][2]);
+    }
+    const R eab = eijk - S.ev[0][la] - S.ev[1][lb];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int lc = lc0 + u, c = C + lc;
+      if (b > c || c >= v) continue;
+      R w[6], vv[6];
+#pragma unroll
+      for (int m = 0; m < 6; ++m) {
+        const double w0 = S.W[0][m][F[m] + u * kStep[m]];
+        const double w1 = S.W[1][kSwap[m]][F[kSwap[m]] + u * kStep[kSwap[m]]];
+        const double w2 = S.W[2][kCycle[m]][F[kCycle[m]] + u * kStep[kCycle[m]]];
+        if constexpr (kPair) {
+          // words of (hi, lo) floats
+          const float2 f0 = *reinterpret_cast<const float2*>(&w0), f1 = *reinterpret_cast<const float2*>(&w1),
+                       f2 = *reinterpret_cast<const float2*>(&w2);
+          float hi = f0.x, lo = f0.y;
+          add_ff(hi, lo, f1.x);
+          add_ff(hi, lo, f2.x);
+          w[m] = hi + (lo + (f1.y + f2.y));
+        } else {
+          w[m] = w0 + w1 + w2;
+        }
+        auto l = [&](int q) { return q == 0 ? la : (q == 1 ? lb : lc); };
+        const int px = kPerm[m][0], py = kPerm[m][1], pz = kPerm[m][2];
+        const int x = l(px), y = l(py), z = l(pz);
+        vv[m] = S.G[0][px * 3 + py][x * kRowLd + y] * S.t1[2][pz][z] + S.G[1][py * 3 + pz][y * kRowLd + z] * S.t1[0][px][x] +
+                S.G[2][px * 3 + pz][x * kRowLd + z] * S.t1[1][py][y];
+      }
+      const R even = w[0] + w[1] + w[2], odd = w[3] + w[4] + w[5];
+      // 4 t3(abc) + the two cyclic orderings - 2 the three others
+      R sum[6];
+#pragma unroll
+      for (int m = 0; m < 6; ++m)
+        sum[m] = (w[m] + vv[m]) * (R(3) * w[m] + (m < 3 ? even - R(2) * odd : odd - R(2) * even));
+      // a set with equal members has its orderings counted that many times
+      const R share = a == b ? (b == c ? R(1) / R(6) : R(0.5)) : (b == c ? R(0.5) : R(1));
+      const R f = share / (eab - S.ev[2][lc]);
+      const R term = (((sum[0] + sum[1]) + sum[2]) + ((sum[3] + sum[4]) + sum[5])) * f;
+      if constexpr (kPair) add_ff(ahi, alo, term);
+      else acc += term;
+    }
+  }
+  if constexpr (kPair) acc = static_cast<double>(ahi) + static_cast<double>(alo);
+  __syncthreads();
+  const double s = block_sum_det(acc, S.red);
+  if (tid == 0) g.partial[static_cast<int64_t>(blockIdx.y) * gridDim.x + blockIdx.x] = mult * s;
+}
+
+// out[blockIdx.x] = sum of its share of x (strided; fixed order)
+__global__ void __launch_bounds__(kThreads) sum_blocks_kernel(const double* __restrict__ x, int64_t n,
+                                                             double* __restrict__ out) {
+  __shared__ double sh[kThreads];
+  double acc = 0.0;
+  for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < n;
+       e += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    acc += x[e];
+  const double s = block_sum_det(acc, sh);
+  if (threadIdx.x == 0) out[blockIdx.x] = s;
+}
+
+template <typename R>
+void launch_blocks(const EnergyArgs& g, dim3 grid, cudaStream_t st) {
+  static const bool attr = cudaFuncSetAttribute(triples_blocks_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                sizeof(EnergySmem<R>)) == cudaSuccess;
+  if (!attr) throw Error(GBCC_ERR_CUDA, "(T): energy kernel shared memory");
+  triples_blocks_kernel<R><<<grid, kThreads, sizeof(EnergySmem<R>), st>>>(g);
+}
+
+double triples_tc(const TriplesInputs& in, int precision, cudaStream_t st, int* err) {
+  const int64_t o = in.o, v = in.v, v3 = v * v * v, K = v + o, kblocks = (K + 63) / 64;
+  const int slices = precision == GBCC_PREC_MIXED ? 3 : kFixedSlices;
+  const int64_t rowsA = o * v * v, rowsB = o * o * v;
+  const int64_t nvb = (v + kB - 1) / kB;
+  if (nvb > 1023) throw Error(GBCC_ERR_STATE, "(T): too many virtual orbitals");
+  std::vector<int4> tr;
+  for (int i = 0; i < o; ++i)
+    for (int j = i; j < o; ++j)
+      for (int k = j; k < o; ++k) tr.push_back(make_int4(i, j, k, 0));
+  std::vector<unsigned> bl;
+  for (unsigned a = 0; a < nvb; ++a)
+    for (unsigned b = a; b < nvb; ++b)
+      for (unsigned c = b; c < nvb; ++c) bl.push_back(a | (b << 10) | (c << 20));
+  const int64_t ntr = static_cast<int64_t>(tr.size()), nbl = static_cast<int64_t>(bl.size());
+  int64_t batch = std::max<int64_t>(1, std::min<int64_t>(ntr, (int64_t{96} << 20) / (3 * v3 * 8)));
+  batch = std::min<int64_t>(batch, 32768);  // the energy grid's second dimension
+  if (g_triples_chunk > 0) batch = std::min(batch, g_triples_chunk);
+  // energy blocks per triplet: a few waves of the chip per batch, 32 MB of partial sums
+  const int64_t gx = std::min(nbl, std::max<int64_t>(1, std::min<int64_t>(std::max<int64_t>((2432 + batch - 1) / batch, 16),
+                                                                         (int64_t{1} << 22) / ntr)));
+  constexpr int kSums = 152;
+  size_t total = 0;
+  auto part = [&](size_t bytes) {
+    const size_t at = total;
+    total += (bytes + 1023) / 1024 * 1024;
+    return at;
+  };
+  const size_t elems_a = static_cast<size_t>(slices) * kblocks * rowsA * 64, elems_b = static_cast<size_t>(slices) * kblocks * rowsB * 64;
+  const size_t oA = part(elems_a * 2), oA2 = part(elems_a * 2), oB = part(elems_b * 2), oW = part(static_cast<size_t>(batch) * 3 * v3 * 8),
+               oT = part(ntr * sizeof(int4)), oBl = part(nbl * sizeof(unsigned)), oP = part(static_cast<size_t>(ntr) * gx * 8),
+               oS = part((kSums + 1) * 8);
+  struct Owned {
+    char* p;
+    ~Owned() { dev_free(p); }
+  } ws{static_cast<char*>(dev_alloc(total))};
+  auto* A = reinterpret_cast<__nv_bfloat16*>(ws.p + oA);
+  auto* A2 = reinterpret_cast<__nv_bfloat16*>(ws.p + oA2);
+  auto* B = reinterpret_cast<__nv_bfloat16*>(ws.p + oB);
+  auto* W = reinterpret_cast<double*>(ws.p + oW);
+  auto* d_tr = reinterpret_cast<int4*>(ws.p + oT);
+  auto* d_bl = reinterpret_cast<unsigned*>(ws.p + oBl);
+  auto* partial = reinterpret_cast<double*>(ws.p + oP);
+  auto* sums = reinterpret_cast<double*>(ws.p + oS);
+  GBCC_CK(cudaMemcpyAsync(d_tr, tr.data(), ntr * sizeof(int4), cudaMemcpyHostToDevice, st));
+  GBCC_CK(cudaMemcpyAsync(d_bl, bl.data(), nbl * sizeof(unsigned), cudaMemcpyHostToDevice, st));
+  for (int kind = 0; kind < 3; ++kind) {
+    PackArgs p{kind, o, v, kind == 2 ? rowsB : rowsA, K, kblocks, in.Giabc, in.Gijka, in.t2,
+               kind == 0 ? A : (kind == 1 ? A2 : B)};
+    const unsigned grid = static_cast<unsigned>((p.rows + 31) / 32);
+    if (slices == 3) triples_pack_kernel<3><<<grid, kThreads, 0, st>>>(p);
+    else triples_pack_kernel<kFixedSlices><<<grid, kThreads, 0, st>>>(p);
+  }
+  GemmMultiArgs g{};
+  g.K = K;
+  g.kblocks = kblocks;
+  g.A = A;
+  g.A2 = A2;
+  g.B = B;
+  g.a_rows = rowsA;
+  g.o = static_cast<int>(o);
+  g.v = static_cast<int>(v);
+  g.W = W;
+  g.err = err;
+  EnergyArgs e{};
+  e.o = static_cast<int>(o);
+  e.v = static_cast<int>(v);
+  e.blocks = d_bl;
+  e.nblocks = static_cast<int>(nbl);
+  e.W = W;
+  e.Gijab = in.Gijab;
+  e.t1 = in.t1;
+  e.eps_o = in.eps_o;
+  e.eps_v = in.eps_v;
+  for (int64_t t0 = 0; t0 < ntr; t0 += batch) {
+    const int n = static_cast<int>(std::min(batch, ntr - t0));
+    g.triples = d_tr + t0;
+    if (!launch_gemm_triples(g, slices, n, st)) throw Error(GBCC_ERR_CUDA, "(T): tcgen05 launch rejected");
+    e.triples = d_tr + t0;
+    e.partial = partial + t0 * gx;
+    const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(n));
+    if (slices == 3) launch_blocks<float>(e, grid, st);
+    else launch_blocks<double>(e, grid, st);
+  }
+  sum_blocks_kernel<<<kSums, kThreads, 0, st>>>(partial, ntr * gx, sums);
+  sum_kernel<<<1, kThreads, 0, st>>>(sums, kSums, 1.0 / 3.0, sums + kSums);
+  double out = 0.0;
+  GBCC_CK(cudaMemcpyAsync(&out, sums + kSums, sizeof(double), cudaMemcpyDeviceToHost, st));
+  GBCC_CK(cudaStreamSynchronize(st));
+  GBCC_CK(cudaGetLastError());
+  return out;
+}
+
 }  // namespace
 
 double triples_energy(const TriplesInputs& in, int precision, cudaStream_t st, int* err) {
-  Triples t(in, precision, st, err);
+  if (precision != GBCC_PREC_FP64) return triples_tc(in, precision, st, err);
+  Triples t(in, st);
   return t.run();
 }
 
