@@ -1192,8 +1192,12 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
           ks = 1;
         }
         if (ks > 1) wspart_ = std::max(wspart_, static_cast<size_t>(ks * p.P[0].rows_pad * npad));
-        // both slices of a k-block per stage: two slices, tiles up to 192 wide
-        const int nsps = (slices == 2 && bns[c] >= 64 && bns[c] <= 192) ? 2 : 1;
+        // both slices of a k-block per stage: two slices, tiles up to 192 wide;
+        // every slice per stage on CTA pairs: 256 x 256 tiles, where the padding
+        // of M to 256 is small
+        const int nsps = ((slices == 2 && bns[c] >= 64 && bns[c] <= 192) || (slices > 1 && bns[c] == 256 && p.M >= 512))
+                             ? 2
+                             : 1;
         // bands of 8 M tiles: many N tiles per row and enough rows
         const bool banded = npad / bns[c] >= 8 && p.P[0].rows_pad / kTcBM >= 16;
         for (int sp = 1; sp <= nsps; ++sp) {

@@ -699,6 +699,11 @@ bool launch_gemm_tc(const GemmTcArgs& g, cudaStream_t st) {
       default: return false;
     }
   }
+  if (g.sps == 2 && g.bn == 256) {
+    GemmTcArgs h = g;
+    h.chunk = g.chunk > 0 ? g.chunk : 4;
+    return launch_gemm_pair(h, st);
+  }
   if (g.sps == 2) {
     // both slices per stage: two slices, every pair (p, q) with p, q < 2
     if (g.a_slices != 2 || g.b_slices != 2) return false;

@@ -233,7 +233,8 @@ struct GemmTcArgs {
   // hold more rows than the launch covers (padded for every candidate tile)
   int64_t a_rows, b_rows;
   // slices per pipeline stage: 0 or 1, one (A, B) slice pair per stage; 2, both
-  // slices of A and B of a k-block per stage (2 slices, bn 64 / 128 / 192)
+  // slices of A and B of a k-block per stage (2 slices, bn 64 / 128 / 192), or,
+  // with bn 256, every slice per stage on CTA pairs (gemm_pair.cu)
   int sps;
   // > 1: output tiles run in bands of `group` M tiles, N outer within a band
   // (CTAs working at the same time then share fewer, wider operand panels in
@@ -258,6 +259,8 @@ int num_sms();
 
 // Returns false if the tensor maps could not be encoded (bad alignment / size).
 bool launch_gemm_tc(const GemmTcArgs& g, cudaStream_t st);
+// its 256 x 256 tiles on CTA pairs (gemm_pair.cu); launch_gemm_tc forwards to it
+bool launch_gemm_pair(const GemmTcArgs& g, cudaStream_t st);
 // N tile for a GEMM of N columns; allow256: 256- or 192-wide tiles (faster,
 // FP32 register accumulation of the chunks) for N >= 256
 int gemm_tc_pick_bn(int64_t N, bool allow256);
