@@ -215,6 +215,19 @@ void residual_program(Engine& E, const CcsdTensors& S) {
   double *r1d = r1.d, *r2d = r2.d, *tmp2 = S.tmp2->d;
   const bool direct = S.nao > 0;
 
+  // Four lanes (engine.h), so that small systems, whose time is launches and
+  // dependent kernels that fill a few SMs, run about as long as the longest
+  // chain, and large ones fill the last waves of one product with the next:
+  //   0  P, r2u, the assembly
+  //   1  K, g_ac, tmp
+  //   2  the pair ladders (integral-direct: the U intermediate)
+  //   3  tmp2, the small products, r1
+  // Mixed residual at o = 13, v = 57: 1.14 -> 0.75 ms; at o = 30, v = 120: 5.17 ->
+  // 4.69; at o = 50, v = 190 (every product fills the chip): 37.3 -> 37.8; FP64
+  // solve at o = 5, v = 19: 5.5 -> 3.65 ms.
+
+  E.lane(2);
+  int tmp2_done = -1;
   if (direct) {
     // integral-direct (ccsd.h:581-603): tau_AO(q,s,i,j) = Ca(q,a) tau(a,b,i,j) Ca(s,b)
     // and u(p,r,i,j) = (pq|rs) tau_AO(q,s,i,j) over AO pairs p <= r, q <= s
@@ -235,16 +248,27 @@ void residual_program(Engine& E, const CcsdTensors& S) {
              1);
     E.contract(ix(*S.U2, "krij"), 0.0, 1.0, {{1.0, ix(Ci, "pk")}}, {{1.0, ix(u, "prij")}}, O);
     E.contract(ix(*S.tmp2, "kaij"), 0.0, 1.0, {{1.0, ix(*S.U2, "krij")}}, {{1.0, ix(Ca, "ra")}}, O);
+    tmp2_done = E.mark(2);
+    E.contract(ix(*S.U1, "arij"), 0.0, 1.0, {{1.0, ix(*S.Ca, "pa")}}, {{1.0, ix(u, "prij")}}, O);
   } else {
-    // tmp2(k,a,i,j) = Giabc(k,a,c,d) tau(c,d,i,j) (ccsd_r1_r2.h:277) as sums over
-    // c <= d of the pair-(anti)symmetric combinations (kernels.cu), unpacked
     double *taup = S.taup->d, *taum = S.taum->d, *Xp = S.Xp->d, *Xm = S.Xm->d;
     E.custom([=](cudaStream_t st) { launch_tau_pm(o, v, tau_d, taup, taum, st); }, 1);
+    const int tau_pm_done = E.mark(2);
+    E.lane(3);
+    E.wait(3, tau_pm_done);
+    // tmp2(k,a,i,j) = Giabc(k,a,c,d) tau(c,d,i,j) (ccsd_r1_r2.h:277) as sums over
+    // c <= d of the pair-(anti)symmetric combinations (kernels.cu), unpacked
     E.contract(ix(*S.Xp, "RS"), 0.0, 1.0, {{1.0, ix(*S.Gip, "RQ")}}, {{1.0, ix(*S.taup, "QS")}}, R);
     if (minus) E.contract(ix(*S.Xm, "RZ"), 0.0, 1.0, {{1.0, ix(*S.Gim, "RY")}}, {{1.0, ix(*S.taum, "YZ")}}, R);
     E.custom([=](cudaStream_t st) { launch_pair_unpack(o, v, o, false, Xp, minus ? Xm : nullptr, 0.0, tmp2, st); },
              1);
   }
+
+  // Y1, Y2 of the permutation part of r2 (:206-212)
+  E.lane(3);
+  E.contract(ix(*S.Y1, "kbij"), 0.0, 1.0, {{1.0, ix(Giajb, "kbic")}}, {{1.0, ix(t1, "cj")}}, O);
+  E.contract(ix(*S.Y2, "ikaj"), 0.0, 1.0, {{1.0, ix(Gijab, "ikac")}}, {{1.0, ix(t1, "cj")}}, O);
+  const int y_done = E.mark(3);
 
   // ----- R1 (ccsd_r1_r2.h:70-124) -----
   // r1(a,i) = Fia(i,a) - 2 (Fia(k,c) t1(c,i)) t1(a,k)
@@ -262,6 +286,13 @@ void residual_program(Engine& E, const CcsdTensors& S) {
   E.contract(ix(*S.FIJ, "ki"), 1.0, 1.0, {{2.0, ix(Gijab, "klab")}, {-1.0, ix(Gijab, "lkab")}},
              {{1.0, ix(tau, "abil")}}, O);
   E.contract(ix(r1, "ai"), 1.0, -1.0, {{1.0, ix(t1, "ak")}}, {{1.0, ix(*S.FIJ, "ki")}}, O);
+  const int fock_done = E.mark(3);
+  // g_ki = F_OO(FIJ, Fia, gbar_ijka, t1), gbar_ijka(k,l,i,c) = 2 Gijka(k,l,i,c) - Gijka(l,k,i,c)
+  E.assign(ix(*S.gki, "ki"), 0.0, {f1(1.0, ix(*S.FIJ, "ki"))});
+  E.contract(ix(*S.gki, "ki"), 1.0, 1.0, {{1.0, ix(Fia, "kc")}}, {{1.0, ix(t1, "ci")}}, O);
+  E.contract(ix(*S.gki, "ki"), 1.0, 1.0, {{2.0, ix(Gijka, "klic")}, {-1.0, ix(Gijka, "lkic")}},
+             {{1.0, ix(t1, "cl")}}, O);
+  const int gki_done = E.mark(3);
   // h_kc = F_ov(Fia, gbar, t1); r1 += h_kc(k,c) (2 t2(c,a,k,i) - t2(c,a,i,k) + t1(c,i) t1(a,k))
   E.assign(ix(*S.hkc, "kc"), 0.0, {f1(1.0, ix(Fia, "kc"))});
   E.contract(ix(*S.hkc, "kc"), 1.0, 1.0, {{2.0, ix(Gijab, "klcd")}, {-1.0, ix(Gijab, "lkcd")}},
@@ -273,6 +304,7 @@ void residual_program(Engine& E, const CcsdTensors& S) {
   // r1 += (2 Gijab(k,i,c,a) - Giajb(k,a,i,c)) t1(c,k)
   E.contract(ix(r1, "ai"), 1.0, 1.0, {{2.0, ix(Gijab, "kica")}, {-1.0, ix(Giajb, "kaic")}},
              {{1.0, ix(t1, "ck")}}, O);
+  if (direct) E.wait(3, tmp2_done);
   // r1 += (2 Giabc(k,a,c,d) - Giabc(k,a,d,c)) tau(c,d,k,i) (:111-114) = 2 tmp2(k,a,k,i) - tmp2(k,a,i,k)
   E.custom([=](cudaStream_t st) { launch_r1_from_tmp2(o, v, tmp2, r1d, st); }, 1);
   // r1 -= (2 Gijka(l,k,i,c) - Gijka(k,l,i,c)) tau(c,a,k,l), read through
@@ -295,6 +327,7 @@ void residual_program(Engine& E, const CcsdTensors& S) {
   //   -2 G_cd T + (2 G_cd - G_dc) t2(a,d,i,l) + G_dc T = (2 G_cd - G_dc) (t2(a,d,i,l) - T)
   // (G_cd = Gijab(k,l,c,d), G_dc = Gijab(k,l,d,c), summed over l, d) is one
   // contraction instead of j's two and a share of k's
+  E.lane(1);
   const std::vector<Lin> T = {{1.0, ix(tau, "dail")}, {-0.5, ix(t2, "dail")}};
   E.contract(ix(K, "kaic"), 0.0, -1.0, {{1.0, ix(Gijab, "kldc")}}, T, R);
   E.assign(ix(K, "kaic"), 1.0, {f1(1.0, ix(Giajb, "kaic"))});
@@ -303,6 +336,7 @@ void residual_program(Engine& E, const CcsdTensors& S) {
   double *dK = S.diagK->d, *dP = S.diagP->d;
   E.custom([=](cudaStream_t st) { launch_diag_snapshot(o, v, 0, Kd, dK, st); }, 1);
   E.contract(ix(K, "kaic"), 1.0, 1.0, {{1.0, ix(Giabc, "kadc")}}, {{1.0, ix(t1, "di")}}, O);
+  E.lane(0);
   E.contract(ix(P, "akic"), 0.0, 1.0, {{2.0, ix(Gijab, "klcd")}, {-1.0, ix(Gijab, "kldc")}},
              {{1.0, ix(t2, "adil")}, {0.5, ix(t2, "dail")}, {-1.0, ix(tau, "dail")}}, R);
   // the rest of 2 j - k: 2 Gijab(i,k,a,c) - Giajb(k,a,i,c) - (2 Gijka(l,k,i,c) -
@@ -313,23 +347,10 @@ void residual_program(Engine& E, const CcsdTensors& S) {
   E.custom([=](cudaStream_t st) { launch_diag_snapshot(o, v, 1, Pd, dP, st); }, 1);
   E.contract(ix(P, "akic"), 1.0, 1.0, {{2.0, ix(Giabc, "kacd")}, {-1.0, ix(Giabc, "kadc")}},
              {{1.0, ix(t1, "di")}}, O);
-  // r2 += 0.5 (2 j(a,k,i,c) - k(k,a,i,c)) (2 t2(c,b,k,j) - t2(b,c,k,j))   (:251-252)
-  E.contract(ix(r2u, "abij"), 0.0, 0.5, {{1.0, ix(P, "akic")}}, {{2.0, ix(t2, "cbkj")}, {-1.0, ix(t2, "bckj")}},
-             R);
-  // permutation part (:206-212)
-  // r2u -= Y1(k,a,j,i) t1(b,k) [image of Y1(k,b,i,j) t1(a,k)] + Gijka(j,i,k,a) t1(b,k)
-  //        + Y2(i,k,a,j) t1(b,k) + tmp2(k,a,j,i) t1(b,k) [the ladder's t1 terms, :278-280]
-  E.contract(ix(r2u, "abij"), 1.0, 1.0, {{1.0, ix(Giabc, "icab")}}, {{1.0, ix(t1, "cj")}}, O);
-  E.contract(ix(*S.Y1, "kbij"), 0.0, 1.0, {{1.0, ix(Giajb, "kbic")}}, {{1.0, ix(t1, "cj")}}, O);
-  E.contract(ix(*S.Y2, "ikaj"), 0.0, 1.0, {{1.0, ix(Gijab, "ikac")}}, {{1.0, ix(t1, "cj")}}, O);
-  E.contract(ix(r2u, "abij"), 1.0, -1.0,
-             {{1.0, ix(*S.Y1, "kaji")}, {1.0, ix(Gijka, "jika")}, {1.0, ix(*S.Y2, "ikaj")}, {1.0, ix(*S.tmp2, "kaji")}},
-             {{1.0, ix(t1, "bk")}}, O);
-  // g_ki = F_OO(FIJ, Fia, gbar_ijka, t1), gbar_ijka(k,l,i,c) = 2 Gijka(k,l,i,c) - Gijka(l,k,i,c)
-  E.assign(ix(*S.gki, "ki"), 0.0, {f1(1.0, ix(*S.FIJ, "ki"))});
-  E.contract(ix(*S.gki, "ki"), 1.0, 1.0, {{1.0, ix(Fia, "kc")}}, {{1.0, ix(t1, "ci")}}, O);
-  E.contract(ix(*S.gki, "ki"), 1.0, 1.0, {{2.0, ix(Gijka, "klic")}, {-1.0, ix(Gijka, "lkic")}},
-             {{1.0, ix(t1, "cl")}}, O);
+  const int p_done = E.mark(0);
+  E.lane(1);
+  E.wait(1, p_done);
+  E.wait(1, fock_done);
   // g_ac = F_VV(FAB, Fia, gbar_iabc, t1), gbar_iabc(k,a,d,c) = 2 Giabc(k,a,d,c) - Giabc(k,a,c,d)
   // (the reference's 4-argument F_VV adds + Fia(k,c) t1(a,k); kept as written)
   E.assign(ix(*S.gac, "ac"), 0.0, {f1(1.0, ix(*S.FAB, "ac"))});
@@ -338,16 +359,33 @@ void residual_program(Engine& E, const CcsdTensors& S) {
   // (kernels.cu): no pass over Giabc of its own
   double* gacd = S.gac->d;
   E.custom([=](cudaStream_t st) { launch_gac_from_diagonals(o, v, Kd, Pd, dK, dP, gacd, st); }, 1);
-  // r2 += g_ac(a,c) t2(c,b,i,j) - g_ki(k,i) t2(a,b,k,j)
-  E.contract(ix(r2u, "abij"), 1.0, 1.0, {{1.0, ix(*S.gac, "ac")}}, {{1.0, ix(t2, "cbij")}}, O);
-  E.contract(ix(r2u, "abij"), 1.0, -1.0, {{1.0, ix(*S.gki, "ki")}}, {{1.0, ix(t2, "abkj")}}, O);
+  const int gac_done = E.mark(1);
   // tmp(a,b,i,j) = k(k,a,i,c) t2(c,b,j,k); r2 -= 0.5 tmp(a,b,i,j) + tmp(b,a,i,j)   (:254-256)
   // (t2(c,b,j,k) read as t2(b,c,k,j): its rows (b,j) then run along j in storage)
   E.contract(ix(*S.tmp, "abij"), 0.0, 1.0, {{1.0, ix(K, "kaic")}}, {{1.0, ix(t2, "bckj")}}, R);
+  E.lane(0);
+  // r2 += 0.5 (2 j(a,k,i,c) - k(k,a,i,c)) (2 t2(c,b,k,j) - t2(b,c,k,j))   (:251-252)
+  E.contract(ix(r2u, "abij"), 0.0, 0.5, {{1.0, ix(P, "akic")}}, {{2.0, ix(t2, "cbkj")}, {-1.0, ix(t2, "bckj")}},
+             R);
+  // permutation part (:206-212)
+  // r2u -= Y1(k,a,j,i) t1(b,k) [image of Y1(k,b,i,j) t1(a,k)] + Gijka(j,i,k,a) t1(b,k)
+  //        + Y2(i,k,a,j) t1(b,k) + tmp2(k,a,j,i) t1(b,k) [the ladder's t1 terms, :278-280]
+  E.contract(ix(r2u, "abij"), 1.0, 1.0, {{1.0, ix(Giabc, "icab")}}, {{1.0, ix(t1, "cj")}}, O);
+  E.wait(0, y_done);
+  if (direct) E.wait(0, tmp2_done);
+  E.contract(ix(r2u, "abij"), 1.0, -1.0,
+             {{1.0, ix(*S.Y1, "kaji")}, {1.0, ix(Gijka, "jika")}, {1.0, ix(*S.Y2, "ikaj")}, {1.0, ix(*S.tmp2, "kaji")}},
+             {{1.0, ix(t1, "bk")}}, O);
+  // r2 += g_ac(a,c) t2(c,b,i,j) - g_ki(k,i) t2(a,b,k,j)
+  E.wait(0, gki_done);
+  E.contract(ix(r2u, "abij"), 1.0, -1.0, {{1.0, ix(*S.gki, "ki")}}, {{1.0, ix(t2, "abkj")}}, O);
+  E.wait(0, gac_done);
+  E.contract(ix(r2u, "abij"), 1.0, 1.0, {{1.0, ix(*S.gac, "ac")}}, {{1.0, ix(t2, "cbij")}}, O);
   // r2(a,b,i,j) = r2u(a,b,i,j) + r2u(b,a,j,i) + Gijab(i,j,a,b)   (:260-262), with the
   // tmp terms, is added by the assembly pass below (g_abij(a,b,i,j) = Gijab(i,j,a,b),
   // stored in r2's order)
   const double *r2u_d = r2u.d, *tmp_d = S.tmp->d, *gab_d = S.g_abij->d;
+  E.lane(2);
   // hole-hole ladder: W_oooo (intermediates :182-193), r2 += W(k,l,i,j) tau(a,b,k,l)
   const Tensor& W = *S.W;
   E.assign(ix(W, "klij"), 0.0, {f1(1.0, ix(Gijkl, "klij"))});
@@ -356,11 +394,14 @@ void residual_program(Engine& E, const CcsdTensors& S) {
   if (direct) {
     E.contract(ix(W, "klij"), 1.0, 1.0, {{1.0, ix(Gijab, "klcd")}}, {{1.0, ix(tau, "cdij")}}, O);
     E.contract(ix(r2, "abij"), 0.0, 1.0, {{1.0, ix(W, "klij")}}, {{1.0, ix(tau, "abkl")}}, O);
+    const int w_done = E.mark(2);
+    E.lane(0);
+    E.wait(0, E.mark(1));
+    E.wait(0, w_done);
     E.custom([=](cudaStream_t st) { launch_r2_assemble(o, v, r2u_d, tmp_d, gab_d, nullptr, nullptr, true, r2d, st); },
              1);
     // integral-direct (:282-286): r2 += Ca(p,a) u(p,r,i,j) Ca(r,b); the T1 parts
     // (Ci u terms) are the tmp2 terms of r2u above
-    E.contract(ix(*S.U1, "arij"), 0.0, 1.0, {{1.0, ix(*S.Ca, "pa")}}, {{1.0, ix(*S.u, "prij")}}, O);
     E.contract(ix(r2, "abij"), 1.0, 1.0, {{1.0, ix(*S.U1, "arij")}}, {{1.0, ix(*S.Ca, "rb")}}, O);
     return;
   }
@@ -399,6 +440,10 @@ void residual_program(Engine& E, const CcsdTensors& S) {
   E.contract(ix(*S.Bp, "RS"), 1.0, 1.0, {{1.0, ix(*S.taup, "RP")}}, {{1.0, ix(*S.Wt, "PS")}}, O);
   if (minus) E.contract(ix(*S.Bm, "UZ"), 1.0, 1.0, {{1.0, ix(*S.taum, "UX")}}, {{1.0, ix(*S.Wm, "XZ")}}, O);
   // r2 = the symmetrised r2u and tmp terms, g_abij and both ladders' pair products
+  const int ladders_done = E.mark(2);
+  E.lane(0);
+  E.wait(0, E.mark(1));
+  E.wait(0, ladders_done);
   E.custom(
       [=](cudaStream_t st) { launch_r2_assemble(o, v, r2u_d, tmp_d, gab_d, Bp, minus ? Bm : nullptr, false, r2d, st); },
       1);

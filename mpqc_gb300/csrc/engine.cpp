@@ -221,6 +221,9 @@ struct OperandPlan {
   bool cache_first = false;  // packs into cache_buf
   bool cache_reuse = false;  // reads cache_buf packed by an earlier contraction
   __nv_bfloat16* cache_buf = nullptr;
+  int lane = 0;
+  cudaEvent_t packed_ev = nullptr;  // first use: recorded after the pack when another lane reads it
+  OperandPlan* first_use = nullptr;  // reuse in another lane: the operand to wait for
   // FP64_TC: fixed-point slices under per-row exponents (rows_pad words)
   bool fixed = false;
   unsigned* rowexp = nullptr;
@@ -273,11 +276,15 @@ struct Site {
   GemmPlan plan[3];  // by plan_index(precision)
   cudaEvent_t e0 = nullptr, e1 = nullptr, eg = nullptr;  // profiling: start, end, GEMM start
   bool has_gemm = false;
+  int lane = 0;
   std::string label;  // NVTX range name: the operation and its operands
   ~Site() {
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     if (eg) cudaEventDestroy(eg);
+    for (const GemmPlan& p : plan)
+      for (const OperandPlan& op : p.P)
+        if (op.packed_ev) cudaEventDestroy(op.packed_ev);
   }
 };
 
@@ -298,18 +305,18 @@ void Engine::prof_begin(Site& s) {
   if (!s.e0) GBCC_CK(cudaEventCreate(&s.e0));
   if (!s.e1) GBCC_CK(cudaEventCreate(&s.e1));
   if (!s.eg) GBCC_CK(cudaEventCreate(&s.eg));
-  GBCC_CK(cudaEventRecord(s.e0, stream_));
+  GBCC_CK(cudaEventRecord(s.e0, run_));
   s.has_gemm = false;
 }
 
 void Engine::prof_gemm(Site& s) {
   if (!profile_) return;
-  GBCC_CK(cudaEventRecord(s.eg, stream_));
+  GBCC_CK(cudaEventRecord(s.eg, run_));
   s.has_gemm = true;
 }
 
 void Engine::prof_end(Site& s) {
-  if (profile_) GBCC_CK(cudaEventRecord(s.e1, stream_));
+  if (profile_) GBCC_CK(cudaEventRecord(s.e1, run_));
   if (nvtx_enabled()) nvtxRangePop();
 }
 
@@ -359,12 +366,46 @@ Engine::Engine() = default;
 Engine::~Engine() {
   for (void* p : owned_) dev_free(p);
   for (auto& kv : tensors_) dev_free(kv.second->d);
-  dev_free(w64a_);
-  dev_free(w64b_);
-  dev_free(wbfa_);
-  dev_free(wbfb_);
-  dev_free(wpart_);
-  dev_free(wcount_);
+  free_workspaces();
+  for (cudaEvent_t e : marks_) cudaEventDestroy(e);
+  for (int k = 1; k < kLanes; ++k)
+    if (lane_ws_[k].stream) cudaStreamDestroy(lane_ws_[k].stream);
+}
+
+// every pointer is cleared before any new allocation: one that fails leaves no
+// pointer to freed memory behind
+void Engine::free_workspaces() {
+  for (Lane& w : lane_ws_) {
+    for (void** p : {reinterpret_cast<void**>(&w.w64a), reinterpret_cast<void**>(&w.w64b),
+                     reinterpret_cast<void**>(&w.wbfa), reinterpret_cast<void**>(&w.wbfb),
+                     reinterpret_cast<void**>(&w.wpart), reinterpret_cast<void**>(&w.wcount)}) {
+      dev_free(*p);
+      *p = nullptr;
+    }
+  }
+}
+
+void Engine::lane(int k) {
+  lane_ = k;
+  if (mode_ == Mode::kPlan) nlanes_ = std::max(nlanes_, k + 1);
+}
+
+int Engine::mark(int k) {
+  const int m = mark_cursor_++;
+  if (mode_ == Mode::kPlan) {
+    if (m >= static_cast<int>(marks_.size())) {
+      cudaEvent_t e = nullptr;
+      GBCC_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      marks_.push_back(e);
+    }
+  } else if (concurrent()) {
+    GBCC_CK(cudaEventRecord(marks_.at(m), lane_ws_[k].stream));
+  }
+  return m;
+}
+
+void Engine::wait(int k, int m) {
+  if (mode_ == Mode::kExec && concurrent()) GBCC_CK(cudaStreamWaitEvent(lane_ws_[k].stream, marks_.at(m), 0));
 }
 
 Tensor& Engine::tensor(const std::string& name, std::initializer_list<int64_t> dims, bool constant) {
@@ -420,17 +461,9 @@ void Engine::reset_plans() {
   owned_.clear();
   tables_.clear();
   planned_ = false;
-  ws64_a_ = ws64_b_ = wsbf_a_ = wsbf_b_ = wspart_ = wscount_ = 0;
-  dev_free(wcount_);
-  wcount_ = nullptr;
-  dev_free(wpart_);
-  wpart_ = nullptr;
-  dev_free(w64a_);
-  dev_free(w64b_);
-  dev_free(wbfa_);
-  dev_free(wbfb_);
-  w64a_ = w64b_ = nullptr;
-  wbfa_ = wbfb_ = nullptr;
+  free_workspaces();
+  for (Lane& w : lane_ws_) w.n64a = w.n64b = w.nbfa = w.nbfb = w.npart = w.ncount = 0;
+  nlanes_ = 1;
 }
 
 void Engine::begin(Mode m, int precision) {
@@ -441,24 +474,45 @@ void Engine::begin(Mode m, int precision) {
   flops_ = 0.0;
   n_tc_ = 0;
   n_launch_ = 0;
+  lane_ = 0;
+  mark_cursor_ = 0;
+  run_ = stream_;
+  ws_ = &lane_ws_[0];
+  if (m == Mode::kPlan) {
+    (void)mark(0);  // mark 0: the lanes' common start
+  } else {
+    lane_ws_[0].stream = stream_;
+    const int m0 = mark(0);
+    for (int k = 1; k < nlanes_; ++k) wait(k, m0);
+  }
 }
 
 void Engine::end() {
   if (mode_ == Mode::kPlan) {
+    for (int k = 1; k < nlanes_; ++k) (void)mark(k);
     planned_ = true;
-  } else if (cursor_ != sites_.size()) {
-    throw Error(GBCC_ERR_STATE, "engine: program ended early");
+  } else {
+    if (cursor_ != sites_.size()) throw Error(GBCC_ERR_STATE, "engine: program ended early");
+    for (int k = 1; k < nlanes_; ++k) wait(0, mark(k));
   }
+  lane_ = 0;
+  run_ = stream_;
+  ws_ = &lane_ws_[0];
 }
 
 Site& Engine::site() {
   if (mode_ == Mode::kPlan) {
     sites_.push_back(std::make_unique<Site>());
     ++cursor_;
+    sites_.back()->lane = lane_;
+    ws_ = &lane_ws_[lane_];
     return *sites_.back();
   }
   if (cursor_ >= sites_.size()) throw Error(GBCC_ERR_STATE, "engine: program longer than its plan");
-  return *sites_[cursor_++];
+  Site& s = *sites_[cursor_++];
+  ws_ = &lane_ws_[s.lane];
+  run_ = concurrent() ? ws_->stream : stream_;
+  return s;
 }
 
 // Offset tables are small and many (several per operand and plan): they share
@@ -495,7 +549,7 @@ void Engine::assign(const Ix& c, double beta, const std::vector<Factor>& terms) 
   if (mode_ == Mode::kExec) {
     if (s.kind != 0) throw Error(GBCC_ERR_STATE, "engine: site kind mismatch");
     prof_begin(s);
-    launch_gather(s.gather, stream_);
+    launch_gather(s.gather, run_);
     ++n_launch_;
     prof_end(s);
     return;
@@ -576,9 +630,14 @@ __nv_bfloat16* Engine::tc_panel(OperandPlan& op, int side) {
     if (!op.packed) throw Error(GBCC_ERR_STATE, "engine: constant operand not packed");
     return op.packed;
   }
-  if (op.cache_reuse) return op.cache_buf;
-  __nv_bfloat16* out = op.cache_first ? op.cache_buf : (side == 0 ? wbfa_ : wbfb_);
+  if (op.cache_reuse) {
+    if (op.first_use && concurrent() && mode_ == Mode::kExec)
+      GBCC_CK(cudaStreamWaitEvent(run_, op.first_use->packed_ev, 0));
+    return op.cache_buf;
+  }
+  __nv_bfloat16* out = op.cache_first ? op.cache_buf : (side == 0 ? ws_->wbfa : ws_->wbfb);
   pack_panel(op, out);
+  if (op.packed_ev && concurrent() && mode_ == Mode::kExec) GBCC_CK(cudaEventRecord(op.packed_ev, run_));
   return out;
 }
 
@@ -588,13 +647,13 @@ void Engine::pack_panel(const OperandPlan& op, __nv_bfloat16* out) {
   GatherArgs g = op.gather;
   g.outs = out;
   if (op.fixed) {
-    GBCC_CK(cudaMemsetAsync(op.rowexp, 0, static_cast<size_t>(op.rows_pad) * sizeof(unsigned), stream_));
+    GBCC_CK(cudaMemsetAsync(op.rowexp, 0, static_cast<size_t>(op.rows_pad) * sizeof(unsigned), run_));
     g.fixed = 1;
-    launch_gather(g, stream_);
+    launch_gather(g, run_);
     g.fixed = 2;
     ++n_launch_;  // the exponent pass (the memset is not a kernel)
   }
-  launch_gather(g, stream_);
+  launch_gather(g, run_);
   ++n_launch_;
 }
 
@@ -635,7 +694,7 @@ GemmTcArgs Engine::tc_args(const GemmPlan& p, TermClass cls, __nv_bfloat16* cons
   t.err = err_;
   t.ksplit = p.ksplit;
   t.kb_per_split = static_cast<int>(p.k_per_split);
-  t.partial = wpart_;
+  t.partial = ws_->wpart;
   t.m_major = p.m_major ? 1 : 0;
   // a slice limit makes the packed slices a superset of the used ones: one
   // pair per stage then
@@ -645,12 +704,12 @@ GemmTcArgs Engine::tc_args(const GemmPlan& p, TermClass cls, __nv_bfloat16* cons
 }
 
 void Engine::launch_tc(const GemmPlan& p, const GemmTcArgs& t) {
-  if (!launch_gemm_tc(t, stream_)) throw Error(GBCC_ERR_CUDA, "tcgen05 GEMM launch rejected (tensor map or size)");
+  if (!launch_gemm_tc(t, run_)) throw Error(GBCC_ERR_CUDA, "tcgen05 GEMM launch rejected (tensor map or size)");
   ++n_tc_;
   ++tc_total_;
   ++n_launch_;
   if (p.ksplit > 1) {
-    launch_splitk_reduce(p.M, p.N, p.ksplit, wpart_, t.Mpad, t.Npad, p.C, p.cm, p.cn, t.alpha, t.beta, stream_);
+    launch_splitk_reduce(p.M, p.N, p.ksplit, ws_->wpart, t.Mpad, t.Npad, p.C, p.cm, p.cn, t.alpha, t.beta, run_);
     ++n_launch_;
   }
 }
@@ -675,15 +734,15 @@ void Engine::launch_fixed(const GemmPlan& p, __nv_bfloat16* const panel[2]) {
   t.m_major = p.m_major ? 1 : 0;
   t.ksplit = p.ksplit;
   t.hb_per_split = static_cast<int>(p.k_per_split);
-  t.partial = wpart_;
+  t.partial = ws_->wpart;
   t.err = err_;
-  if (!launch_gemm_fixed(t, stream_)) throw Error(GBCC_ERR_CUDA, "tcgen05 GEMM launch rejected (tensor map or size)");
+  if (!launch_gemm_fixed(t, run_)) throw Error(GBCC_ERR_CUDA, "tcgen05 GEMM launch rejected (tensor map or size)");
   ++n_tc_;
   ++tc_total_;
   ++n_launch_;
   if (p.ksplit > 1) {
-    launch_splitk_reduce(p.M, p.N, p.ksplit, wpart_, round_up(p.M, kTcBM), round_up(p.N, p.bn), p.C, p.cm, p.cn,
-                         p.alpha, p.beta, stream_);
+    launch_splitk_reduce(p.M, p.N, p.ksplit, ws_->wpart, round_up(p.M, kTcBM), round_up(p.N, p.bn), p.C, p.cm, p.cn,
+                         p.alpha, p.beta, run_);
     ++n_launch_;
   }
 }
@@ -731,6 +790,7 @@ void Engine::autotune(int reps) {
         continue;
       }
     }
+    ws_ = &lane_ws_[sp->lane];
     __nv_bfloat16* panel[2];
     for (int side = 0; side < 2; ++side) panel[side] = tc_panel(p.P[side], side);
     float best = 0.f;
@@ -743,10 +803,10 @@ void Engine::autotune(int reps) {
       q.sps = p.cand_sps[c];
       q.group = p.cand_group[c];
       const GemmTcArgs t = tc_args(q, sp->cls, panel);
-      if (!launch_gemm_tc(t, stream_)) continue;
+      if (!launch_gemm_tc(t, run_)) continue;
       ++tc_total_;
       if (q.ksplit > 1)
-        launch_splitk_reduce(q.M, q.N, q.ksplit, wpart_, t.Mpad, t.Npad, q.C, q.cm, q.cn, q.alpha, q.beta, stream_);
+        launch_splitk_reduce(q.M, q.N, q.ksplit, ws_->wpart, t.Mpad, t.Npad, q.C, q.cm, q.cn, q.alpha, q.beta, run_);
       GBCC_CK(cudaEventRecord(e0, stream_));
       for (int r = 0; r < reps; ++r) launch_tc(q, t);
       GBCC_CK(cudaEventRecord(e1, stream_));
@@ -776,7 +836,7 @@ void Engine::custom(const std::function<void(cudaStream_t)>& fn, int launches) {
   if (mode_ == Mode::kExec) {
     if (s.kind != 2) throw Error(GBCC_ERR_STATE, "engine: site kind mismatch");
     prof_begin(s);
-    fn(stream_);
+    fn(run_);
     n_launch_ += launches;
     prof_end(s);
     return;
@@ -805,10 +865,10 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
       }
     } else if (p.small) {
       GemmSmallArgs g = p.sg;
-      g.partial = wpart_;
-      g.count = wcount_;
+      g.partial = ws_->wpart;
+      g.count = ws_->wcount;
       prof_gemm(s);
-      launch_gemm_small(g, stream_);
+      launch_gemm_small(g, run_);
       ++n_launch_;
     } else {
       const double* panel[2];
@@ -819,10 +879,10 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
         } else if (op.inplace) {
           panel[side] = op.gather.t[0].a;
         } else {
-          double* w = side == 0 ? w64a_ : w64b_;
+          double* w = side == 0 ? ws_->w64a : ws_->w64b;
           GatherArgs g = op.gather;
           g.out = w;
-          launch_gather(g, stream_);
+          launch_gather(g, run_);
           ++n_launch_;
           panel[side] = w;
         }
@@ -842,7 +902,7 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
       f.beta = p.beta;
       f.ksplit = p.ksplit;
       f.k_per_split = p.k_per_split;
-      f.partial = wpart_;
+      f.partial = ws_->wpart;
       f.m_major = p.m_major ? 1 : 0;
       if (p.P[0].inplace) {
         f.a_ra = p.P[0].gather.t[0].ra;
@@ -851,10 +911,10 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
       }
       prof_gemm(s);
       if (p.smallk) {
-        if (!launch_gemm_smallk(f, stream_)) throw Error(GBCC_ERR_STATE, "engine: in-place small-K operand off the stream kernel");
+        if (!launch_gemm_smallk(f, run_)) throw Error(GBCC_ERR_STATE, "engine: in-place small-K operand off the stream kernel");
         ++n_launch_;
       } else {
-        launch_gemm_f64(f, stream_);
+        launch_gemm_f64(f, run_);
         n_launch_ += p.ksplit > 1 ? 2 : 1;
       }
     }
@@ -1020,8 +1080,8 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
         g.ldo = op.K;
         g.beta = 0.0;
         size_t need = static_cast<size_t>(op.rows * op.K);
-        if (side == 0) ws64_a_ = std::max(ws64_a_, need);
-        else ws64_b_ = std::max(ws64_b_, need);
+        if (side == 0) ws_->n64a = std::max(ws_->n64a, need);
+        else ws_->n64b = std::max(ws_->n64b, need);
       }
     }
     p.alpha = alpha * coef_direct;
@@ -1050,8 +1110,8 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
       g.alpha = p.alpha;
       g.beta = p.beta;
       p.ksplit = g.ksplit;
-      wspart_ = std::max(wspart_, g.partial_elems);
-      if (g.ksplit > 1) wscount_ = std::max(wscount_, static_cast<size_t>(g.tiles));
+      ws_->npart = std::max(ws_->npart, g.partial_elems);
+      if (g.ksplit > 1) ws_->ncount = std::max(ws_->ncount, static_cast<size_t>(g.tiles));
     } else if (!p.use_tc && !p.smallk) {
       // fewer 64 x 64 output tiles than two per SM: split K over blocks (one SM
       // runs FP64 at ~1/150 of the GPU's already low FP64 rate, so even a
@@ -1066,7 +1126,7 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
           ks = (K + kps - 1) / kps;
           p.ksplit = static_cast<int>(ks);
           p.k_per_split = kps;
-          wspart_ = std::max(wspart_, static_cast<size_t>(ks * p.M * p.N));
+          ws_->npart = std::max(ws_->npart, static_cast<size_t>(ks * p.M * p.N));
         }
       }
     }
@@ -1097,6 +1157,7 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
       const int64_t Kpad = round_up(std::max<int64_t>(K, 1), kTcBK);
       for (int side = 0; side < 2; ++side) {
         OperandPlan& op = p.P[side];
+        op.lane = lane_;
         op.slices = slices;
         op.Kpad = Kpad;
         // (the FP64_TC kernel's tensor maps end at the last row)
@@ -1138,9 +1199,9 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
         if (op.constant) {
           op.pack_elems = need;  // allocated and packed by prepack()
         } else if (side == 0) {
-          wsbf_a_ = std::max(wsbf_a_, need);
+          ws_->nbfa = std::max(ws_->nbfa, need);
         } else {
-          wsbf_b_ = std::max(wsbf_b_, need);
+          ws_->nbfb = std::max(ws_->nbfb, need);
         }
       }
       // fewer output tiles than SMs and a long K: split K over CTAs.  The
@@ -1161,7 +1222,7 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
         }
         p.ksplit = static_cast<int>(std::max<int64_t>(ks, 1));
         if (p.ksplit > 1)
-          wspart_ = std::max(wspart_, static_cast<size_t>(ks * round_up(p.M, kTcBM) * round_up(p.N, p.bn)));
+          ws_->npart = std::max(ws_->npart, static_cast<size_t>(ks * round_up(p.M, kTcBM) * round_up(p.N, p.bn)));
         continue;
       }
       for (int c = 0; c < nbn; ++c) {
@@ -1191,7 +1252,7 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
         } else {
           ks = 1;
         }
-        if (ks > 1) wspart_ = std::max(wspart_, static_cast<size_t>(ks * p.P[0].rows_pad * npad));
+        if (ks > 1) ws_->npart = std::max(ws_->npart, static_cast<size_t>(ks * p.P[0].rows_pad * npad));
         // both slices of a k-block per stage: two slices, tiles up to 192 wide;
         // every slice per stage on CTA pairs: 256 x 256 tiles, where the padding
         // of M to 256 is small
@@ -1229,22 +1290,20 @@ void Engine::finalize() {
   for (const TableChunk& c : tables_)
     GBCC_CK(cudaMemcpy(c.d, c.host.data(), c.host.size() * sizeof(int64_t), cudaMemcpyHostToDevice));
   tables_.clear();
-  // every old workspace is released and its pointer cleared before the first
-  // new allocation: one that fails leaves no pointer to freed memory behind
-  for (void** p : {reinterpret_cast<void**>(&w64a_), reinterpret_cast<void**>(&w64b_),
-                   reinterpret_cast<void**>(&wbfa_), reinterpret_cast<void**>(&wbfb_),
-                   reinterpret_cast<void**>(&wpart_), reinterpret_cast<void**>(&wcount_)}) {
-    dev_free(*p);
-    *p = nullptr;
+  free_workspaces();
+  for (int k = 0; k < nlanes_; ++k) {
+    Lane& w = lane_ws_[k];
+    if (k > 0 && !w.stream) GBCC_CK(cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking));
+    w.w64a = static_cast<double*>(dev_alloc(w.n64a * sizeof(double)));
+    w.w64b = static_cast<double*>(dev_alloc(w.n64b * sizeof(double)));
+    w.wbfa = static_cast<__nv_bfloat16*>(dev_alloc(w.nbfa * sizeof(__nv_bfloat16)));
+    w.wbfb = static_cast<__nv_bfloat16*>(dev_alloc(w.nbfb * sizeof(__nv_bfloat16)));
+    w.wpart = static_cast<double*>(dev_alloc(w.npart * sizeof(double)));
+    w.wcount = static_cast<unsigned*>(dev_alloc(w.ncount * sizeof(unsigned)));
+    GBCC_CK(cudaMemsetAsync(w.wcount, 0, std::max<size_t>(w.ncount, 1) * sizeof(unsigned), stream_));
+    bytes_ += w.ncount * sizeof(unsigned) + (w.n64a + w.n64b + w.npart) * sizeof(double) +
+              (w.nbfa + w.nbfb) * sizeof(__nv_bfloat16);
   }
-  w64a_ = static_cast<double*>(dev_alloc(ws64_a_ * sizeof(double)));
-  w64b_ = static_cast<double*>(dev_alloc(ws64_b_ * sizeof(double)));
-  wbfa_ = static_cast<__nv_bfloat16*>(dev_alloc(wsbf_a_ * sizeof(__nv_bfloat16)));
-  wbfb_ = static_cast<__nv_bfloat16*>(dev_alloc(wsbf_b_ * sizeof(__nv_bfloat16)));
-  wpart_ = static_cast<double*>(dev_alloc(wspart_ * sizeof(double)));
-  wcount_ = static_cast<unsigned*>(dev_alloc(wscount_ * sizeof(unsigned)));
-  GBCC_CK(cudaMemsetAsync(wcount_, 0, std::max<size_t>(wscount_, 1) * sizeof(unsigned), stream_));
-  bytes_ += wscount_ * sizeof(unsigned) + (ws64_a_ + ws64_b_ + wspart_) * sizeof(double) + (wsbf_a_ + wsbf_b_) * sizeof(__nv_bfloat16);
   // packs shared by several contractions of a residual get their own buffer
   for (auto& kv : pack_uses_) {
     if (kv.second.size() < 2) continue;
@@ -1258,6 +1317,10 @@ void Engine::finalize() {
     for (size_t i = 1; i < kv.second.size(); ++i) {
       kv.second[i]->cache_reuse = true;
       kv.second[i]->cache_buf = first->cache_buf;
+      if (kv.second[i]->lane != first->lane) {
+        kv.second[i]->first_use = first;
+        if (!first->packed_ev) GBCC_CK(cudaEventCreateWithFlags(&first->packed_ev, cudaEventDisableTiming));
+      }
     }
   }
   packed_[0] = packed_[1] = packed_[2] = false;

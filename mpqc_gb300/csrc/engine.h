@@ -137,7 +137,7 @@ class Engine {
   Engine(const Engine&) = delete;
   Engine& operator=(const Engine&) = delete;
 
-  void set_stream(cudaStream_t s) { stream_ = s; }
+  void set_stream(cudaStream_t s) { stream_ = run_ = s; }
   cudaStream_t stream() const { return stream_; }
   void set_slices(int ladder, int ring, int other) {
     slices_[0] = ladder;
@@ -206,6 +206,18 @@ class Engine {
   // the stored choice untimed
   void autotune(int reps);
 
+  // Lanes: the operations after lane(k) run in lane k (0..kLanes-1), a stream of
+  // its own with its own workspaces; lanes start together and EXEC's end waits
+  // for all.  mark() is a point after everything enqueued so far in a lane,
+  // wait(k, m) makes lane k wait for it; program order must put a mark before
+  // its waits.  With lanes off (set_lanes, or while profiling) everything runs
+  // in program order on the engine's stream.
+  static constexpr int kLanes = 4;
+  void lane(int k);
+  int mark(int k);
+  void wait(int k, int m);
+  void set_lanes(bool on) { lanes_on_ = on; }
+
   // Statistics of the last EXEC pass (FLOPs of the contractions as planned).
   double flops() const { return flops_; }
   size_t device_bytes() const { return bytes_; }
@@ -243,14 +255,27 @@ class Engine {
     std::vector<int64_t> host;
   };
   std::vector<TableChunk> tables_;
-  // shared workspaces (sized during PLAN)
-  size_t ws64_a_ = 0, ws64_b_ = 0, wsbf_a_ = 0, wsbf_b_ = 0, wspart_ = 0, wscount_ = 0;
-  double* wpart_ = nullptr;  // K-split partial tiles
-  unsigned* wcount_ = nullptr;  // finished splits of each tile (gemm_small.cu), zero between launches
-  double* w64a_ = nullptr;
-  double* w64b_ = nullptr;
-  __nv_bfloat16* wbfa_ = nullptr;
-  __nv_bfloat16* wbfb_ = nullptr;
+  // a lane's stream and workspaces (sized during PLAN)
+  struct Lane {
+    cudaStream_t stream = nullptr;  // lanes 1..: created when a plan uses them
+    size_t n64a = 0, n64b = 0, nbfa = 0, nbfb = 0, npart = 0, ncount = 0;
+    double* w64a = nullptr;
+    double* w64b = nullptr;
+    __nv_bfloat16* wbfa = nullptr;
+    __nv_bfloat16* wbfb = nullptr;
+    double* wpart = nullptr;      // K-split partial tiles
+    unsigned* wcount = nullptr;   // finished splits of each tile (gemm_small.cu), zero between launches
+  };
+  void free_workspaces();
+  bool concurrent() const { return lanes_on_ && nlanes_ > 1 && !profile_; }
+  Lane lane_ws_[kLanes];
+  int nlanes_ = 1;           // lanes the plan uses
+  bool lanes_on_ = true;
+  int lane_ = 0;             // current lane of the program pass
+  cudaStream_t run_ = nullptr;  // stream of the current operation
+  Lane* ws_ = lane_ws_;      // workspaces of the current operation
+  std::vector<cudaEvent_t> marks_;
+  int mark_cursor_ = 0;
   int* err_ = nullptr;
   // (k-block, slice pair) steps per TMEM accumulation of the tensor-core GEMM.
   // The tensor core's FP32 accumulation loses about an ulp of the running sum
