@@ -38,7 +38,9 @@ struct gbcc_handle {
   int* d_err = nullptr;
   double* d_partial = nullptr;  // reduction scratch [kReduceBlocks * 16]
   double* d_out = nullptr;      // reduction results
-  double* h_out = nullptr;      // pinned mirror
+  double* h_out = nullptr;      // pinned mirror; [12] mirrors the error word
+  unsigned* d_count = nullptr;  // finished-block counters of the reductions: energy, DIIS
+  cudaEvent_t ev_check = nullptr;
   // DIIS storage (allocated on the first solve)
   double *x1 = nullptr, *x2 = nullptr, *e1 = nullptr, *e2 = nullptr;
   double *Bmat = nullptr, *coef = nullptr;
@@ -137,13 +139,14 @@ void read_back(gbcc_handle* h, void* dst, const void* src, size_t bytes) {
   GBCC_CK(cudaStreamSynchronize(h->stream));
 }
 
-// Check the device error word and any pending CUDA error after a sync.
+// Synchronise the stream, and check the device error word and any pending CUDA
+// error.
 void sync_check(gbcc_handle* h) {
+  int* err = reinterpret_cast<int*>(h->h_out + 12);
+  GBCC_CK(cudaMemcpyAsync(err, h->d_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   GBCC_CK(cudaStreamSynchronize(h->stream));
   GBCC_CK(cudaGetLastError());
-  int err = 0;
-  read_back(h, &err, h->d_err, sizeof(int));
-  if (err != gbcc::kDevOk) {
+  if (*err != gbcc::kDevOk) {
     GBCC_CK(cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream));
     GBCC_CK(cudaStreamSynchronize(h->stream));
     throw Error(GBCC_ERR_TIMEOUT, "a bounded device-side wait gave up (tensor-core pipeline)");
@@ -242,11 +245,26 @@ void run_residual(gbcc_handle* h, int precision) {
   h->last_launches = 1 + enqueue_residual_program(h, precision);
 }
 
-// E and error of the current t/tau/r (device-resident); returns {E, error}
-std::pair<double, double> energy_error(gbcc_handle* h) {
-  gbcc::launch_energy_terms(h->cfg.o, h->cfg.v, h->S.r1->d, h->S.r2->d, h->S.f_ai->d, h->S.g_abij->d,
-                            h->S.t1->d, h->S.tau->d, h->d_partial, h->d_out, h->stream);
-  GBCC_CK(cudaMemcpyAsync(h->h_out, h->d_out, 4 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+gbcc::EnergyTermsArgs energy_args(gbcc_handle* h) {
+  gbcc::EnergyTermsArgs e{};
+  e.o = h->cfg.o;
+  e.v = h->cfg.v;
+  e.r1 = h->S.r1->d;
+  e.r2 = h->S.r2->d;
+  e.f_ai = h->S.f_ai->d;
+  e.g_abij = h->S.g_abij->d;
+  e.t1 = h->S.t1->d;
+  e.tau = h->S.tau->d;
+  e.partial = h->d_partial;
+  e.count = h->d_count;
+  e.out = h->d_out;
+  return e;
+}
+
+// E and error from the sums (written to pinned memory by the kernel); returns {E, error}
+std::pair<double, double> energy_error(gbcc_handle* h, gbcc::EnergyTermsArgs e) {
+  e.out = h->h_out;
+  gbcc::launch_energy_terms(e, h->stream);
   sync_check(h);
   const double* s = h->h_out;
   const double E = 2.0 * s[2] + s[3];
@@ -387,15 +405,14 @@ void build_solve_graph(gbcc_handle* h) {
   p.cond_mixed = hmix;
   p.cond_fp64 = hf64;
   capture_into(h, body, [&] {
-    gbcc::launch_energy_terms(c.o, c.v, S.r1->d, S.r2->d, S.f_ai->d, S.g_abij->d, S.t1->d, S.tau->d, h->d_partial,
-                              h->d_out, st);
-    gbcc::launch_solve_decide(p, st);
+    gbcc::launch_energy_decide(energy_args(h), p, st);
   });
   cudaGraphNode_t decide = sink_node(body);
   cudaGraphNode_t nup;
   cudaGraph_t ub = add_conditional(body, &decide, hup, cudaGraphCondTypeIf, &nup);
   gbcc::DiisArgs d{};
   d.dyn = &h->d_state->diis;
+  d.count = h->d_count + 1;
   d.o = c.o;
   d.v = c.v;
   d.eps_o = S.eps_o->d;
@@ -485,16 +502,29 @@ void tune_plan(gbcc_handle* h) {
 }
 
 // The particle-particle ladder runs over a <= b, i <= j: amplitudes must be
-// pair-symmetric, t2(a,b,i,j) = t2(b,a,j,i) (closed-shell CCSD amplitudes are)
-void check_pair_symmetric(gbcc_handle* h) {
+// pair-symmetric, t2(a,b,i,j) = t2(b,a,j,i) (closed-shell CCSD amplitudes are).
+// Enqueue the check of S.t2; its result is there after ev_check.
+void enqueue_pair_check(gbcc_handle* h) {
   auto* out = reinterpret_cast<unsigned long long*>(h->d_out + 8);
   GBCC_CK(cudaMemsetAsync(out, 0, 2 * sizeof(double), h->stream));
   gbcc::launch_pair_asym(h->cfg.o, h->cfg.v, h->S.t2->d, out, h->stream);
   GBCC_CK(cudaMemcpyAsync(h->h_out + 8, h->d_out + 8, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  sync_check(h);
-  if (!(h->h_out[8] <= 1e-12 * h->h_out[9]))
+  GBCC_CK(cudaEventRecord(h->ev_check, h->stream));
+}
+
+void finish_pair_check(gbcc_handle* h) {
+  GBCC_CK(cudaEventSynchronize(h->ev_check));
+  if (!(h->h_out[8] <= 1e-12 * h->h_out[9])) {
+    const double md = h->h_out[8], mb = h->h_out[9];
+    sync_check(h);  // what was enqueued behind the check
     throw Error(GBCC_ERR_INVALID_ARG, "t2 is not pair-symmetric (t2(a,b,i,j) != t2(b,a,j,i)): max difference " +
-                                          std::to_string(h->h_out[8]) + " of max |t2| " + std::to_string(h->h_out[9]));
+                                          std::to_string(md) + " of max |t2| " + std::to_string(mb));
+  }
+}
+
+void check_pair_symmetric(gbcc_handle* h) {
+  enqueue_pair_check(h);
+  finish_pair_check(h);
 }
 
 void plan_residual(gbcc_handle* h) {
@@ -531,16 +561,18 @@ void calibrate_slices(gbcc_handle* h, const double* t1_in, const double* t2_in) 
     h->slices_used[k] = req[k] == 0 ? 3 : req[k];
     h->slice_err[k] = -1.0;
   }
-  plan_residual(h);
+  h->eng->set_trial(true);
   struct Guard {
     gbcc_handle* h;
     double* ref = nullptr;
     ~Guard() {
       h->calibrating = false;
+      h->eng->set_trial(false);
       h->eng->set_slice_limit(0, 0, 0);
       gbcc::dev_free(ref);
     }
   } guard{h};
+  plan_residual(h);
   h->calibrating = true;
   if (t1_in && t2_in) {
     GBCC_CK(cudaMemcpyAsync(S.t1->d, t1_in, n1 * sizeof(double), cudaMemcpyDefault, st));
@@ -562,8 +594,6 @@ void calibrate_slices(gbcc_handle* h, const double* t1_in, const double* t2_in) 
   for (int k = 0; k < 3; ++k) {
     if (req[k] != 0) continue;
     h->slice_err[k] = 0.0;
-    // (a class whose contractions all run in FP64 has nothing to choose)
-    if (!h->eng->class_on_tensor_cores(static_cast<gbcc::TermClass>(k))) continue;
     for (int s = 2; s >= 1; --s) {
       int lim[3] = {0, 0, 0};
       lim[k] = s;
@@ -581,7 +611,8 @@ void calibrate_slices(gbcc_handle* h, const double* t1_in, const double* t2_in) 
   GBCC_CK(cudaMemsetAsync(S.tau->d, 0, n2 * sizeof(double), st));
   sync_check(h);
   h->calibrating = false;
-  if (h->slices_used[0] != 3 || h->slices_used[1] != 3 || h->slices_used[2] != 3) plan_residual(h);
+  h->eng->set_trial(false);
+  plan_residual(h);
   sync_check(h);
   tune_plan(h);
 }
@@ -708,13 +739,17 @@ gbcc_status gbcc_create(gbcc_handle** out, const gbcc_config* cfg) {
     h->eng->set_error_word(h->d_err);
     h->d_partial = static_cast<double*>(gbcc::dev_alloc(gbcc::kReduceBlocks * 16 * sizeof(double)));
     h->d_out = static_cast<double*>(gbcc::dev_alloc(16 * sizeof(double)));
+    h->d_count = static_cast<unsigned*>(gbcc::dev_alloc(2 * sizeof(unsigned)));
+    GBCC_CK(cudaMemset(h->d_count, 0, 2 * sizeof(unsigned)));
     GBCC_CK(cudaMallocHost(&h->h_out, 16 * sizeof(double)));
+    GBCC_CK(cudaEventCreateWithFlags(&h->ev_check, cudaEventDisableTiming));
   } catch (const Error& e) {
     g_create_error = e.what();
     if (h->h_out) cudaFreeHost(h->h_out);
     gbcc::dev_free(h->d_err);
     gbcc::dev_free(h->d_partial);
     gbcc::dev_free(h->d_out);
+    gbcc::dev_free(h->d_count);
     return e.status;
   }
   *out = h.release();
@@ -877,8 +912,10 @@ gbcc_status gbcc_residual_ex(gbcc_handle* h, int32_t precision, const double* t1
     h->have_solution = false;
     copy_in(h->S.t1->d, t1_ai, n1_of(h), h->stream);
     copy_in(h->S.t2->d, t2_abij, n2_of(h), h->stream);
-    check_pair_symmetric(h);
+    // the residual runs behind the check, the results leave only after it
+    enqueue_pair_check(h);
     run_residual(h, precision);
+    finish_pair_check(h);
     copy_out(r1_ai, h->S.r1->d, n1_of(h), h->stream);
     copy_out(r2_abij, h->S.r2->d, n2_of(h), h->stream);
     sync_check(h);
@@ -899,12 +936,23 @@ gbcc_status gbcc_energy(gbcc_handle* h, const double* t1_ai, const double* t2_ab
     if (!t1_ai || !t2_abij || !r1_ai || !r2_abij)
       throw Error(GBCC_ERR_INVALID_ARG, "gbcc_energy: NULL argument");
     h->have_solution = false;
-    copy_in(h->S.t1->d, t1_ai, n1_of(h), h->stream);
-    copy_in(h->S.t2->d, t2_abij, n2_of(h), h->stream);
-    copy_in(h->S.r1->d, r1_ai, n1_of(h), h->stream);
-    copy_in(h->S.r2->d, r2_abij, n2_of(h), h->stream);
-    gbcc::launch_make_tau(h->cfg.o, h->cfg.v, h->S.t1->d, h->S.t2->d, h->S.tau->d, h->stream);
-    auto ee = energy_error(h);
+    // device arrays are read where they are; host arrays through the handle's own
+    gbcc::EnergyTermsArgs e = energy_args(h);
+    auto on_device = [&](const double* src, gbcc::Tensor* own, int64_t n) -> const double* {
+      cudaPointerAttributes at{};
+      if (cudaPointerGetAttributes(&at, src) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
+          at.device == h->cfg.device)
+        return src;
+      cudaGetLastError();
+      copy_in(own->d, src, n, h->stream);
+      return own->d;
+    };
+    e.t1 = on_device(t1_ai, h->S.t1, n1_of(h));
+    e.t2 = on_device(t2_abij, h->S.t2, n2_of(h));
+    e.r1 = on_device(r1_ai, h->S.r1, n1_of(h));
+    e.r2 = on_device(r2_abij, h->S.r2, n2_of(h));
+    e.tau = nullptr;
+    auto ee = energy_error(h, e);
     if (energy) *energy = ee.first;
     if (error) *error = ee.second;
     return GBCC_OK;
@@ -998,7 +1046,7 @@ gbcc_status gbcc_solve(gbcc_handle* h, double* t1_ai, double* t2_abij, double* e
         for (int k = 1; k < ntest; ++k) print_iter(k, hist[3 * k + 1], hist[3 * k + 2], hist[3 * k], 0.0);
     }
     while (!graph_solve && iter < c.max_iter) {
-      auto ee = energy_error(h);
+      auto ee = energy_error(h, energy_args(h));
       error = ee.second;
       E0 = E1;
       E1 = ee.first;
@@ -1047,6 +1095,7 @@ gbcc_status gbcc_solve(gbcc_handle* h, double* t1_ai, double* t2_abij, double* e
       else ++nvec;
       slots.push_back(head);
       gbcc::DiisArgs d{};
+      d.count = h->d_count + 1;
       d.o = c.o;
       d.v = c.v;
       d.eps_o = S.eps_o->d;
@@ -1200,12 +1249,12 @@ gbcc_status gbcc_destroy(gbcc_handle* h) {
   h->eng.reset();
   h->aux.reset();
   for (void* p : {(void*)h->x1, (void*)h->x2, (void*)h->e1, (void*)h->e2, (void*)h->Bmat, (void*)h->coef,
-                  (void*)h->d_nskip, (void*)h->d_err, (void*)h->d_partial, (void*)h->d_out,
+                  (void*)h->d_nskip, (void*)h->d_err, (void*)h->d_partial, (void*)h->d_out, (void*)h->d_count,
                   (void*)h->seed1, (void*)h->seed2, (void*)h->d_state, (void*)h->d_history, (void*)h->d_stamps})
     gbcc::dev_free(p);
   if (h->h_out) cudaFreeHost(h->h_out);
-  if (h->ev0) cudaEventDestroy(h->ev0);
-  if (h->ev1) cudaEventDestroy(h->ev1);
+  for (cudaEvent_t e : {h->ev0, h->ev1, h->ev_check})
+    if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : h->slots)
     if (e) cudaEventDestroy(e);
   if (h->stream) cudaStreamDestroy(h->stream);

@@ -239,6 +239,11 @@ struct OperandPlan {
 constexpr double kSmallUs = 800.0;
 constexpr double kSmallUsMixed = 20.0;
 constexpr double kSmallUsFixed = 80.0;
+// While slice counts are chosen (set_trial) the mixed plan runs in FP64 only
+// contractions below this many FLOPs, so that the choice is made from the split
+// error of the same contractions at every size and does not loosen where a
+// size runs some of them in FP64.
+constexpr double kTrialFlops = 1.0e6;
 
 struct GemmPlan {
   bool use_tc = false;
@@ -353,12 +358,6 @@ std::vector<SiteStat> Engine::site_stats(int precision) {
     out.push_back(st);
   }
   return out;
-}
-
-bool Engine::class_on_tensor_cores(TermClass cls) const {
-  for (const auto& sp : sites_)
-    if (sp->kind == 1 && sp->cls == cls && sp->plan[1].use_tc) return true;
-  return false;
 }
 
 Engine::Engine() = default;
@@ -969,6 +968,7 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
     p.sg.N = std::min(rowsA, rowsB);
     p.sg.K = K;
     p.small = plan_gemm_small(p.sg) <= (pm == 0 ? kSmallUs : (emu ? kSmallUsFixed : kSmallUsMixed));
+    if (trial_ && pm == 1) p.small = flops < kTrialFlops;
     int slices = p.small || pm == 0 ? 0 : (emu ? kFixedSlices : slices_for(cls));
     // a short contraction into a large output is memory-bound: CUDA cores
     // (measured faster for N > 32; the tensor-core kernel wins below).  The

@@ -152,6 +152,9 @@ class Engine {
     slice_limit_[1] = ring;
     slice_limit_[2] = other;
   }
+  // Whether the next PLAN is for choosing slice counts (tensor cores for all but
+  // the smallest contractions of the mixed plan)
+  void set_trial(bool on) { trial_ = on; }
   // MMAs per TMEM accumulation, in (k-block, slice pair) steps, for
   // contractions with 3 slices and with fewer
   void set_chunk(int three_slices, int fewer) {
@@ -168,8 +171,6 @@ class Engine {
   // packs of them can be shared between contractions.
   void set_frozen(std::initializer_list<const Tensor*> ts) { frozen_ = std::unordered_set<const Tensor*>(ts); }
   std::vector<SiteStat> site_stats(int precision);
-  // whether the mixed plan has a tensor-core contraction of this class
-  bool class_on_tensor_cores(TermClass cls) const;
 
   // Persistent device tensor owned by the engine (allocated on first request).
   Tensor& tensor(const std::string& name, std::initializer_list<int64_t> dims, bool constant = false);
@@ -288,6 +289,7 @@ class Engine {
   int chunk_lo_ = 24;
   bool profile_ = false;
   bool emu_ = false;
+  bool trial_ = false;
   bool packed_[3] = {false, false, false};
   std::unordered_set<const Tensor*> frozen_;
   std::unordered_map<std::string, std::vector<struct OperandPlan*>> pack_uses_;

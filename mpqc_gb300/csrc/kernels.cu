@@ -7,6 +7,7 @@
 // BF16 split works on bit patterns and FP32 remainders, and single-term packs
 // are plain copies (their coefficient scales the GEMM instead).
 #include "fp_bits.cuh"
+#include "energy_terms.cuh"
 #include "gather.cuh"
 #include "kernels.h"
 
@@ -72,55 +73,7 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   return r;
 }
 
-__global__ void __launch_bounds__(kThreads) energy_partial_kernel(
-    int64_t o, int64_t v, const double* __restrict__ r1, const double* __restrict__ r2,
-    const double* __restrict__ f_ai, const double* __restrict__ g_abij,
-    const double* __restrict__ t1, const double* __restrict__ tau, double* __restrict__ partial) {
-  __shared__ double sh[kThreads];
-  const int64_t o2 = o * o;
-  double s_r1 = 0.0, s_r2 = 0.0, s_e1 = 0.0, s_e2 = 0.0;
-  for (int64_t p = blockIdx.x; p < v * v; p += gridDim.x) {
-    int64_t a, b;
-    divmod32(p, v, a, b);
-    const double* r2p = r2 + p * o2;
-    const double* gp = g_abij + p * o2;
-    const double* tp = tau + p * o2;
-    const double* tq = tau + (b * v + a) * o2;
-    for (int64_t ij = threadIdx.x; ij < o2; ij += blockDim.x) {
-      const double r = r2p[ij];
-      s_r2 = fma(r, r, s_r2);
-      s_e2 = fma(gp[ij] + r, 2.0 * tp[ij] - tq[ij], s_e2);
-    }
-  }
-  const int64_t n1 = v * o;
-  for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < n1;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const double r = r1[e];
-    s_r1 = fma(r, r, s_r1);
-    s_e1 = fma(f_ai[e] + r, t1[e], s_e1);
-  }
-  s_r1 = block_sum(s_r1, sh);
-  s_r2 = block_sum(s_r2, sh);
-  s_e1 = block_sum(s_e1, sh);
-  s_e2 = block_sum(s_e2, sh);
-  if (threadIdx.x == 0) {
-    partial[blockIdx.x * 4 + 0] = s_r1;
-    partial[blockIdx.x * 4 + 1] = s_r2;
-    partial[blockIdx.x * 4 + 2] = s_e1;
-    partial[blockIdx.x * 4 + 3] = s_e2;
-  }
-}
-
-__global__ void __launch_bounds__(kThreads) reduce_partials_kernel(const double* __restrict__ partial,
-                                                                   int nblocks, int nq, double* out) {
-  __shared__ double sh[kThreads];
-  for (int q = 0; q < nq; ++q) {
-    double s = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) s += partial[b * nq + q];
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) out[q] = s;
-  }
-}
+__global__ void __launch_bounds__(kEnergyThreads) energy_terms_kernel(EnergyTermsArgs g) { (void)energy_terms(g); }
 
 __global__ void __launch_bounds__(kThreads) make_tau_kernel(int64_t o, int64_t v,
                                                             const double* __restrict__ t1,
@@ -640,9 +593,164 @@ __device__ __forceinline__ void load_diis_meta(const DiisArgs& d, DiisMeta* m) {
   __syncthreads();
 }
 
+// |det| of the normalised bordered DIIS matrix below which the oldest stored
+// vector is dropped (TiledArray's TA::DIIS test, threshold fixed by the water
+// 6-31G iteration trace MPQC records in its validation outputs).
+constexpr double kDiisDetMin = 1.0e-15;
+
+// The bordered system of a DIIS step, in shared memory for one warp.
+struct DiisSystem {
+  double A[(kDiisMax + 1) * (kDiisMax + 1)];
+  double rhs[kDiisMax + 1], sol[kDiisMax + 1], f[kDiisMax + 1];
+};
+
+// Gaussian elimination with partial pivoting on the row-major n x n system, by
+// one warp (every element sees the operations of the serial algorithm in its
+// order); returns |det A| (product of the pivots), 0 with sol unset if a pivot
+// is zero.  (One thread on arrays in local memory took most of a small solve's
+// time outside its residuals.)
+__device__ double gepp(DiisSystem& S, int n) {
+  const int lane = threadIdx.x % 32;
+  double* A = S.A;
+  double det = 1.0;
+  for (int col = 0; col < n; ++col) {
+    // the first row of the largest |A[r][col]|
+    double best = (lane >= col && lane < n) ? fabs(A[lane * n + col]) : -1.0;
+    int p = lane;
+    for (int d = 16; d > 0; d >>= 1) {
+      const double ob = __shfl_down_sync(0xffffffffu, best, d);
+      const int op = __shfl_down_sync(0xffffffffu, p, d);
+      if (ob > best || (ob == best && op < p)) {
+        best = ob;
+        p = op;
+      }
+    }
+    best = __shfl_sync(0xffffffffu, best, 0);
+    p = __shfl_sync(0xffffffffu, p, 0);
+    if (!(best > 0.0)) return best == 0.0 ? 0.0 : best;
+    det *= best;
+    if (p != col) {
+      if (lane < n) {
+        const double t = A[col * n + lane];
+        A[col * n + lane] = A[p * n + lane];
+        A[p * n + lane] = t;
+      }
+      if (lane == 0) {
+        const double t = S.rhs[col];
+        S.rhs[col] = S.rhs[p];
+        S.rhs[p] = t;
+      }
+      __syncwarp();
+    }
+    if (lane > col && lane < n) {
+      const double f = A[lane * n + col] / A[col * n + col];
+      S.f[lane] = f;
+      S.rhs[lane] -= f * S.rhs[col];
+    }
+    __syncwarp();
+    const int w = n - col;
+    for (int e = lane; e < (w - 1) * w; e += 32) {
+      const int r = col + 1 + e / w, c = col + e % w;
+      A[r * n + c] -= S.f[r] * A[col * n + c];
+    }
+    __syncwarp();
+  }
+  if (lane == 0) {
+    for (int r = n - 1; r >= 0; --r) {
+      double s = S.rhs[r];
+      for (int c = r + 1; c < n; ++c) s -= A[r * n + c] * S.sol[c];
+      S.sol[r] = s / A[r * n + r];
+    }
+  }
+  __syncwarp();
+  return det;
+}
+
+// DIIS coefficients (TiledArray's TA::DIIS extrapolation, cc/solvers.h:112-121)
+// from the B matrix of the n stored vectors (slots, oldest first, B by slot
+// with leading dimension nd): the bordered system [[0, -1], [-1, B]] on the
+// newest n - nskip vectors, normalised by the oldest kept <e, e>, damped on
+// the diagonal; the oldest vectors are dropped while |det| < kDiisDetMin (a
+// singular or near-singular B), the newest alone as the last resort.  coef
+// (by slot, nd entries) is written; returns nskip.  Called by one warp.
+__device__ int diis_coefficients(DiisSystem& S, const double* Bmat, int nd, const int* slots, int n, double damping,
+                                 double* coef) {
+  const int lane = threadIdx.x % 32;
+  if (lane < nd) coef[lane] = 0.0;
+  for (int nskip = 0; nskip < n; ++nskip) {
+    const int m = n - nskip;
+    const int w = m + 1;
+    // normalise by the oldest kept vector's <e, e>
+    const double b0 = fabs(Bmat[slots[nskip] * nd + slots[nskip]]);
+    const double norm = b0 > 0.0 ? 1.0 / b0 : 1.0;
+    __syncwarp();
+    if (lane < w) S.rhs[lane] = (lane == 0) ? -1.0 : 0.0;
+    for (int e = lane; e < w * w; e += 32) {
+      const int r = e / w, c = e % w;
+      double val;
+      if (r == 0 && c == 0) val = 0.0;
+      else if (r == 0 || c == 0) val = -1.0;
+      else val = Bmat[slots[nskip + r - 1] * nd + slots[nskip + c - 1]] * norm;
+      if (r > 0 && r == c) val *= 1.0 + damping;
+      S.A[e] = val;
+    }
+    __syncwarp();
+    const double det = gepp(S, w);
+    if (det > 0.0 && (det >= kDiisDetMin || nskip == n - 1)) {
+      if (lane < m) coef[slots[nskip + lane]] = S.sol[lane + 1];
+      return nskip;
+    }
+  }
+  __syncwarp();
+  if (lane == 0) coef[slots[n - 1]] = 1.0;
+  return n - 1;
+}
+
+// test hook: diis_coefficients on a given B (slots 0..n-1 in order)
+__global__ void diis_coefficients_test_kernel(const double* Bmat, int n, double damping, double* coef,
+                                              int* nskip) {
+  __shared__ DiisSystem S;
+  int slots[kDiisMax];
+  for (int q = 0; q < n; ++q) slots[q] = q;
+  const int k = diis_coefficients(S, Bmat, n, slots, n, damping, coef);
+  if (threadIdx.x == 0) *nskip = k;
+}
+
+// Sums of the block partials into the new row and column of B, and the
+// coefficients: the last block of diis_jacobi_dots_kernel.
+__device__ void diis_solve(const DiisArgs& d, const DiisMeta& meta, unsigned nblocks) {
+  __shared__ double dots[kDiisMax];
+  __shared__ DiisSystem S;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int slot = meta.slot;
+  for (int q = warp; q < meta.nvec; q += kThreads / 32) {
+    double s = 0.0;
+    for (unsigned b = lane; b < nblocks; b += 32) s += __ldcg(d.partial + b * kDiisMax + q);
+    for (int m = 16; m > 0; m >>= 1) s += __shfl_down_sync(0xffffffffu, s, m);
+    if (lane == 0) dots[q] = s;
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  const int nd = d.ndiis;
+  const int* slots = meta.slots;
+  if (lane < meta.nvec) {
+    d.Bmat[slot * nd + slots[lane]] = dots[lane];
+    d.Bmat[slots[lane] * nd + slot] = dots[lane];
+  }
+  __syncwarp();
+  if (!meta.extrapolate) {
+    if (lane < nd) d.coef[lane] = lane == slot ? 1.0 : 0.0;
+    if (lane == 0) *d.nskip_out = -1;
+    return;
+  }
+  const int k = diis_coefficients(S, d.Bmat, nd, slots, meta.nvec, d.damping, d.coef);
+  if (lane == 0) *d.nskip_out = k;
+}
+
 __global__ void __launch_bounds__(kThreads) diis_jacobi_dots_kernel(DiisArgs d) {
   __shared__ double sh[kThreads];
   __shared__ DiisMeta meta;
+  __shared__ bool last;
   load_diis_meta(d, &meta);
   const int slot = meta.slot, nvec = meta.nvec;
   const int64_t o = d.o, v = d.v, o2 = o * o, n2 = v * v * o2, n1 = v * o;
@@ -685,121 +793,18 @@ __global__ void __launch_bounds__(kThreads) diis_jacobi_dots_kernel(DiisArgs d) 
   }
   for (int q = 0; q < nvec; ++q) {
     const double s = block_sum(acc[q], sh);
-    if (threadIdx.x == 0) d.partial[blockIdx.x * kDiisMax + q] = s;
+    if (threadIdx.x == 0) __stcg(d.partial + blockIdx.x * kDiisMax + q, s);
   }
-}
-
-// |det| of the normalised bordered DIIS matrix below which the oldest stored
-// vector is dropped (TiledArray's TA::DIIS test, threshold fixed by the water
-// 6-31G iteration trace MPQC records in its validation outputs).
-constexpr double kDiisDetMin = 1.0e-15;
-
-// Gaussian elimination with partial pivoting on a row-major n x n system;
-// returns |det A| (product of the pivots), 0 with x unset if a pivot is zero.
-__device__ double gepp(double* A, double* b, double* x, int n) {
-  double det = 1.0;
-  for (int col = 0; col < n; ++col) {
-    int p = col;
-    double best = fabs(A[col * n + col]);
-    for (int r = col + 1; r < n; ++r) {
-      if (fabs(A[r * n + col]) > best) { best = fabs(A[r * n + col]); p = r; }
-    }
-    if (best == 0.0) return 0.0;
-    det *= best;
-    if (p != col) {
-      for (int c = 0; c < n; ++c) { double t = A[col * n + c]; A[col * n + c] = A[p * n + c]; A[p * n + c] = t; }
-      double t = b[col]; b[col] = b[p]; b[p] = t;
-    }
-    for (int r = col + 1; r < n; ++r) {
-      const double f = A[r * n + col] / A[col * n + col];
-      for (int c = col; c < n; ++c) A[r * n + c] -= f * A[col * n + c];
-      b[r] -= f * b[col];
-    }
-  }
-  for (int r = n - 1; r >= 0; --r) {
-    double s = b[r];
-    for (int c = r + 1; c < n; ++c) s -= A[r * n + c] * x[c];
-    x[r] = s / A[r * n + r];
-  }
-  return det;
-}
-
-// DIIS coefficients (TiledArray's TA::DIIS extrapolation, cc/solvers.h:112-121)
-// from the B matrix of the n stored vectors (slots, oldest first, B by slot
-// with leading dimension nd): the bordered system [[0, -1], [-1, B]] on the
-// newest n - nskip vectors, normalised by the oldest kept <e, e>, damped on
-// the diagonal; the oldest vectors are dropped while |det| < kDiisDetMin (a
-// singular or near-singular B), the newest alone as the last resort.  coef
-// (by slot, nd entries) is written; returns nskip.
-__device__ int diis_coefficients(const double* Bmat, int nd, const int* slots, int n, double damping,
-                                 double* coef) {
-  for (int s = 0; s < nd; ++s) coef[s] = 0.0;
-  double A[(kDiisMax + 1) * (kDiisMax + 1)];
-  double rhs[kDiisMax + 1];
-  double sol[kDiisMax + 1];
-  for (int nskip = 0; nskip < n; ++nskip) {
-    const int m = n - nskip;
-    const int w = m + 1;
-    // normalise by the oldest kept vector's <e, e>
-    const double b0 = fabs(Bmat[slots[nskip] * nd + slots[nskip]]);
-    const double norm = b0 > 0.0 ? 1.0 / b0 : 1.0;
-    for (int r = 0; r < w; ++r) {
-      rhs[r] = (r == 0) ? -1.0 : 0.0;
-      for (int c = 0; c < w; ++c) {
-        double val;
-        if (r == 0 && c == 0) val = 0.0;
-        else if (r == 0 || c == 0) val = -1.0;
-        else val = Bmat[slots[nskip + r - 1] * nd + slots[nskip + c - 1]] * norm;
-        if (r > 0 && r == c) val *= 1.0 + damping;
-        A[r * w + c] = val;
-      }
-    }
-    const double det = gepp(A, rhs, sol, w);
-    if (det > 0.0 && (det >= kDiisDetMin || nskip == n - 1)) {
-      for (int q = 0; q < m; ++q) coef[slots[nskip + q]] = sol[q + 1];
-      return nskip;
-    }
-  }
-  coef[slots[n - 1]] = 1.0;
-  return n - 1;
-}
-
-// test hook: diis_coefficients on a given B (slots 0..n-1 in order)
-__global__ void diis_coefficients_test_kernel(const double* Bmat, int n, double damping, double* coef,
-                                              int* nskip) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int slots[kDiisMax];
-  for (int q = 0; q < n; ++q) slots[q] = q;
-  *nskip = diis_coefficients(Bmat, n, slots, n, damping, coef);
-}
-
-__global__ void __launch_bounds__(kThreads) diis_solve_kernel(DiisArgs d) {
-  __shared__ double sh[kThreads];
-  __shared__ double dots[kDiisMax];
-  __shared__ DiisMeta meta;
-  load_diis_meta(d, &meta);
-  const int slot = meta.slot;
-  for (int q = 0; q < meta.nvec; ++q) {
-    double s = 0.0;
-    for (int b = threadIdx.x; b < kReduceBlocks; b += blockDim.x) s += d.partial[b * kDiisMax + q];
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) dots[q] = s;
+  // the last block to finish solves for the coefficients
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(d.count, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  const int nd = d.ndiis;
-  const int* slots = meta.slots;
-  for (int q = 0; q < meta.nvec; ++q) {
-    d.Bmat[slot * nd + slots[q]] = dots[q];
-    d.Bmat[slots[q] * nd + slot] = dots[q];
-  }
-  if (!meta.extrapolate) {
-    for (int s = 0; s < nd; ++s) d.coef[s] = 0.0;
-    d.coef[slot] = 1.0;
-    *d.nskip_out = -1;
-    return;
-  }
-  *d.nskip_out = diis_coefficients(d.Bmat, nd, slots, meta.nvec, d.damping, d.coef);
+  if (!last) return;
+  __threadfence();
+  if (threadIdx.x == 0) *d.count = 0u;  // ready for the next launch
+  diis_solve(d, meta, gridDim.x);
 }
 
 struct ExtrapArgs {
@@ -821,6 +826,11 @@ __device__ __forceinline__ void load_extrap_meta(const ExtrapArgs& x, int* s_slo
   __syncthreads();
 }
 
+// t1, t2 and tau of the extrapolated amplitudes.  FUSED: a block forms the rows
+// a and b of t1 that its tau needs (2 o FMA chains beside o^2 of them) and blocks
+// (a, 0) store them; otherwise (rows beyond shared memory) t1 is there already.
+constexpr int kExtrapRows = 1024;  // o of the fused form
+
 __global__ void __launch_bounds__(kThreads) extrapolate_t1_kernel(ExtrapArgs x) {
   __shared__ int slots[kDiisMax];
   __shared__ int nvec;
@@ -834,17 +844,34 @@ __global__ void __launch_bounds__(kThreads) extrapolate_t1_kernel(ExtrapArgs x) 
   }
 }
 
+template <bool FUSED>
 __global__ void __launch_bounds__(kThreads) extrapolate_t2_tau_kernel(ExtrapArgs x) {
   __shared__ int slots[kDiisMax];
   __shared__ int s_nvec;
+  __shared__ double rows[FUSED ? 2 * kExtrapRows : 1];
   load_extrap_meta(x, slots, &s_nvec);
   const int nvec = s_nvec;
-  const int64_t o = x.o, v = x.v, o2 = o * o, n2 = v * v * o2;
+  const int64_t o = x.o, v = x.v, o2 = o * o, n2 = v * v * o2, n1 = v * o;
   double c[kDiisMax];
   for (int q = 0; q < kDiisMax; ++q) c[q] = (q < nvec) ? x.coef[slots[q]] : 0.0;
   for (int64_t p = blockIdx.x; p < v * v; p += gridDim.x) {
     int64_t a, b;
     divmod32(p, v, a, b);
+    const double *ta = x.t1 + a * o, *tb = x.t1 + b * o;
+    if constexpr (FUSED) {
+      __syncthreads();
+      for (int e = threadIdx.x; e < 2 * o; e += blockDim.x) {
+        const bool second = e >= o;
+        const int64_t at = second ? b * o + e - o : a * o + e;
+        double acc = 0.0;
+        for (int q = 0; q < nvec; ++q) acc = fma(c[q], x.x1[slots[q] * n1 + at], acc);
+        rows[second ? kExtrapRows + e - o : e] = acc;
+        if (!second && b == 0) x.t1[at] = acc;
+      }
+      __syncthreads();
+      ta = rows;
+      tb = rows + kExtrapRows;
+    }
     for (int64_t ij = threadIdx.x; ij < o2; ij += blockDim.x) {
       int64_t i, j;
       divmod32(ij, o, i, j);
@@ -852,7 +879,7 @@ __global__ void __launch_bounds__(kThreads) extrapolate_t2_tau_kernel(ExtrapArgs
       double acc = 0.0;
       for (int q = 0; q < nvec; ++q) acc = fma(c[q], x.x2[slots[q] * n2 + e], acc);
       x.t2[e] = acc;
-      x.tau[e] = fma(x.t1[a * o + i], x.t1[b * o + j], acc);
+      x.tau[e] = fma(ta[i], tb[j], acc);
     }
   }
 }
@@ -940,12 +967,8 @@ void launch_gather(const GatherArgs& g, cudaStream_t st) {
   else gather_kernel<<<sh.grid, sh.block, 0, st>>>(g);
 }
 
-void launch_energy_terms(int64_t o, int64_t v, const double* r1, const double* r2,
-                         const double* f_ai, const double* g_abij, const double* t1,
-                         const double* tau, double* partial, double* out, cudaStream_t st) {
-  energy_partial_kernel<<<kReduceBlocks, kThreads, 0, st>>>(o, v, r1, r2, f_ai, g_abij, t1, tau,
-                                                           partial);
-  reduce_partials_kernel<<<1, kThreads, 0, st>>>(partial, kReduceBlocks, 4, out);
+void launch_energy_terms(const EnergyTermsArgs& g, cudaStream_t st) {
+  energy_terms_kernel<<<energy_blocks(g.v), kEnergyThreads, 0, st>>>(g);
 }
 
 void launch_make_tau(int64_t o, int64_t v, const double* t1, const double* t2, double* tau,
@@ -1028,8 +1051,7 @@ void launch_maxabs_diff(int64_t n, const double* a, const double* b, unsigned lo
 }
 
 void launch_diis_step(const DiisArgs& d, cudaStream_t st) {
-  diis_jacobi_dots_kernel<<<kReduceBlocks, kThreads, 0, st>>>(d);
-  diis_solve_kernel<<<1, kThreads, 0, st>>>(d);
+  diis_jacobi_dots_kernel<<<energy_blocks(d.v), kThreads, 0, st>>>(d);
 }
 
 void launch_diis_coefficients_test(const double* Bmat, int n, double damping, double* coef, int* nskip,
@@ -1053,8 +1075,12 @@ void launch_diis_extrapolate(int64_t o, int64_t v, const double* x1, const doubl
   x.t2 = t2;
   x.tau = tau;
   x.dyn = dyn;
+  if (o <= kExtrapRows) {
+    extrapolate_t2_tau_kernel<true><<<grid_for(v * v, 1), kThreads, 0, st>>>(x);
+    return;
+  }
   extrapolate_t1_kernel<<<grid_for(v * o, kThreads), kThreads, 0, st>>>(x);
-  extrapolate_t2_tau_kernel<<<grid_for(v * v, 1), kThreads, 0, st>>>(x);
+  extrapolate_t2_tau_kernel<false><<<grid_for(v * v, 1), kThreads, 0, st>>>(x);
 }
 
 }  // namespace gbcc

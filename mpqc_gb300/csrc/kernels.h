@@ -310,15 +310,25 @@ bool launch_gemm_triples(GemmMultiArgs g, int slices, int ntriples, cudaStream_t
 
 // ---------------------------------------------------------------------------
 // Deterministic FP64 reductions for the residual-augmented energy and the
-// residual norm (two passes, fixed grid, fixed order).
+// residual norm (energy_terms.cuh: one launch, fixed grid, fixed order).
 //   out[0] = sum r1^2, out[1] = sum r2^2,
 //   out[2] = sum (f_ai + r1) t1, out[3] = sum (g_abij + r2)(2 tau - tau(b,a,i,j))
-// partial: scratch of kReduceBlocks * 4 doubles.
 // ---------------------------------------------------------------------------
 constexpr int kReduceBlocks = 608;
-void launch_energy_terms(int64_t o, int64_t v, const double* r1, const double* r2,
-                         const double* f_ai, const double* g_abij, const double* t1,
-                         const double* tau, double* partial, double* out, cudaStream_t st);
+struct EnergyTermsArgs {
+  int64_t o, v;
+  const double* r1;
+  const double* r2;
+  const double* f_ai;
+  const double* g_abij;
+  const double* t1;
+  const double* t2;    // read when tau is null
+  const double* tau;
+  double* partial;     // kReduceBlocks * 4
+  unsigned* count;     // zero between launches
+  double* out;         // device memory, or pinned host memory
+};
+void launch_energy_terms(const EnergyTermsArgs& g, cudaStream_t st);
 
 // tau(a,b,i,j) = t2(a,b,i,j) + t1(a,i) t1(b,j)
 // Pair-(anti)symmetric ladder (see kernels.cu): G+/G- over (a <= b or any row
@@ -388,6 +398,7 @@ struct DiisDyn {
 };
 
 struct DiisArgs {
+  unsigned* count;     // zero between launches (the last block solves for the coefficients)
   const DiisDyn* dyn;  // non-NULL: slot, nvec, slots and extrapolate are read from here
   int64_t o, v;
   const double* eps_o;
@@ -462,7 +473,8 @@ struct SolveParams {
 void launch_solve_init(SolveState* s, int mixed, cudaStream_t st);
 // one thread: E, error, convergence test, phase switch, DIIS bookkeeping,
 // and the conditions of the loop, the update and the residual precision
-void launch_solve_decide(const SolveParams& p, cudaStream_t st);
+// the energy terms, then the iteration's decision in the same launch
+void launch_energy_decide(const EnergyTermsArgs& e, const SolveParams& p, cudaStream_t st);
 // nanosecond timestamp (globaltimer) of the current iteration's residual:
 // base[2 (iter - 1) + which]
 void launch_stamp(unsigned long long* base, const SolveState* s, int which, cudaStream_t st);

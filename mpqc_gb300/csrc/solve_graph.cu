@@ -1,7 +1,7 @@
 // Device side of the whole-solve CUDA graph: the per-iteration decision of
 // CCSD::compute_ccsd (src/mpqc/chemistry/qc/lcao/cc/ccsd.h:367-468) and
 // DIISSolver (src/mpqc/chemistry/qc/cc/solvers.h:112-121, 141-152) on one
-// thread, driving the graph's conditional nodes:
+// thread (of the energy kernel's last block), driving the graph's conditional nodes:
 //
 //   while (loop) {                      WHILE node, condition `loop`
 //     energy terms -> decide            E, error, convergence test, phase switch,
@@ -13,6 +13,7 @@
 //
 // It makes the same decisions, in the same order, as the host loop of
 // gbcc_solve (api.cpp), so both give identical iterations and energies.
+#include "energy_terms.cuh"
 #include "kernels.h"
 
 namespace gbcc {
@@ -28,7 +29,7 @@ __global__ void solve_init_kernel(SolveState* s, int mixed) {
   *s = z;
 }
 
-__global__ void solve_decide_kernel(SolveParams p) {
+__device__ void solve_decide(const SolveParams& p) {
   SolveState& s = *p.state;
   if (s.pending_reset) {
     // a new DIIS subspace for the FP64 refinement (requested at the previous update)
@@ -114,6 +115,10 @@ __global__ void solve_decide_kernel(SolveParams p) {
   cudaGraphSetConditional(p.cond_loop, s.iter < p.max_iter ? 1u : 0u);
 }
 
+__global__ void __launch_bounds__(kEnergyThreads) energy_decide_kernel(EnergyTermsArgs e, SolveParams p) {
+  if (energy_terms(e)) solve_decide(p);
+}
+
 // timestamps around the residual of the current iteration (iteration iter-1)
 __global__ void stamp_kernel(unsigned long long* base, const SolveState* s, int which) {
   unsigned long long t;
@@ -125,7 +130,9 @@ __global__ void stamp_kernel(unsigned long long* base, const SolveState* s, int 
 
 void launch_solve_init(SolveState* s, int mixed, cudaStream_t st) { solve_init_kernel<<<1, 1, 0, st>>>(s, mixed); }
 
-void launch_solve_decide(const SolveParams& p, cudaStream_t st) { solve_decide_kernel<<<1, 1, 0, st>>>(p); }
+void launch_energy_decide(const EnergyTermsArgs& e, const SolveParams& p, cudaStream_t st) {
+  energy_decide_kernel<<<energy_blocks(e.v), kEnergyThreads, 0, st>>>(e, p);
+}
 
 void launch_stamp(unsigned long long* base, const SolveState* s, int which, cudaStream_t st) {
   stamp_kernel<<<1, 1, 0, st>>>(base, s, which);
