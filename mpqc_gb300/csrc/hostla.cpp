@@ -57,12 +57,14 @@ void symmetrize(int n, double* A) {
 
 void eigh(int n, std::vector<double> A, std::vector<double>& w, std::vector<double>& V) {
   auto at = [&](int i, int j) -> double& { return A[static_cast<size_t>(i) * n + j]; };
+  // the transformation is kept transposed (row k: vector k), so that reflections
+  // and rotations run along contiguous rows
   std::vector<double> Q(static_cast<size_t>(n) * n, 0.0);
-  auto q = [&](int i, int j) -> double& { return Q[static_cast<size_t>(i) * n + j]; };
-  for (int i = 0; i < n; ++i) q(i, i) = 1.0;
+  auto qrow = [&](int k) { return Q.data() + static_cast<size_t>(k) * n; };
+  for (int i = 0; i < n; ++i) qrow(i)[i] = 1.0;
 
   // Householder: A <- H_k A H_k zeroes column k below the subdiagonal; Q <- Q H_k
-  std::vector<double> v(n), p(n), wv(n);
+  std::vector<double> v(n), p(n), wv(n), qv(n);
   for (int k = 0; k + 2 < n; ++k) {
     const int m = n - k - 1;  // trailing size
     double xn = 0.0;
@@ -79,13 +81,15 @@ void eigh(int n, std::vector<double> A, std::vector<double>& w, std::vector<doub
     const double beta = 2.0 / vn2;
     at(k + 1, k) = at(k, k + 1) = alpha;
     for (int i = 1; i < m; ++i) at(k + 1 + i, k) = at(k, k + 1 + i) = 0.0;
-    // trailing block B <- H B H = B - v w^T - w v^T, w = p - (beta/2)(p.v) v, p = beta B v
-    for (int i = 0; i < m; ++i) {
-      double s = 0.0;
-      const double* row = &at(k + 1 + i, k + 1);
-      for (int j = 0; j < m; ++j) s += row[j] * v[j];
-      p[i] = beta * s;
+    // trailing block B <- H B H = B - v w^T - w v^T, w = p - (beta/2)(p.v) v, p =
+    // beta B v (B symmetric: summed over its rows)
+    std::fill(p.begin(), p.begin() + m, 0.0);
+    for (int j = 0; j < m; ++j) {
+      const double* row = &at(k + 1 + j, k + 1);
+      const double vj = v[j];
+      for (int i = 0; i < m; ++i) p[i] += row[i] * vj;
     }
+    for (int i = 0; i < m; ++i) p[i] *= beta;
     double pv = 0.0;
     for (int i = 0; i < m; ++i) pv += p[i] * v[i];
     const double kk = 0.5 * beta * pv;
@@ -95,12 +99,16 @@ void eigh(int n, std::vector<double> A, std::vector<double>& w, std::vector<doub
       for (int j = 0; j < m; ++j) row[j] -= v[i] * wv[j] + wv[i] * v[j];
     }
     // Q[:, k+1:] -= beta (Q[:, k+1:] v) v^T
-    for (int r = 0; r < n; ++r) {
-      double* row = &q(r, k + 1);
-      double s = 0.0;
-      for (int j = 0; j < m; ++j) s += row[j] * v[j];
-      s *= beta;
-      for (int j = 0; j < m; ++j) row[j] -= s * v[j];
+    std::fill(qv.begin(), qv.end(), 0.0);
+    for (int j = 0; j < m; ++j) {
+      const double* row = qrow(k + 1 + j);
+      const double vj = v[j];
+      for (int r = 0; r < n; ++r) qv[r] += row[r] * vj;
+    }
+    for (int j = 0; j < m; ++j) {
+      double* row = qrow(k + 1 + j);
+      const double bv = beta * v[j];
+      for (int r = 0; r < n; ++r) row[r] -= qv[r] * bv;
     }
   }
   std::vector<double> d(n), e(n > 1 ? n - 1 : 1, 0.0);
@@ -129,7 +137,9 @@ void eigh(int n, std::vector<double> A, std::vector<double>& w, std::vector<doub
     const double mu = d[hi] - eh * eh / (dl + sg * std::hypot(dl, eh));
     double x = d[lo] - mu, z = e[lo];
     for (int k = lo; k < hi; ++k) {
-      const double r = std::hypot(x, z);
+      // (hypot guards a range that the sums rarely leave, at the cost of the rotation)
+      const double h2 = x * x + z * z;
+      const double r = (h2 > 1e-280 && h2 < 1e280) ? std::sqrt(h2) : std::hypot(x, z);
       const double c = r == 0.0 ? 1.0 : x / r, s = r == 0.0 ? 0.0 : z / r;
       // rows/columns k, k+1 of T rotated by R = [c s; -s c]: T <- R T R^T
       if (k > lo) e[k - 1] = r;  // the bulge of the previous step is absorbed
@@ -142,10 +152,12 @@ void eigh(int n, std::vector<double> A, std::vector<double>& w, std::vector<doub
         bulge = s * e[k + 1];
         e[k + 1] *= c;
       }
+      double* __restrict__ q0 = qrow(k);
+      double* __restrict__ q1 = qrow(k + 1);
       for (int i = 0; i < n; ++i) {
-        const double qk = q(i, k), qk1 = q(i, k + 1);
-        q(i, k) = c * qk + s * qk1;
-        q(i, k + 1) = -s * qk + c * qk1;
+        const double qk = q0[i], qk1 = q1[i];
+        q0[i] = c * qk + s * qk1;
+        q1[i] = c * qk1 - s * qk;
       }
       x = e[k];
       z = bulge;
@@ -158,7 +170,8 @@ void eigh(int n, std::vector<double> A, std::vector<double>& w, std::vector<doub
   V.assign(static_cast<size_t>(n) * n, 0.0);
   for (int j = 0; j < n; ++j) {
     w[j] = d[order[j]];
-    for (int i = 0; i < n; ++i) V[static_cast<size_t>(i) * n + j] = q(i, order[j]);
+    const double* row = qrow(order[j]);
+    for (int i = 0; i < n; ++i) V[static_cast<size_t>(i) * n + j] = row[i];
   }
 }
 

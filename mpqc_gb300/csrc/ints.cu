@@ -22,6 +22,7 @@
 // F_0 = (pi/T)^{1/2} / 2 and the upward recurrence.
 #include "ints.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -404,7 +405,8 @@ void launch_eri_t(const EriArgs& a, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
-// one-body integrals: one thread per Cartesian function pair
+// one-body integrals: one warp per Cartesian function pair mu >= nu, its lanes on
+// the nuclei (a thread per pair and all nuclei: 2.1 ms for four waters in 6-31G**)
 
 struct OneBodyKernelArgs {
   OneBodyArgs a;
@@ -448,10 +450,14 @@ __global__ void __launch_bounds__(128) one_body_kernel(OneBodyKernelArgs ka) {
   __shared__ STab tab;
   load_tables(ka.herm, &tab);
   __syncthreads();
-  const int64_t n = a.ncart_total;
-  const int64_t id = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (id >= n * n) return;
-  const int mu = static_cast<int>(id / n), nu = static_cast<int>(id % n);
+  const int n = a.ncart_total;
+  const int lane = threadIdx.x & 31;
+  const int id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (id >= n * (n + 1) / 2) return;
+  int mu = static_cast<int>((sqrtf(8.0f * static_cast<float>(id) + 1.0f) - 1.0f) * 0.5f);
+  while (mu * (mu + 1) / 2 > id) --mu;
+  while ((mu + 1) * (mu + 2) / 2 <= id) ++mu;
+  const int nu = id - mu * (mu + 1) / 2;
   const int sA = a.cf_shell[mu], sB = a.cf_shell[nu];
   const int cA = a.cf_comp[mu], cB = a.cf_comp[nu];
   const int ia[3] = {cA >> 4, (cA >> 2) & 3, cA & 3};
@@ -482,7 +488,7 @@ __global__ void __launch_bounds__(128) one_body_kernel(OneBodyKernelArgs ka) {
       s += cw * s1[0] * s1[1] * s1[2];
       t += cw * (t1[0] * s1[1] * s1[2] + s1[0] * t1[1] * s1[2] + s1[0] * s1[1] * t1[2]);
       const double P[3] = {(ea * A[0] + eb * B[0]) / p, (ea * A[1] + eb * B[1]) / p, (ea * A[2] + eb * B[2]) / p};
-      for (int c = 0; c < a.natom; ++c) {
+      for (int c = lane; c < a.natom; c += 32) {
         hermite_r(L, R, P[0] - a.atom_xyz[3 * c], P[1] - a.atom_xyz[3 * c + 1], P[2] - a.atom_xyz[3 * c + 2], p,
                   1.0, a.boys, tab);
         double h = 0.0;
@@ -502,9 +508,14 @@ __global__ void __launch_bounds__(128) one_body_kernel(OneBodyKernelArgs ka) {
       }
     }
   }
-  a.S[id] = s;
-  a.T[id] = t;
-  a.V[id] = v;
+  v = warp_sum(v);
+  if (lane == 0) {
+    for (const int64_t at : {static_cast<int64_t>(mu) * n + nu, static_cast<int64_t>(nu) * n + mu}) {
+      a.S[at] = s;
+      a.T[at] = t;
+      a.V[at] = v;
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -521,24 +532,103 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   return r;
 }
 
-// one block per (mu, nu): J = sum G[mu nu la si] D[la si], K = sum G[mu la nu si] D[la si]
+// One block per mu >= nu: J = sum G[mu nu la si] D[la si], K = sum G[mu la nu si]
+// D[la si], both symmetric for a symmetric D.  A warp takes whole rows la, its
+// lanes si, so no index is divided (64-bit divisions occupy the FP64 pipe that
+// the sums need: all pairs with one division per element took 411 us at n = 100).
 __global__ void __launch_bounds__(256) jk_kernel(int n, const double* __restrict__ G, const double* __restrict__ D,
                                                 double* J, double* K) {
   __shared__ double sh[8];
-  const int64_t nn = n;
-  const int64_t mu = blockIdx.x / n, nu = blockIdx.x % n;
-  const double* gj = G + (mu * nn + nu) * nn * nn;
+  const int id = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int mu = static_cast<int>((sqrtf(8.0f * static_cast<float>(id) + 1.0f) - 1.0f) * 0.5f);
+  while (mu * (mu + 1) / 2 > id) --mu;
+  while ((mu + 1) * (mu + 2) / 2 <= id) ++mu;
+  const int nu = id - mu * (mu + 1) / 2;
+  const int64_t nn = n, n2 = nn * nn;
+  const double* gj = G + (mu * nn + nu) * n2;
+  const double* gk = G + mu * nn * n2 + nu * nn;
   double sj = 0.0, sk = 0.0;
-  for (int64_t x = threadIdx.x; x < nn * nn; x += blockDim.x) sj = fma(gj[x], D[x], sj);
-  for (int64_t x = threadIdx.x; x < nn * nn; x += blockDim.x) {
-    const int64_t la = x / nn, si = x % nn;
-    sk = fma(G[((mu * nn + la) * nn + nu) * nn + si], D[x], sk);
+  // four rows at a time: twelve loads in flight
+  for (int la = 4 * warp; la < n; la += 32) {
+    for (int si = lane; si < n; si += 32) {
+      double x[4], yj[4], yk[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool in = la + u < n;
+        x[u] = in ? D[(la + u) * nn + si] : 0.0;
+        yj[u] = in ? __ldcs(gj + (la + u) * nn + si) : 0.0;
+        yk[u] = in ? __ldcs(gk + (la + u) * n2 + si) : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        sj = fma(yj[u], x[u], sj);
+        sk = fma(yk[u], x[u], sk);
+      }
+    }
   }
   sj = block_sum(sj, sh);
   sk = block_sum(sk, sh);
   if (threadIdx.x == 0) {
-    J[mu * nn + nu] = sj;
-    K[mu * nn + nu] = sk;
+    J[mu * nn + nu] = J[nu * nn + mu] = sj;
+    K[mu * nn + nu] = K[nu * nn + mu] = sk;
+  }
+}
+
+// row i of F = H + 2 J - K (symmetrised H), and its share sum_j D (H + F) of the energy
+__global__ void __launch_bounds__(128) fock_kernel(int n, const double* __restrict__ H, const double* __restrict__ J,
+                                                   const double* __restrict__ K, const double* __restrict__ D,
+                                                   double* __restrict__ F, double* __restrict__ rows, int ld) {
+  __shared__ double sh[8];
+  const int i = blockIdx.x;
+  double e = 0.0;
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+    const int64_t ij = static_cast<int64_t>(i) * n + j, ji = static_cast<int64_t>(j) * n + i;
+    const double g = 2.0 * J[ij] - K[ij];
+    e = fma(D[ij], H[ij] + (H[ij] + g), e);
+    F[ij] = 0.5 * ((H[ij] + g) + (H[ji] + (2.0 * J[ji] - K[ji])));
+  }
+  e = block_sum(e, sh);
+  if (threadIdx.x == 0) rows[static_cast<int64_t>(i) * ld] = e;
+}
+
+// slots of a DIIS step and their coefficients, as a launch argument
+constexpr int kListMax = 16;
+struct SlotList {
+  int n, first;  // entries, and how many of the whole list come before them
+  int slot[kListMax];
+  double coef[kListMax];
+};
+
+// row i of the orbital gradient G = X - X^T (X = F D S, X^T = S D F) into its
+// slot (first part of the list only), and the row's share of <G, G_q> for the
+// listed slots (the new one among them)
+__global__ void __launch_bounds__(128) gradient_kernel(int n, const double* __restrict__ X, double* slots,
+                                                       int64_t slot_stride, int slot, SlotList list,
+                                                       double* __restrict__ rows, int ld) {
+  __shared__ double sh[8];
+  const int i = blockIdx.x;
+  double* out = slots + slot * slot_stride + static_cast<int64_t>(i) * n;
+  if (list.first == 0)
+    for (int j = threadIdx.x; j < n; j += blockDim.x)
+      out[j] = X[static_cast<int64_t>(i) * n + j] - X[static_cast<int64_t>(j) * n + i];
+  __syncthreads();
+  for (int q = 0; q < list.n; ++q) {
+    const double* gq = slots + list.slot[q] * slot_stride + static_cast<int64_t>(i) * n;
+    double s = 0.0;
+    for (int j = threadIdx.x; j < n; j += blockDim.x) s = fma(out[j], gq[j], s);
+    s = block_sum(s, sh);
+    if (threadIdx.x == 0) rows[static_cast<int64_t>(i) * ld + 1 + list.first + q] = s;
+  }
+}
+
+// out (+)= sum_q coef[q] slots[slot[q]], overwritten by the first part of the list
+__global__ void __launch_bounds__(256) combine_kernel(int64_t n, const double* __restrict__ slots, int64_t slot_stride,
+                                                      SlotList list, double* __restrict__ out) {
+  for (int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < n;
+       k += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    double s = list.first ? out[k] : 0.0;
+    for (int q = 0; q < list.n; ++q) s = fma(list.coef[q], slots[list.slot[q] * slot_stride + k], s);
+    out[k] = s;
   }
 }
 
@@ -596,15 +686,52 @@ void launch_eri_class(int cP, int cQ, const EriArgs& a, cudaStream_t st) {
 }
 
 void launch_one_body(const OneBodyArgs& a, cudaStream_t st) {
-  const int64_t n2 = static_cast<int64_t>(a.ncart_total) * a.ncart_total;
-  if (n2 == 0) return;
+  const int64_t pairs = static_cast<int64_t>(a.ncart_total) * (a.ncart_total + 1) / 2;
+  if (pairs == 0) return;
   OneBodyKernelArgs ka{a, device_tables()};
-  one_body_kernel<<<static_cast<unsigned>((n2 + 127) / 128), 128, 0, st>>>(ka);
+  one_body_kernel<<<static_cast<unsigned>((pairs + 3) / 4), 128, 0, st>>>(ka);
 }
 
 void launch_coulomb_exchange(int n, const double* G, const double* D, double* J, double* K, cudaStream_t st) {
   if (n <= 0) return;
-  jk_kernel<<<static_cast<unsigned>(n * n), 256, 0, st>>>(n, G, D, J, K);
+  jk_kernel<<<static_cast<unsigned>(n * (n + 1) / 2), 256, 0, st>>>(n, G, D, J, K);
+}
+
+void launch_fock(int n, const double* H, const double* J, const double* K, const double* D, double* F, double* rows,
+                 int ld, cudaStream_t st) {
+  fock_kernel<<<static_cast<unsigned>(n), 128, 0, st>>>(n, H, J, K, D, F, rows, ld);
+}
+
+namespace {
+template <class F>
+void for_parts(const std::vector<int>& order, const double* coef, F&& f) {
+  for (size_t q0 = 0; q0 < order.size(); q0 += kListMax) {
+    SlotList l{};
+    l.first = static_cast<int>(q0);
+    l.n = static_cast<int>(std::min<size_t>(kListMax, order.size() - q0));
+    for (int q = 0; q < l.n; ++q) {
+      l.slot[q] = order[q0 + q];
+      l.coef[q] = coef ? coef[q0 + q] : 0.0;
+    }
+    f(l);
+  }
+}
+}  // namespace
+
+void launch_scf_gradient(int n, const double* X, double* slots, int slot, const std::vector<int>& order, double* rows,
+                         int ld, cudaStream_t st) {
+  for_parts(order, nullptr, [&](const SlotList& l) {
+    gradient_kernel<<<static_cast<unsigned>(n), 128, 0, st>>>(n, X, slots, static_cast<int64_t>(n) * n, slot, l, rows,
+                                                              ld);
+  });
+}
+
+void launch_scf_combine(int n, const double* slots, const std::vector<int>& order, const std::vector<double>& coef,
+                        double* out, cudaStream_t st) {
+  const int64_t n2 = static_cast<int64_t>(n) * n;
+  for_parts(order, coef.data(), [&](const SlotList& l) {
+    combine_kernel<<<static_cast<unsigned>((n2 + 255) / 256), 256, 0, st>>>(n2, slots, n2, l, out);
+  });
 }
 
 void launch_mo_block(int64_t n, const double* mo, const int64_t dims[4], const int perm[4], const int64_t off[4],

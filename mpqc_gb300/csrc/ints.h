@@ -106,8 +106,20 @@ struct OneBodyArgs {
 void launch_one_body(const OneBodyArgs& a, cudaStream_t st);
 
 // Fock contributions from the stored (mu nu|la si): J = (mu nu|la si) D_la_si,
-// K = (mu la|nu si) D_la_si, deterministic per element.
+// K = (mu la|nu si) D_la_si for a symmetric D, deterministic per element.
 void launch_coulomb_exchange(int n, const double* G, const double* D, double* J, double* K, cudaStream_t st);
+
+// RHF steps on n x n matrices.  F = H + 2 J - K symmetrised, rows[i ld] = sum_j
+// D_ij (H + F)_ij.
+void launch_fock(int n, const double* H, const double* J, const double* K, const double* D, double* F, double* rows,
+                 int ld, cudaStream_t st);
+// slot = X - X^T (the orbital gradient for X = F D S), rows[i ld + 1 + q] = row
+// i's share of <slot, order[q]>
+void launch_scf_gradient(int n, const double* X, double* slots, int slot, const std::vector<int>& order, double* rows,
+                         int ld, cudaStream_t st);
+// out = sum_q coef[q] slots[order[q]]
+void launch_scf_combine(int n, const double* slots, const std::vector<int>& order, const std::vector<double>& coef,
+                        double* out, cudaStream_t st);
 
 // out[x0][x1][x2][x3] = mo[o + x permuted]: the MO block extraction, with
 // mo[p][q][r][s] = (pq|rs) over n orbitals; perm[k] = position in `out` of mo

@@ -351,6 +351,27 @@ void build_integrals(gbcc_scf* h, const gbcc_molecule* mol, const gbcc_basis* bs
   ea.nbf = N;
   ea.pure = h->pure;
   ea.G = h->d_G;
+  // the classes write disjoint quartets: their kernels run side by side on a few
+  // streams (one after the other, each class's last blocks leave the chip idle)
+  struct Streams {
+    cudaStream_t s[4] = {};
+    cudaEvent_t e = nullptr;
+    ~Streams() {
+      for (cudaStream_t x : s)
+        if (x) {
+          cudaStreamSynchronize(x);
+          cudaStreamDestroy(x);
+        }
+      if (e) cudaEventDestroy(e);
+    }
+  } par;
+  GBCC_CK(cudaEventCreateWithFlags(&par.e, cudaEventDisableTiming));
+  GBCC_CK(cudaEventRecord(par.e, st));
+  for (cudaStream_t& x : par.s) {
+    GBCC_CK(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+    GBCC_CK(cudaStreamWaitEvent(x, par.e, 0));
+  }
+  int next = 0;
   for (int cp = 0; cp < I::kNumPairClasses; ++cp)
     for (int cq = 0; cq <= cp; ++cq) {
       ea.p0 = cls_start[cp];
@@ -359,34 +380,115 @@ void build_integrals(gbcc_scf* h, const gbcc_molecule* mol, const gbcc_basis* bs
       ea.nq = cls_start[cq + 1] - cls_start[cq];
       ea.same = cp == cq;
       ea.nquart = ea.same ? static_cast<int64_t>(ea.np) * (ea.np + 1) / 2 : static_cast<int64_t>(ea.np) * ea.nq;
-      I::launch_eri_class(cp, cq, ea, st);
+      if (ea.nquart == 0) continue;
+      I::launch_eri_class(cp, cq, ea, par.s[next++ % 4]);
       GBCC_CK(cudaGetLastError());
     }
+  for (cudaStream_t x : par.s) GBCC_CK(cudaStreamSynchronize(x));
   GBCC_CK(cudaStreamSynchronize(st));
   h->t_eri = now_s() - t1;
 }
 
-// orbitals of Fock matrix F: eigenvectors of X^T F X, C = X C'
-void diagonalise_fock(const gbcc_scf* h, const std::vector<double>& F, std::vector<double>& C,
-                      std::vector<double>& eps) {
-  const int N = h->nbf;
-  std::vector<double> tmp(static_cast<size_t>(N) * N), Fp(static_cast<size_t>(N) * N), V;
-  gbcc::hostla::gemm_tn(N, N, N, h->X.data(), F.data(), tmp.data());   // X^T F
-  gbcc::hostla::gemm_nn(N, N, N, tmp.data(), h->X.data(), Fp.data());  // X^T F X
-  gbcc::hostla::symmetrize(N, Fp.data());
-  gbcc::hostla::eigh(N, Fp, eps, V);
-  C.assign(static_cast<size_t>(N) * N, 0.0);
-  gbcc::hostla::gemm_nn(N, N, N, h->X.data(), V.data(), C.data());
-}
-
-void density(int N, int nocc, const std::vector<double>& C, std::vector<double>& D) {
-  D.assign(static_cast<size_t>(N) * N, 0.0);
-  for (int i = 0; i < N; ++i)
-    for (int j = 0; j < N; ++j) {
-      double s = 0.0;
-      for (int k = 0; k < nocc; ++k) s += C[static_cast<size_t>(i) * N + k] * C[static_cast<size_t>(j) * N + k];
-      D[static_cast<size_t>(i) * N + j] = s;
+// The SCF iteration's matrices on the device (n x n each) and its products on
+// the in-place FP64 kernel (gemm_small.cu).
+class ScfDevice {
+ public:
+  ScfDevice(int n, int nocc, int n_diis, cudaStream_t st) : n_(n), st_(st), n2_(static_cast<size_t>(n) * n) {
+    ld_ = n_diis + 1;
+    gbcc::GemmSmallArgs g{};
+    g.M = g.N = n;
+    g.K = std::max(n, nocc);
+    gbcc::plan_gemm_small(g);
+    size_t partial = g.partial_elems, tiles = static_cast<size_t>(g.tiles);
+    g.K = std::max(nocc, 1);
+    gbcc::plan_gemm_small(g);
+    partial = std::max(partial, g.partial_elems);
+    tiles = std::max(tiles, static_cast<size_t>(g.tiles));
+    const size_t doubles = n2_ * (8 + 2 * n_diis) + static_cast<size_t>(n) * ld_ + partial;
+    const size_t words = static_cast<size_t>(n) * 2 * sizeof(int64_t) + tiles * sizeof(unsigned);
+    buf_ = std::make_unique<DevBuf>(doubles * sizeof(double) + words + 256);
+    double* p = buf_->as<double>();
+    auto take = [&](size_t k) {
+      double* q = p;
+      p += k;
+      return q;
+    };
+    H = take(n2_), S = take(n2_), X = take(n2_), F = take(n2_), C = take(n2_), V = take(n2_), T = take(n2_), T2 = take(n2_);
+    fs = take(n2_ * n_diis), gs = take(n2_ * n_diis);
+    rows = take(static_cast<size_t>(n) * ld_), partial_ = take(partial);
+    step_ = reinterpret_cast<int64_t*>(p);
+    unit_ = step_ + n;
+    count_ = reinterpret_cast<unsigned*>(unit_ + n);
+    std::vector<int64_t> tab(2 * static_cast<size_t>(n));
+    for (int i = 0; i < n; ++i) {
+      tab[i] = static_cast<int64_t>(i) * n;
+      tab[n + i] = i;
     }
+    GBCC_CK(cudaMemcpyAsync(step_, tab.data(), tab.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+    GBCC_CK(cudaMemsetAsync(count_, 0, tiles * sizeof(unsigned), st));
+    GBCC_CK(cudaStreamSynchronize(st));
+  }
+  int ld() const { return ld_; }
+  void up(double* dst, const std::vector<double>& src) {
+    GBCC_CK(cudaMemcpyAsync(dst, src.data(), src.size() * sizeof(double), cudaMemcpyHostToDevice, st_));
+  }
+  void down(std::vector<double>& dst, const double* src) {
+    GBCC_CK(cudaMemcpyAsync(dst.data(), src, dst.size() * sizeof(double), cudaMemcpyDeviceToHost, st_));
+  }
+  // C = A B (or A^T B, A B^T) over K inner elements, n x n row-major arrays
+  void product(const double* A, bool ta, const double* B, bool tb, double* Cm, int K) {
+    if (K < 1) {
+      GBCC_CK(cudaMemsetAsync(Cm, 0, n2_ * sizeof(double), st_));
+      return;
+    }
+    gbcc::GemmSmallArgs g{};
+    g.M = g.N = n_;
+    g.K = K;
+    auto operand = [&](gbcc::GatherArgs& x, const double* a, bool along_rows) {
+      x.nterms = x.plain = 1;
+      x.t[0].a = a;
+      x.t[0].ra = along_rows ? unit_ : step_;
+      x.t[0].ca = along_rows ? step_ : unit_;
+      x.transpose = along_rows ? 1 : 0;
+    };
+    operand(g.a, A, ta);
+    operand(g.b, B, !tb);
+    g.C = Cm;
+    g.cm = step_;
+    g.cn = unit_;
+    g.alpha = 1.0;
+    gbcc::plan_gemm_small(g);
+    g.partial = partial_;
+    g.count = count_;
+    gbcc::launch_gemm_small(g, st_);
+    GBCC_CK(cudaGetLastError());
+  }
+
+  double *H, *S, *X, *F, *C, *V, *T, *T2, *fs, *gs, *rows;
+  std::vector<double> V_host;  // source of the copy in flight
+
+ private:
+  int n_, ld_;
+  cudaStream_t st_;
+  size_t n2_;
+  std::unique_ptr<DevBuf> buf_;
+  double* partial_ = nullptr;
+  int64_t *step_ = nullptr, *unit_ = nullptr;
+  unsigned* count_ = nullptr;
+};
+
+// orbitals of the Fock matrix F (device): eigenvectors of X^T F X on the host, C = X C'
+void diagonalise_fock(gbcc_scf* h, ScfDevice& d, const double* F, std::vector<double>& eps) {
+  const int N = h->nbf;
+  std::vector<double> Fp(static_cast<size_t>(N) * N);
+  d.product(d.X, true, F, false, d.T, N);
+  d.product(d.T, false, d.X, false, d.T2, N);
+  d.down(Fp, d.T2);
+  GBCC_CK(cudaStreamSynchronize(h->stream));
+  gbcc::hostla::symmetrize(N, Fp.data());
+  gbcc::hostla::eigh(N, std::move(Fp), eps, d.V_host);
+  d.up(d.V, d.V_host);
+  d.product(d.X, false, d.V, false, d.C, N);
 }
 
 // rows x K panel times C: dst[cm[r] + cn[s]] = sum_k src[r K + k] C[k][s], in row chunks
@@ -500,13 +602,12 @@ gbcc_status gbcc_scf_create(gbcc_scf** out, const gbcc_molecule* mol, const gbcc
     gbcc::hostla::eigh(N, Sc, w, U);
     if (!(w[0] > 1e-10)) throw Error(GBCC_ERR_INVALID_ARG, "overlap matrix (near) singular");
     h->X.assign(static_cast<size_t>(N) * N, 0.0);
-    for (int i = 0; i < N; ++i)
-      for (int j = 0; j < N; ++j) {
-        double s = 0.0;
-        for (int k = 0; k < N; ++k)
-          s += U[static_cast<size_t>(i) * N + k] * U[static_cast<size_t>(j) * N + k] / std::sqrt(w[k]);
-        h->X[static_cast<size_t>(i) * N + j] = s;
-      }
+    std::vector<double> Ut(static_cast<size_t>(N) * N);
+    for (int k = 0; k < N; ++k) {
+      const double r = 1.0 / std::sqrt(w[k]);
+      for (int j = 0; j < N; ++j) Ut[static_cast<size_t>(k) * N + j] = r * U[static_cast<size_t>(j) * N + k];
+    }
+    gbcc::hostla::gemm_nn(N, N, N, U.data(), Ut.data(), h->X.data());
     h->d_D = static_cast<double*>(gbcc::dev_alloc(sizeof(double) * N * N));
     h->d_J = static_cast<double*>(gbcc::dev_alloc(sizeof(double) * N * N));
     h->d_K = static_cast<double*>(gbcc::dev_alloc(sizeof(double) * N * N));
@@ -528,40 +629,47 @@ gbcc_status gbcc_scf_run(gbcc_scf* h, gbcc_scf_report* report) {
     const int N = h->nbf, nocc = h->nocc;
     const size_t NN = static_cast<size_t>(N) * N;
     const double t0 = now_s();
-    std::vector<double> C, eps, D, J(NN), K(NN), F(NN), FDS(NN), SDF(NN), tmp(NN), tmp2(NN);
-    diagonalise_fock(h, h->H, C, eps);  // core-Hamiltonian guess
-    density(N, nocc, C, D);
-    std::vector<std::vector<double>> fs, gs;
+    // The Fock build, the products and the DIIS vectors stay on the device; the
+    // host diagonalises, solves the DIIS system and tests convergence.
+    const int nd = std::max(h->cfg.n_diis, 1);
+    ScfDevice d(N, nocc, nd, h->stream);
+    d.up(d.H, h->H);
+    d.up(d.S, h->S);
+    d.up(d.X, h->X);
+    std::vector<double> eps, rows(static_cast<size_t>(N) * d.ld());
+    diagonalise_fock(h, d, d.H, eps);  // core-Hamiltonian guess
+    std::vector<int> order;            // slots, oldest first
+    std::vector<std::vector<double>> B(nd, std::vector<double>(nd, 0.0));  // <G, G> by slot
+    int slot = -1;
     const double thr = h->cfg.threshold;
     double e_old = 0.0, de = 1.0, grad = 1.0;
     bool conv = false;
     int it = 0;
     if (h->cfg.verbose) std::printf("Starting SCF:\n\tThreshold: %g\n\tMaximum number of iterations: %d\n", thr, h->cfg.max_iter);
     while (it < h->cfg.max_iter) {
-      GBCC_CK(cudaMemcpyAsync(h->d_D, D.data(), NN * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+      d.product(d.C, false, d.C, true, h->d_D, nocc);  // density of the occupied columns
       gbcc::ints::launch_coulomb_exchange(N, h->d_G, h->d_D, h->d_J, h->d_K, h->stream);
+      slot = (slot + 1) % nd;
+      if (static_cast<int>(order.size()) == nd) order.erase(order.begin());
+      order.push_back(slot);
+      const int m = static_cast<int>(order.size());
+      double* F = d.fs + slot * NN;
+      gbcc::ints::launch_fock(N, d.H, h->d_J, h->d_K, h->d_D, F, d.rows, d.ld(), h->stream);
+      // orbital gradient FDS - SDF and its products with the stored ones
+      d.product(F, false, h->d_D, false, d.T, N);
+      d.product(d.T, false, d.S, false, d.T2, N);
+      gbcc::ints::launch_scf_gradient(N, d.T2, d.gs, slot, order, d.rows, d.ld(), h->stream);
       GBCC_CK(cudaGetLastError());
-      GBCC_CK(cudaMemcpyAsync(J.data(), h->d_J, NN * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-      GBCC_CK(cudaMemcpyAsync(K.data(), h->d_K, NN * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+      d.down(rows, d.rows);
       GBCC_CK(cudaStreamSynchronize(h->stream));
       double e = h->e_nuc;
-      for (size_t k = 0; k < NN; ++k) {
-        F[k] = h->H[k] + 2.0 * J[k] - K[k];
-        e += D[k] * (h->H[k] + F[k]);
+      for (int i = 0; i < N; ++i) e += rows[static_cast<size_t>(i) * d.ld()];
+      for (int q = 0; q < m; ++q) {
+        double s = 0.0;
+        for (int i = 0; i < N; ++i) s += rows[static_cast<size_t>(i) * d.ld() + 1 + q];
+        B[slot][order[q]] = B[order[q]][slot] = s;
       }
-      gbcc::hostla::symmetrize(N, F.data());
-      // orbital gradient FDS - SDF
-      gbcc::hostla::gemm_nn(N, N, N, F.data(), D.data(), tmp.data());
-      gbcc::hostla::gemm_nn(N, N, N, tmp.data(), h->S.data(), FDS.data());
-      gbcc::hostla::gemm_nn(N, N, N, h->S.data(), D.data(), tmp2.data());
-      gbcc::hostla::gemm_nn(N, N, N, tmp2.data(), F.data(), SDF.data());
-      double g2 = 0.0;
-      std::vector<double> G(NN);
-      for (size_t k = 0; k < NN; ++k) {
-        G[k] = FDS[k] - SDF[k];
-        g2 += G[k] * G[k];
-      }
-      grad = std::sqrt(g2) / static_cast<double>(NN);
+      grad = std::sqrt(B[slot][slot]) / static_cast<double>(NN);
       de = std::fabs(e - e_old);
       e_old = e;
       ++it;
@@ -569,42 +677,35 @@ gbcc_status gbcc_scf_run(gbcc_scf* h, gbcc_scf_report* report) {
         std::printf("iteration: %d\n\tEnergy: %.15f\n\tabs(Energy Change): %.3e\n\t(Gradient Norm)/n^2: %.3e\n", it, e,
                     de, grad);
       if (!std::isfinite(e)) throw Error(GBCC_ERR_NUMERIC, "non-finite SCF energy");
-      h->F = F;
       h->energy = e;
       if (it > 1 && de <= thr && grad <= thr) {
         conv = true;
         break;
       }
       // DIIS on F with the gradient (Pulay)
-      fs.push_back(F);
-      gs.push_back(G);
-      if (static_cast<int>(fs.size()) > h->cfg.n_diis) {
-        fs.erase(fs.begin());
-        gs.erase(gs.begin());
-      }
-      const int m = static_cast<int>(fs.size());
-      std::vector<double> B((m + 1) * (m + 1), -1.0), rhs(m + 1, 0.0);
-      B[m * (m + 1) + m] = 0.0;
+      std::vector<double> A((m + 1) * (m + 1), -1.0), rhs(m + 1, 0.0), coef;
+      A[m * (m + 1) + m] = 0.0;
       rhs[m] = -1.0;
       for (int i = 0; i < m; ++i)
-        for (int j = 0; j <= i; ++j) {
-          double s = 0.0;
-          for (size_t k = 0; k < NN; ++k) s += gs[i][k] * gs[j][k];
-          B[i * (m + 1) + j] = B[j * (m + 1) + i] = s;
-        }
-      std::vector<double> coef;
-      std::vector<double> Fd(NN, 0.0);
-      if (gbcc::hostla::solve(m + 1, B, rhs, coef)) {
-        for (int i = 0; i < m; ++i)
-          for (size_t k = 0; k < NN; ++k) Fd[k] += coef[i] * fs[i][k];
-      } else {
-        Fd = F;
+        for (int j = 0; j < m; ++j) A[i * (m + 1) + j] = B[order[i]][order[j]];
+      const double* Fd = F;
+      if (gbcc::hostla::solve(m + 1, A, rhs, coef)) {
+        gbcc::ints::launch_scf_combine(N, d.fs, order, coef, d.F, h->stream);
+        GBCC_CK(cudaGetLastError());
+        Fd = d.F;
       }
-      diagonalise_fock(h, Fd, C, eps);
-      density(N, nocc, C, D);
+      diagonalise_fock(h, d, Fd, eps);
     }
     // canonical orbitals of the last Fock matrix
-    diagonalise_fock(h, h->F, h->C, h->eps);
+    h->F.resize(NN);
+    h->C.resize(NN);
+    h->eps = eps;
+    if (slot >= 0) {
+      d.down(h->F, d.fs + slot * NN);
+      diagonalise_fock(h, d, d.fs + slot * NN, h->eps);
+    }
+    d.down(h->C, d.C);
+    GBCC_CK(cudaStreamSynchronize(h->stream));
     h->scf_done = true;
     h->iters = it;
     h->converged = conv;
