@@ -107,6 +107,13 @@ int gbcc_testing_dmma_peak(double* gflops);
  * vectors dropped. */
 int gbcc_testing_diis_coefficients(int32_t n, const double* B, double damping, double* coef, int32_t* nskip);
 
+/* The last pass of r2 (kernels.h, launch_r2_assemble) on host arrays r2u, tmp,
+ * g, r2 [v][v][o][o], Bp [v(v+1)/2][o(o+1)/2] and Bm [v(v-1)/2][o(o-1)/2]
+ * (either may be NULL), run repeat times from the same r2; *ms (may be NULL):
+ * the time of one. */
+int gbcc_testing_r2_assemble(int64_t o, int64_t v, const double* r2u, const double* tmp, const double* g,
+                             const double* Bp, const double* Bm, int accumulate, double* r2, int repeat, float* ms);
+
 /* Device allocations of the engine: *count (may be NULL) receives how many
  * were made so far in the process; from now on `after` more succeed and the
  * next one fails with GBCC_ERR_OOM as if the device were full (-1: none fails). */

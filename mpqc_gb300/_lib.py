@@ -37,7 +37,7 @@ SCF_EXPORTS = (
     "gbcc_scf_ccsd_inputs", "gbcc_scf_destroy", "gbcc_last_scf_error",
 )
 # test hooks of include/gbcc_testing.h
-TESTING_EXPORTS = ("gbcc_testing_gemm", "gbcc_testing_gemm_ex", "gbcc_testing_gemm_ex2", "gbcc_testing_gemm_ex3", "gbcc_testing_gemm_small", "gbcc_testing_split", "gbcc_testing_scale", "gbcc_testing_fp64_peak", "gbcc_testing_dmma_peak", "gbcc_testing_diis_coefficients", "gbcc_testing_fail_alloc", "gbcc_testing_fixed_split", "gbcc_testing_gemm_fp64tc", "gbcc_testing_gemm_timeout", "gbcc_testing_triples_chunk", "gbcc_testing_profile_residual",
+TESTING_EXPORTS = ("gbcc_testing_gemm", "gbcc_testing_gemm_ex", "gbcc_testing_gemm_ex2", "gbcc_testing_gemm_ex3", "gbcc_testing_gemm_small", "gbcc_testing_r2_assemble", "gbcc_testing_split", "gbcc_testing_scale", "gbcc_testing_fp64_peak", "gbcc_testing_dmma_peak", "gbcc_testing_diis_coefficients", "gbcc_testing_fail_alloc", "gbcc_testing_fixed_split", "gbcc_testing_gemm_fp64tc", "gbcc_testing_gemm_timeout", "gbcc_testing_triples_chunk", "gbcc_testing_profile_residual",
                    "gbcc_testing_last_launches", "gbcc_testing_record", "gbcc_testing_elapsed",
                    "gbcc_testing_profile_gemm_ms", "gbcc_testing_profile_dims",
                    "gbcc_testing_profile_tiles", "gbcc_testing_tc_launches_total", "gbcc_testing_eigh",
@@ -147,6 +147,9 @@ def load(path: str | os.PathLike | None = None) -> C.CDLL:
     lib.gbcc_testing_gemm_small.restype = C.c_int
     lib.gbcc_testing_gemm_small.argtypes = [C.c_int64, C.c_int64, C.c_int64, vp, vp, vp, C.c_int, C.c_int,
                                             C.POINTER(C.c_float)]
+    lib.gbcc_testing_r2_assemble.restype = C.c_int
+    lib.gbcc_testing_r2_assemble.argtypes = [C.c_int64, C.c_int64, vp, vp, vp, vp, vp, C.c_int, vp, C.c_int,
+                                             C.POINTER(C.c_float)]
     lib.gbcc_testing_split.restype = C.c_int
     lib.gbcc_testing_split.argtypes = [vp, C.c_int64, C.c_int, vp]
     lib.gbcc_testing_scale.restype = C.c_int

@@ -320,12 +320,123 @@ __global__ void __launch_bounds__(kThreads) pair_unpack_kernel(int64_t rows_v, i
 //   Q(a,b,i,j) = q(a,b,i,j) + q(b,a,j,i),  q = r2u - 0.5 tmp - tmp(b,a,i,j),
 // i.e. the symmetrisation r2u(a,b,i,j) + r2u(b,a,j,i) after r2u -= 0.5
 // tmp(a,b,i,j) + tmp(b,a,i,j), with P the unpack of pair_unpack_kernel (Bp
-// null: none).  Q(b,a,j,i) = Q(a,b,i,j) operand for operand, so one block
-// per pair a <= b and 32 x 32 tile (I, J) of (i, j) stages q of the tile
-// [a][b][I][J] and of [b][a][J][I] in shared memory (coalesced along j and
-// along i) and adds the same Q to r2[a][b][I][J] and to r2[b][a][J][I]: every
-// r2u, tmp and g element is read once, r2 read and written once.  On the
-// diagonal a = b only tiles I <= J are taken, and a tile I = J once.
+// null: none).
+//
+// Every r2u, tmp and g element is read once, r2 read (if accumulated to) and
+// written once; beside that memory traffic (0.5 ms at o = 50, v = 190) the FP64
+// pipe, 2 results a clock per SM, bounds it: so Q + P, the same for (a,b,i,j) and
+// (b,a,j,i), is formed once (9 operations for two outputs), and pairs are decoded
+// in FP32.  One block per pair a <= b holds q(a,b,.,.), q(b,a,.,.) and the pair's
+// rows of Bp and Bm in shared memory, loaded as they lie (o^2 consecutive
+// elements), and writes r2(a,b,.,.) and r2(b,a,.,.) as they lie; the transposed
+// reads are of shared memory, at an odd row length.  Against the tiled kernel
+// below: o = 50, v = 190 1.85 -> 0.91 ms, o = 30, v = 120 0.22 -> 0.15.
+constexpr int kAssembleSmem = 113 * 1024;
+
+struct AssembleArgs {
+  int o, v;
+  const double* r2u;
+  const double* tmp;
+  const double* g;
+  const double* Bp;
+  const double* Bm;
+  double* r2;
+};
+
+template <bool ACC>
+__global__ void __launch_bounds__(512) r2_assemble_pair_kernel(AssembleArgs A) {
+  extern __shared__ double asm_smem[];
+  const int o = A.o, v = A.v, o2 = o * o, ld = o | 1, sp = o * (o + 1) / 2, sm = o * (o - 1) / 2;
+  double* qa = asm_smem;        // [i][j] of q(a,b,.,.)
+  double* qb = qa + o * ld;     // [i][j] of q(b,a,.,.)
+  double* sbp = qb + o * ld;
+  double* sbm = sbp + sp;
+  const int T = blockDim.x, tid = threadIdx.x;
+  const int di = T / o, dj = T - di * o, i0 = tid / o, j0 = tid - i0 * o;  // e += T
+  for (int64_t p = blockIdx.x; p < static_cast<int64_t>(v) * (v + 1) / 2; p += gridDim.x) {
+    // pair (a, b) = p - b (b + 1) / 2, a <= b
+    int b = static_cast<int>((sqrtf(8.0f * static_cast<float>(p) + 1.0f) - 1.0f) * 0.5f);
+    while (static_cast<int64_t>(b) * (b + 1) / 2 > p) --b;
+    while (static_cast<int64_t>(b + 1) * (b + 2) / 2 <= p) ++b;
+    const int a = static_cast<int>(p - static_cast<int64_t>(b) * (b + 1) / 2);
+    const int64_t ab = (static_cast<int64_t>(a) * v + b) * o2, ba = (static_cast<int64_t>(b) * v + a) * o2;
+    const double* bp = A.Bp ? A.Bp + pair_sym(a, b, v) * sp : nullptr;
+    const double* bm = (A.Bp && A.Bm && a < b) ? A.Bm + pair_anti(a, b, v) * sm : nullptr;
+    {
+      const double* __restrict__ ua = A.r2u + ab;
+      const double* __restrict__ ub = A.r2u + ba;
+      const double* __restrict__ ta = A.tmp + ab;
+      const double* __restrict__ tb = A.tmp + ba;
+      int i = i0, j = j0;
+#pragma unroll 2
+      for (int e = tid; e < o2; e += T) {
+        const double x = ta[e], y = tb[e];
+        qa[i * ld + j] = fma(-0.5, x, ua[e]) - y;
+        qb[i * ld + j] = fma(-0.5, y, ub[e]) - x;
+        i += di;
+        j += dj;
+        if (j >= o) {
+          j -= o;
+          ++i;
+        }
+      }
+      if (bp)
+        for (int e = tid; e < sp; e += T) sbp[e] = bp[e];
+      if (bm)
+        for (int e = tid; e < sm; e += T) sbm[e] = bm[e];
+    }
+    __syncthreads();
+    {
+      int i = i0, j = j0;
+      for (int e = tid; e < o2; e += T) {
+        double x = qa[i * ld + j] + qb[j * ld + i];
+        if (bp) {
+          // P(a,b,i,j) = P(b,a,j,i): the B- term changes sign with i > j (a < b)
+          const int li = min(i, j), hj = max(i, j);
+          const int s = li * o - li * (li - 1) / 2 + (hj - li);
+          double y = sbp[s];
+          if (bm && i != j) y += flip_sign(sbm[s - li - 1], i > j);  // pair_anti
+          x += y;
+        }
+        qa[i * ld + j] = x;  // read by no other thread before the barrier
+        i += di;
+        j += dj;
+        if (j >= o) {
+          j -= o;
+          ++i;
+        }
+      }
+    }
+    __syncthreads();
+    {
+      const double* __restrict__ ga = A.g + ab;
+      const double* __restrict__ gb = A.g + ba;
+      double* __restrict__ ra = A.r2 + ab;
+      double* __restrict__ rb = A.r2 + ba;
+      int i = i0, j = j0;
+#pragma unroll 2
+      for (int e = tid; e < o2; e += T) {
+        const double va = qa[i * ld + j] + ga[e], vb = qa[j * ld + i] + gb[e];
+        ra[e] = ACC ? ra[e] + va : va;
+        if (a != b) rb[e] = ACC ? rb[e] + vb : vb;
+        i += di;
+        j += dj;
+        if (j >= o) {
+          j -= o;
+          ++i;
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// The same for o whose pair does not fit the shared memory above.  Q(b,a,j,i) =
+// Q(a,b,i,j) operand for operand, so one block per pair a <= b and 32 x 32 tile
+// (I, J) of (i, j) stages q of the tile [a][b][I][J] and of [b][a][J][I] in shared
+// memory (coalesced along j and along i) and adds the same Q to r2[a][b][I][J] and
+// to r2[b][a][J][I].  On the diagonal a = b only tiles I <= J are taken, and a
+// tile I = J once.
 __global__ void __launch_bounds__(256) r2_assemble_kernel(int64_t o, int64_t v, const double* __restrict__ r2u,
                                                           const double* __restrict__ tmp,
                                                           const double* __restrict__ g,
@@ -1013,6 +1124,24 @@ void launch_pair_unpack(int64_t rows_v, int64_t v, int64_t o, bool ab_pairs, con
 
 void launch_r2_assemble(int64_t o, int64_t v, const double* r2u, const double* tmp, const double* g,
                         const double* Bp, const double* Bm, bool accumulate, double* r2, cudaStream_t st) {
+  // a pair's q, Bp and Bm in half the shared memory of an SM or less (o <= 68): two
+  // blocks an SM.  One side of the line and the other, v = 100: o = 68 0.58 ms,
+  // o = 69 (tiled) 0.57; o = 64 0.47, o = 80 (tiled) 1.11
+  const int64_t bytes = (2 * o * (o | 1) + (Bp ? o * o : 0)) * 8;
+  static const bool attr =
+      cudaFuncSetAttribute(r2_assemble_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAssembleSmem) ==
+          cudaSuccess &&
+      cudaFuncSetAttribute(r2_assemble_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAssembleSmem) ==
+          cudaSuccess;
+  if (attr && bytes <= kAssembleSmem) {
+    const AssembleArgs A{static_cast<int>(o), static_cast<int>(v), r2u, tmp, g, Bp, Bm, r2};
+    const int64_t want = (o * o / 4 + 31) / 32 * 32;  // about four elements a thread
+    const unsigned threads = static_cast<unsigned>(std::min<int64_t>(512, std::max<int64_t>(64, want)));
+    const unsigned grid = static_cast<unsigned>(std::min<int64_t>(v * (v + 1) / 2, 152LL * 32));
+    if (accumulate) r2_assemble_pair_kernel<true><<<grid, threads, bytes, st>>>(A);
+    else r2_assemble_pair_kernel<false><<<grid, threads, bytes, st>>>(A);
+    return;
+  }
   const int64_t nt = (o + 31) / 32;
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>(v * v * nt * nt, 152LL * 16));
   r2_assemble_kernel<<<grid, dim3(32, 8), 0, st>>>(o, v, r2u, tmp, g, Bp, Bm, accumulate, r2);

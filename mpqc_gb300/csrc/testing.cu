@@ -286,6 +286,50 @@ extern "C" int gbcc_testing_split(const double* x, int64_t n, int nslices, uint1
   }
 }
 
+extern "C" int gbcc_testing_r2_assemble(int64_t o, int64_t v, const double* r2u, const double* tmp, const double* g,
+                                        const double* Bp, const double* Bm, int accumulate, double* r2, int repeat,
+                                        float* ms) {
+  using namespace gbcc;
+  if (o < 1 || v < 1 || o > 1000 || v > 1000 || !r2u || !tmp || !g || !r2 || repeat < 1) return GBCC_ERR_INVALID_ARG;
+  std::vector<void*> owned;
+  int status = GBCC_OK;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  try {
+    auto upload = [&](const double* src, int64_t n) -> double* {
+      if (!src || n == 0) return nullptr;
+      owned.push_back(dev_alloc(n * sizeof(double)));
+      GBCC_CK(cudaMemcpy(owned.back(), src, n * sizeof(double), cudaMemcpyHostToDevice));
+      return static_cast<double*>(owned.back());
+    };
+    const int64_t n = v * v * o * o;
+    const double *du = upload(r2u, n), *dt = upload(tmp, n), *dg = upload(g, n);
+    const double *dp = upload(Bp, v * (v + 1) / 2 * (o * (o + 1) / 2)), *dm = upload(Bm, v * (v - 1) / 2 * (o * (o - 1) / 2));
+    double* dr = upload(r2, n);
+    GBCC_CK(cudaEventCreate(&e0));
+    GBCC_CK(cudaEventCreate(&e1));
+    float total = 0.f;
+    for (int r = 0; r < repeat; ++r) {
+      GBCC_CK(cudaMemcpy(dr, r2, n * sizeof(double), cudaMemcpyHostToDevice));
+      GBCC_CK(cudaEventRecord(e0, nullptr));
+      launch_r2_assemble(o, v, du, dt, dg, dp, dm, accumulate != 0, dr, nullptr);
+      GBCC_CK(cudaEventRecord(e1, nullptr));
+      GBCC_CK(cudaEventSynchronize(e1));
+      float one = 0.f;
+      GBCC_CK(cudaEventElapsedTime(&one, e0, e1));
+      total += one;
+    }
+    GBCC_CK(cudaGetLastError());
+    GBCC_CK(cudaMemcpy(r2, dr, n * sizeof(double), cudaMemcpyDeviceToHost));
+    if (ms) *ms = total / static_cast<float>(repeat);
+  } catch (const Error& e) {
+    status = e.status;
+  }
+  if (e0) cudaEventDestroy(e0);
+  if (e1) cudaEventDestroy(e1);
+  for (void* p : owned) dev_free(p);
+  return status;
+}
+
 extern "C" int gbcc_testing_scale(const double* x, int64_t n, double coef, double* out) {
   using namespace gbcc;
   if (!x || !out || n < 0) return GBCC_ERR_INVALID_ARG;
