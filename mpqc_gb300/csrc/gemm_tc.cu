@@ -17,7 +17,17 @@
 // every `fold` chunks, fold p into a float-float (hi + lo) accumulator kept in
 // TMEM with Knuth's TwoSum; the error is that of one chunk plus `fold` FP32
 // additions, independent of K.  TMEM holds two accumulators, so the MMAs of
-// the next chunk run while the epilogue drains the previous one.
+// the next chunk run while the epilogue drains the previous one.  A tile of at
+// most `fold` chunks never leaves FP32 (p is its value).
+//
+// The products that only have a few chunks are long and thin (10^6 rows, N and K
+// of an orbital count) and move little more than C, so their time was the
+// epilogue's: the float-float words went through TMEM, C was read after the last
+// MMA and each output took two to five FP64-pipe operations of the 2 a clock an SM
+// has.  Now C is read before the first wait (BN <= 64) and an output costs one
+// FP64 operation or none; BN = 64 has 16 epilogue warps.  1805000 x 50 x 190: 1.22
+// -> 1.00 ms, 108000 x 120 x 120 0.174 -> 0.119, 18145 x 1275 x 1275 0.33 -> 0.26,
+// 17161 x 17161 x 420 1.64 -> 1.41.
 //
 // With BN = 256 the two accumulators fill TMEM, so the chunks of a tile sum in
 // FP32 registers only (error that of one chunk plus one FP32 addition per
@@ -33,7 +43,8 @@
 //   warps 4..11: epilogue; warp w reads TMEM lanes 32*(w%4).. and the column
 //                half (w-4)/4 of the tile (warps 2 and 3 only pad the
 //                block to three warps per scheduler, which leaves 168
-//                registers per thread for the float-float accumulators)
+//                registers per thread for the float-float accumulators); with
+//                BN = 64 warps 2..17, a column quarter each
 // Operand tiles are K-major with the 128-byte swizzle (TMA box 64 x rows).
 // Every mbarrier wait is bounded: on timeout the kernel records kDevTimeout in
 // *err, drains its own copies in flight, waits for its MMAs, frees its TMEM
@@ -66,9 +77,11 @@ struct TcCfg {
   static constexpr uint32_t kBStage = SPS * kBBytes;
   static constexpr uint32_t kStageBytes = kAStage + kBStage;
   // warps 0 (TMA), 1 (MMA), 2-3 idle, 4-11 epilogue: three warps per
-  // scheduler leave 168 registers a thread
-  static constexpr int kEpiWarps = 8;
-  static constexpr int kEpiWarp0 = 4;
+  // scheduler leave 168 registers a thread.  BN = 64, whose products are mostly
+  // long and thin (a tile's MMAs are short, C is most of the traffic): 16
+  // epilogue warps of 16 columns, from warp 2 on
+  static constexpr int kEpiWarps = BN == 64 ? 16 : 8;
+  static constexpr int kEpiWarp0 = BN == 64 ? 2 : 4;
   static constexpr int kThreads = 32 * (kEpiWarp0 + kEpiWarps);
   // staging tile per epilogue warp: (hi, lo) float pairs with the float-float
   // fold (BN <= 128), single floats at BN = 192 (room for a fifth stage, or two
@@ -108,6 +121,7 @@ __global__ void __launch_bounds__(TcCfg<BN, CTA2, SPS>::kThreads, 1)
   const int nunits = CTA2 ? static_cast<int>(gridDim.x / 2) : static_cast<int>(gridDim.x);
   constexpr int S = Cfg::kStages;
   constexpr int COLS = Cfg::kCols;
+  constexpr bool kEarlyC = COLS <= 32;  // registers for a thread's share of C
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -342,6 +356,35 @@ __global__ void __launch_bounds__(TcCfg<BN, CTA2, SPS>::kThreads, 1)
 #pragma unroll
       for (int j = 0; j < COLS; ++j) p[j] = 0.f;
       bool first_fold = true;
+      // a tile of at most `fold` chunks is its FP32 sum p: no float-float words, and
+      // where C is read its elements are in flight while the MMAs run
+      const bool folded = Cfg::kFold && nchunks > fold;
+      const int err_before = *reinterpret_cast<const volatile int*>(g.err);
+      double cv[kEarlyC ? COLS : 16];
+      if constexpr (kEarlyC) {
+        if (!folded && ksplit == 1 && g.beta != 0.0) {
+          if (g.m_major) {
+            const int64_t m = m0 + row;
+            const double* crow = g.C + (m < g.M ? g.cm[m] : 0);
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) {
+              const int64_t n = n0 + col0 + j;
+              cv[j] = m < g.M && n < g.N ? crow[g.cn[n]] : 0.0;
+            }
+          } else {
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+              const int64_t m = m0 + q * 32 + (lane >> 4) + 2 * r;
+              const double* crow = g.C + (m < g.M ? g.cm[m] : 0);
+#pragma unroll
+              for (int j0 = 0; j0 < COLS; j0 += 16) {
+                const int64_t n = n0 + col0 + j0 + (lane & 15);
+                cv[j0 + r] = m < g.M && n < g.N ? crow[g.cn[n]] : 0.0;
+              }
+            }
+          }
+        }
+      }
       for (int cc = 0; cc < nchunks; ++cc, ++c) {
         const uint32_t b = c & 1;
         if (!mbar_wait(&acc_full[b], (c >> 1) & 1, g.err, wait_ns)) {
@@ -366,7 +409,7 @@ __global__ void __launch_bounds__(TcCfg<BN, CTA2, SPS>::kThreads, 1)
           if constexpr (CTA2) mbar_arrive_cluster(b ? acc_empty_leader1 : acc_empty_leader0);
           else mbar_arrive(&acc_empty[b]);
         }
-        if (Cfg::kFold && ((cc + 1) % fold == 0 || cc == nchunks - 1)) {
+        if (folded && ((cc + 1) % fold == 0 || cc == nchunks - 1)) {
           // fold p into the float-float (hi, lo) pair kept in TMEM
 #pragma unroll
           for (int j0 = 0; j0 < COLS; j0 += 16) {
@@ -393,180 +436,175 @@ __global__ void __launch_bounds__(TcCfg<BN, CTA2, SPS>::kThreads, 1)
         }
       }
       if (!ok) break;
-      if (*reinterpret_cast<const volatile int*>(g.err) != kDevOk) continue;
-      if (ksplit == 1 && g.m_major) {
-        // C contiguous in M: every lane owns one row, so the lanes of a warp
-        // write 32 consecutive rows of one column
-        const int64_t m = m0 + row;
-#pragma unroll
-        for (int j0 = 0; j0 < COLS; j0 += 16) {
-          uint32_t h[16], l[16];
-          if constexpr (Cfg::kFold) {
-            tmem_ld16(hi_base + j0, h);
-            tmem_ld16(lo_base + j0, l);
-            tmem_ld_wait();
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              h[j] = __float_as_uint(p[j0 + j]);
-              l[j] = 0u;
-            }
-          }
+      if (err_before != kDevOk) continue;
+      // C from p: alpha x, alpha x + C or alpha x + beta C, at most one FP64 operation
+      // a value where beta is 0 or 1 (none where alpha is 1 or -1 too)
+      auto put = [&](double* c, float pv, double old) {
+        const double x = f2d_exact(pv);
+        *c = g.beta == 1.0 ? fma(g.alpha, x, old) : fma(g.alpha, x, g.beta * old);
+      };
+      const bool pm1 = g.alpha == 1.0 || g.alpha == -1.0;
+      auto put0 = [&](double* c, float pv) {
+        const double x = f2d_exact(pv);
+        if (pm1) *c = flip_sign(x, g.alpha < 0.0);
+        else *c = g.alpha * x;
+      };
+      if (!folded) {
+        if (ksplit == 1 && g.m_major) {
+          const int64_t m = m0 + row;
           if (m < g.M) {
-            const int64_t om = g.cm[m];
-            double cv[16];
-            if (g.beta != 0.0) {
+            double* crow = g.C + g.cm[m];
+            if (g.beta == 0.0) {
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const int64_t n = n0 + col0 + j0 + j;
-                cv[j] = n < g.N ? g.C[om + g.cn[n]] : 0.0;
-              }
-            }
-            if constexpr (Cfg::kFold) {
-              // beta c + alpha (hi + lo): separate loops per beta, so no multiply by
-              // beta is evaluated (as a select) where beta is 0 or 1
-              if (g.beta == 0.0) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                  const int64_t n = n0 + col0 + j0 + j;
-                  if (n < g.N)
-                    g.C[om + g.cn[n]] = g.alpha * (f2d_exact(__uint_as_float(h[j])) + f2d_exact(__uint_as_float(l[j])));
-                }
-              } else if (g.beta == 1.0) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                  const int64_t n = n0 + col0 + j0 + j;
-                  if (n < g.N)
-                    g.C[om + g.cn[n]] = fma(g.alpha, f2d_exact(__uint_as_float(h[j])),
-                                            fma(g.alpha, f2d_exact(__uint_as_float(l[j])), cv[j]));
-                }
-              } else {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                  const int64_t n = n0 + col0 + j0 + j;
-                  if (n < g.N)
-                    g.C[om + g.cn[n]] = fma(g.alpha, f2d_exact(__uint_as_float(h[j])),
-                                            fma(g.alpha, f2d_exact(__uint_as_float(l[j])), g.beta * cv[j]));
-                }
+              for (int j = 0; j < COLS; ++j) {
+                const int64_t n = n0 + col0 + j;
+                if (n < g.N) put0(crow + g.cn[n], p[j]);
               }
             } else {
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const int64_t n = n0 + col0 + j0 + j;
-                if (n < g.N) {
-                  const double val = g.alpha * (static_cast<double>(__uint_as_float(h[j])) +
-                                                static_cast<double>(__uint_as_float(l[j])));
-                  g.C[om + g.cn[n]] = (g.beta == 0.0) ? val : fma(g.beta, cv[j], val);
+              for (int j0 = 0; j0 < COLS; j0 += 16) {
+                if constexpr (!kEarlyC) {
+#pragma unroll
+                  for (int j = 0; j < 16; ++j) {
+                    const int64_t n = n0 + col0 + j0 + j;
+                    cv[j] = n < g.N ? crow[g.cn[n]] : 0.0;
+                  }
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                  const int64_t n = n0 + col0 + j0 + j;
+                  if (n < g.N) put(crow + g.cn[n], p[j0 + j], cv[kEarlyC ? j0 + j : j]);
                 }
               }
             }
           }
+          continue;
+        }
+        // 32 rows x 16 columns at a time through shared memory, the lanes along N
+        float* stgf = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(stg_all) +
+                                               (warp - kEpiWarp0) * 32 * kStgLd * Cfg::kStgElem);
+        const int cj = lane & 15, rl = lane >> 4;
+#pragma unroll
+        for (int j0 = 0; j0 < COLS; j0 += 16) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) stgf[lane * kStgLd + j] = p[j0 + j];
+          __syncwarp();
+          const int64_t n = n0 + col0 + j0 + cj;
+          if (ksplit > 1) {
+            double* P = g.partial + static_cast<int64_t>(split) * g.Mpad * g.Npad + n;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+              const int rr = rl + 2 * r;
+              P[(m0 + q * 32 + rr) * g.Npad] = f2d_exact(stgf[rr * kStgLd + cj]);
+            }
+          } else if (n < g.N) {
+            double* cn = g.C + g.cn[n];
+#pragma unroll
+            for (int r0 = 0; r0 < 16; r0 += 8) {
+              int64_t off[8];
+#pragma unroll
+              for (int r = 0; r < 8; ++r) {
+                const int64_t m = m0 + q * 32 + rl + 2 * (r0 + r);
+                off[r] = m < g.M ? g.cm[m] : -1;
+              }
+              if (g.beta == 0.0) {
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+                  if (off[r] >= 0) put0(cn + off[r], stgf[(rl + 2 * (r0 + r)) * kStgLd + cj]);
+              } else {
+                if constexpr (!kEarlyC) {
+#pragma unroll
+                  for (int r = 0; r < 8; ++r) cv[r] = off[r] >= 0 ? cn[off[r]] : 0.0;
+                }
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+                  if (off[r] >= 0)
+                    put(cn + off[r], stgf[(rl + 2 * (r0 + r)) * kStgLd + cj], cv[kEarlyC ? j0 + r0 + r : r]);
+              }
+            }
+          }
+          __syncwarp();
         }
         continue;
       }
-      // stage 32 rows x 16 columns through shared memory, then write with the
-      // lanes along N (coalesced when C is contiguous in N)
-      uint8_t* stg_w = reinterpret_cast<uint8_t*>(stg_all) + (warp - kEpiWarp0) * 32 * kStgLd * Cfg::kStgElem;
-      double* stg = reinterpret_cast<double*>(stg_w);  // float-float variants: read as float2
-      float* stgf = reinterpret_cast<float*>(stg_w);   // FP32 variants
-      const int cj = lane & 15;
+      if constexpr (Cfg::kFold) {
+        // (hi, lo) from tensor memory
+        auto pair_value = [&](float hi, float lo, double old) {
+          if (g.beta == 0.0) return g.alpha * (f2d_exact(hi) + f2d_exact(lo));
+          return fma(g.alpha, f2d_exact(hi), fma(g.alpha, f2d_exact(lo), g.beta == 1.0 ? old : g.beta * old));
+        };
+        if (ksplit == 1 && g.m_major) {
+          // C contiguous in M: every lane owns one row, so the lanes of a warp
+          // write 32 consecutive rows of one column
+          const int64_t m = m0 + row;
 #pragma unroll
-      for (int j0 = 0; j0 < COLS; j0 += 16) {
-        uint32_t h[16], l[16];
-        if constexpr (Cfg::kFold) {
+          for (int j0 = 0; j0 < COLS; j0 += 16) {
+            uint32_t h[16], l[16];
+            tmem_ld16(hi_base + j0, h);
+            tmem_ld16(lo_base + j0, l);
+            tmem_ld_wait();
+            if (m < g.M) {
+              double* crow = g.C + g.cm[m];
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const int64_t n = n0 + col0 + j0 + j;
+                cv[j] = g.beta != 0.0 && n < g.N ? crow[g.cn[n]] : 0.0;
+              }
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const int64_t n = n0 + col0 + j0 + j;
+                if (n < g.N) crow[g.cn[n]] = pair_value(__uint_as_float(h[j]), __uint_as_float(l[j]), cv[j]);
+              }
+            }
+          }
+          continue;
+        }
+        // stage 32 rows x 16 columns through shared memory, then write with the
+        // lanes along N (coalesced when C is contiguous in N)
+        float2* stg2 = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(stg_all) +
+                                                 (warp - kEpiWarp0) * 32 * kStgLd * Cfg::kStgElem);
+        const int cj = lane & 15;
+#pragma unroll
+        for (int j0 = 0; j0 < COLS; j0 += 16) {
+          uint32_t h[16], l[16];
           tmem_ld16(hi_base + j0, h);
           tmem_ld16(lo_base + j0, l);
           tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            h[j] = __float_as_uint(p[j0 + j]);
-            l[j] = 0u;
-          }
-        }
-        if constexpr (Cfg::kFold) {
-          // (hi, lo) pairs, converted to FP64 at the store
-          float2* stg2 = reinterpret_cast<float2*>(stg);
 #pragma unroll
           for (int j = 0; j < 16; ++j)
             stg2[lane * kStgLd + j] = make_float2(__uint_as_float(h[j]), __uint_as_float(l[j]));
-        } else if constexpr (Cfg::kStgElem == 4) {
+          __syncwarp();
+          const int64_t n = n0 + col0 + j0 + cj;
+          if (ksplit > 1) {
+            // K-split partial tile: plain stores, reduced by splitk_reduce
+            double* P = g.partial + static_cast<int64_t>(split) * g.Mpad * g.Npad + n;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) stgf[lane * kStgLd + j] = __uint_as_float(h[j]);
-        } else {
+            for (int rr = lane >> 4; rr < 32; rr += 2) {
+              const float2 hl = stg2[rr * kStgLd + cj];
+              P[(m0 + q * 32 + rr) * g.Npad] = f2d_exact(hl.x) + f2d_exact(hl.y);
+            }
+          } else if (n < g.N) {
+            const int64_t on = g.cn[n];
+            // 8 rows of a lane: issue every read of C before the stores
 #pragma unroll
-          for (int j = 0; j < 16; ++j)
-            stg[lane * kStgLd + j] =
-                static_cast<double>(__uint_as_float(h[j])) + static_cast<double>(__uint_as_float(l[j]));
+            for (int r0 = 0; r0 < 16; r0 += 8) {
+              int64_t off[8];
+#pragma unroll
+              for (int r = 0; r < 8; ++r) {
+                const int64_t m = m0 + q * 32 + (lane >> 4) + 2 * (r0 + r);
+                off[r] = m < g.M ? g.cm[m] + on : -1;
+                cv[r] = g.beta != 0.0 && off[r] >= 0 ? g.C[off[r]] : 0.0;
+              }
+#pragma unroll
+              for (int r = 0; r < 8; ++r) {
+                if (off[r] < 0) continue;
+                const float2 hl = stg2[((lane >> 4) + 2 * (r0 + r)) * kStgLd + cj];
+                g.C[off[r]] = pair_value(hl.x, hl.y, cv[r]);
+              }
+            }
+          }
+          __syncwarp();
         }
-        __syncwarp();
-        const int64_t n = n0 + col0 + j0 + cj;
-        if (ksplit > 1) {
-          // K-split partial tile: plain stores, reduced by splitk_reduce
-          double* P = g.partial + static_cast<int64_t>(split) * g.Mpad * g.Npad + n;
-#pragma unroll
-          for (int rr = lane >> 4; rr < 32; rr += 2) {
-            const int64_t m = m0 + q * 32 + rr;
-            if constexpr (Cfg::kFold) {
-              const float2 hl = reinterpret_cast<const float2*>(stg)[rr * kStgLd + cj];
-              P[m * g.Npad] = f2d_exact(hl.x) + f2d_exact(hl.y);
-            } else if constexpr (Cfg::kStgElem == 4) {
-              P[m * g.Npad] = static_cast<double>(stgf[rr * kStgLd + cj]);
-            } else {
-              P[m * g.Npad] = stg[rr * kStgLd + cj];
-            }
-          }
-        } else if (cj < COLS && n < g.N) {
-          const int64_t on = g.cn[n];
-          // 16 rows per lane: issue every read of C before the stores
-          double cv[16];
-          int64_t off[16];
-#pragma unroll
-          for (int r = 0; r < 16; ++r) {
-            const int64_t m = m0 + q * 32 + (lane >> 4) + 2 * r;
-            off[r] = m < g.M ? g.cm[m] + on : -1;
-          }
-          if (g.beta != 0.0) {
-#pragma unroll
-            for (int r = 0; r < 16; ++r) cv[r] = off[r] >= 0 ? g.C[off[r]] : 0.0;
-          }
-          if constexpr (Cfg::kFold) {
-            const float2* stg2 = reinterpret_cast<const float2*>(stg);
-            if (g.beta == 0.0) {
-#pragma unroll
-              for (int r = 0; r < 16; ++r) {
-                if (off[r] < 0) continue;
-                const float2 hl = stg2[((lane >> 4) + 2 * r) * kStgLd + cj];
-                g.C[off[r]] = g.alpha * (f2d_exact(hl.x) + f2d_exact(hl.y));
-              }
-            } else if (g.beta == 1.0) {
-#pragma unroll
-              for (int r = 0; r < 16; ++r) {
-                if (off[r] < 0) continue;
-                const float2 hl = stg2[((lane >> 4) + 2 * r) * kStgLd + cj];
-                g.C[off[r]] = fma(g.alpha, f2d_exact(hl.x), fma(g.alpha, f2d_exact(hl.y), cv[r]));
-              }
-            } else {
-#pragma unroll
-              for (int r = 0; r < 16; ++r) {
-                if (off[r] < 0) continue;
-                const float2 hl = stg2[((lane >> 4) + 2 * r) * kStgLd + cj];
-                g.C[off[r]] = fma(g.alpha, f2d_exact(hl.x), fma(g.alpha, f2d_exact(hl.y), g.beta * cv[r]));
-              }
-            }
-          } else {
-#pragma unroll
-            for (int r = 0; r < 16; ++r) {
-              if (off[r] < 0) continue;
-              double sv;
-              if constexpr (Cfg::kStgElem == 4) sv = static_cast<double>(stgf[((lane >> 4) + 2 * r) * kStgLd + cj]);
-              else sv = stg[((lane >> 4) + 2 * r) * kStgLd + cj];
-              const double val = g.alpha * sv;
-              g.C[off[r]] = (g.beta == 0.0) ? val : fma(g.beta, cv[r], val);
-            }
-          }
-        }
-        __syncwarp();
       }
     }
   }
