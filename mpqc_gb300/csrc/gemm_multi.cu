@@ -30,8 +30,8 @@
 // three sums of two permutation terms that share their output order (triples.cu);
 // its two segments name different operand panels and rows.
 //
-// Persistent, 10 warps: 0 TMA, 1 MMA (and TMEM allocation), 2-9 epilogue (warp w
-// reads TMEM lanes 32 (w % 4)..), with the bounded waits and teardown of
+// Persistent: warp 0 TMA, 1 MMA (and TMEM allocation), 8 or 16 (three
+// slices, wide tiles) epilogue warps from 2 on (warp w reads TMEM lanes 32 (w % 4)..), with the bounded waits and teardown of
 // gemm_tc.cu.
 #include <algorithm>
 
@@ -44,9 +44,7 @@ namespace {
 
 constexpr int BM = 128;
 constexpr int HB = 32;          // K elements per stage: 64 bytes, one 64-byte swizzle row
-constexpr int kEpiWarps = 8;
 constexpr int kEpiWarp0 = 2;     // no idle warps: 200 registers a thread (four sums per output, six slices)
-constexpr int kThreads = 32 * (kEpiWarp0 + kEpiWarps);
 
 // Shared-memory matrix descriptor: K-major, 64-byte swizzle, 8-row groups 512
 // bytes apart.
@@ -58,6 +56,12 @@ __device__ __forceinline__ uint64_t sdesc_sw64(uint32_t saddr) {
   d |= static_cast<uint64_t>(1) << 46;          // descriptor version
   d |= static_cast<uint64_t>(4) << 61;          // 64-byte swizzle
   return d;
+}
+
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
 }
 
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
@@ -73,6 +77,12 @@ struct MultiCfg {
   static constexpr uint32_t kBSlice = BN * HB * 2;
   static constexpr uint32_t kAStage = SL * kASlice;
   static constexpr uint32_t kStage = SL * (kASlice + kBSlice);
+  // three slices: a tile's MMAs are short and its epilogue is a chain of TMEM reads
+  // and stores, so four warps a scheduler share it where the tile is wide (v = 120
+  // 242 -> 227 ms, v = 97 16.8 -> 16.2; below, equal or 2 % slower: the staging
+  // takes a pipeline stage)
+  static constexpr int kEpiWarps = SL == 3 && BN > 80 ? 16 : 8;
+  static constexpr int kThreads = 32 * (kEpiWarp0 + kEpiWarps);
   // epilogue staging per warp: 32 rows x kStgCols words of 8 bytes
   static constexpr int kStgCols = SL == 3 ? 8 : 4;
   static constexpr int kStgLd = SL == 3 ? 9 : 4;
@@ -87,7 +97,7 @@ struct MultiCfg {
   static constexpr uint32_t kCols = kBufs * BN <= 64 ? 64 : (kBufs * BN <= 128 ? 128 : (kBufs * BN <= 256 ? 256 : 512));
   static_assert(kBufs * BN <= 512, "tensor memory");
   static_assert(BN % 16 == 0, "MMA width");
-  static constexpr int kOut = BN / 2;                // columns per epilogue thread
+  static constexpr int kOut = BN / (kEpiWarps / 4);  // columns per epilogue thread
 };
 
 // one output tile: where its operand segments and its output lie
@@ -145,7 +155,7 @@ __device__ __forceinline__ Tile decode(const GemmMultiArgs& g, int t, int BN) {
 }
 
 template <int SL, int BN, bool TRIPLES>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(MultiCfg<SL, BN>::kThreads, 1)
     gemm_multi_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
                       const __grid_constant__ CUtensorMap tmB, const __grid_constant__ GemmMultiArgs g) {
   using Cfg = MultiCfg<SL, BN>;
@@ -169,7 +179,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     for (int b = 0; b < NBUF; ++b) {
       mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], kEpiWarps);
+      mbar_init(&acc_empty[b], Cfg::kEpiWarps);
     }
     mbar_init(done, 1);
     fence_barrier_init();
@@ -325,18 +335,25 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           tc_fence_after();
           const uint32_t base = tmem + lane_addr + b * BN + col0;
+          if constexpr (SL == 3) {
+            uint32_t r[OUT];
 #pragma unroll
-          for (int j0 = 0; j0 < OUT; j0 += 16) {
-            uint32_t r0[8], r1[8];
-            tmem_ld8(base + j0, r0);
-            if (j0 + 8 < OUT) tmem_ld8(base + j0 + 8, r1);
+            for (int j0 = 0; j0 < OUT; j0 += 4) tmem_ld4(base + j0, r + j0);
             tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              if (j0 + j >= OUT) continue;
-              const float y = __uint_as_float(j < 8 ? r0[j & 7] : r1[j & 7]);
-              if constexpr (SL == 3) hi[j0 + j] = __fadd_rn(hi[j0 + j], y);
-              else two_sum_acc(hi[j0 + j], lo[j0 + j], y);
+            for (int j = 0; j < OUT; ++j) hi[j] = __fadd_rn(hi[j], __uint_as_float(r[j]));
+          } else {
+#pragma unroll
+            for (int j0 = 0; j0 < OUT; j0 += 16) {
+              uint32_t r0[8], r1[8];
+              tmem_ld8(base + j0, r0);
+              if (j0 + 8 < OUT) tmem_ld8(base + j0 + 8, r1);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                if (j0 + j >= OUT) continue;
+                two_sum_acc(hi[j0 + j], lo[j0 + j], __uint_as_float(j < 8 ? r0[j & 7] : r1[j & 7]));
+              }
             }
           }
           tc_fence_before();
@@ -404,6 +421,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           float2* s2 = reinterpret_cast<float2*>(stg);
 #pragma unroll
           for (int j = 0; j < SC; ++j) {
+            if (j0 + j >= OUT) continue;
             float hi = x0[j0 + j], lo = 0.f;
             two_sum_acc(hi, lo, x1[j0 + j]);
             s2[lane * LD + j] = make_float2(hi, lo);
@@ -416,7 +434,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncwarp();
         const int64_t n = T.n0 + col0 + j0 + cj;
         if constexpr (TRIPLES) {
-          if (n < g.v) {
+          if (n < g.v && (OUT % SC == 0 || j0 + cj < OUT)) {
             double* out = g.W + T.out + n;
 #pragma unroll
             for (int r = 0; r < SC; ++r)
@@ -500,7 +518,7 @@ bool launch(const GemmMultiArgs& g, const CUtensorMap& a, const CUtensorMap& a2,
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 Cfg::kSmem) == cudaSuccess;
   if (!attr) return false;
-  gemm_multi_kernel<SL, BN, TRIPLES><<<std::min(g.tiles, num_sms()), kThreads, Cfg::kSmem, st>>>(a, a2, b, g);
+  gemm_multi_kernel<SL, BN, TRIPLES><<<std::min(g.tiles, num_sms()), Cfg::kThreads, Cfg::kSmem, st>>>(a, a2, b, g);
   return true;
 }
 

@@ -465,32 +465,52 @@ __global__ void __launch_bounds__(kThreads) triples_pack_kernel(PackArgs g) {
 __device__ constexpr int kPerm[6][3] = {{0, 1, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}, {0, 2, 1}, {1, 0, 2}};
 __device__ constexpr int kSwap[6] = {4, 5, 3, 2, 0, 1};
 __device__ constexpr int kCycle[6] = {1, 2, 0, 5, 3, 4};
+// ordered pairs of different things
+__device__ constexpr int kPair[6][2] = {{0, 1}, {0, 2}, {1, 0}, {1, 2}, {2, 0}, {2, 1}};
+__device__ constexpr int pair_id(int s, int f) { return 2 * s + f - (f > s ? 1 : 0); }
 
-constexpr int kB = 8;                 // virtual block
-constexpr int kRowLd = 9, kSlabLd = 73;  // padded strides: reads along any index hit different banks
-constexpr int kCube = kB * kSlabLd;
+constexpr int kB = 8;              // virtual block
+constexpr int kCube = kB * kB * kB;
+constexpr int kEnergyThreads = kCube;
+constexpr int kEnergyGrid = 152;   // one block an SM
 
 template <typename R>
-struct EnergySmem {
-  double W[3][6][kCube];              // float2 (three slices) or double words
-  R G[3][9][kB * kRowLd];             // <ij|, <jk|, <ik| over ordered block pairs
-  R t1[3][3][kB];                     // t1 of i, j, k over the blocks
+struct EnergyStage {
+  double W[3][6][kCube];           // float2 (three slices) or double words
+  R G[3][6][kB * kB];              // <ij|, <jk|, <ik| over ordered block pairs
+  R t1[3][3][kB];                  // t1 of i, j, k over the blocks
   R ev[3][kB];
-  double red[kThreads];
+  R eo;                            // eps_i + eps_j + eps_k
 };
 
 struct EnergyArgs {
   int o, v;
-  const int4* triples;                // this batch's
-  const unsigned* blocks;             // block triples A <= B <= C, 10 bits each
+  int n;                      // triplets of this batch
+  const int4* triples;        // theirs
+  const unsigned* blocks;     // block triples A <= B <= C, 10 bits each
   int nblocks;
-  const double* W;                    // [triple][3][v][v][v]
-  const double* Gijab;
-  const double* t1;
-  const double* eps_o;
-  const double* eps_v;
-  double* partial;                    // [triple][gridDim.x]
+  const double* W;            // [triplet][3][v][v][v]
+  const void* Gijab;          // of type R, as the rest
+  const void* t1;
+  const void* eps_v;
+  const void* eo;             // per triplet of this batch
+  double* partial;            // [gridDim.x]
 };
+
+// x to y as the energy's type
+template <typename R>
+__global__ void __launch_bounds__(kThreads) convert_kernel(const double* __restrict__ x, int64_t n, R* __restrict__ y) {
+  for (int64_t e = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x; e < n;
+       e += static_cast<int64_t>(gridDim.x) * kThreads)
+    y[e] = static_cast<R>(x[e]);
+}
+
+template <typename R>
+__global__ void __launch_bounds__(kThreads) triplet_energies_kernel(const int4* __restrict__ tr, int64_t n,
+                                                                    const double* __restrict__ eps_o, R* __restrict__ eo) {
+  const int64_t t = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
+  if (t < n) eo[t] = static_cast<R>(eps_o[tr[t].x] + eps_o[tr[t].y] + eps_o[tr[t].z]);
+}
 
 // hi + lo += x (TwoSum), for sums of many FP32 terms
 __device__ __forceinline__ void add_ff(float& hi, float& lo, float x) {
@@ -499,134 +519,179 @@ __device__ __forceinline__ void add_ff(float& hi, float& lo, float x) {
   hi = s;
 }
 
-__device__ __forceinline__ void copy8_async(double* dst, const double* src, bool in) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst)), n = in ? 8u : 0u;  // 0 source bytes: zeros
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src, bool in) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst)), n = in ? BYTES : 0u;  // 0 source bytes: zeros
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(BYTES), "r"(n) : "memory");
 }
 
-// Block (bx, t): the block triples bx, bx + gridDim.x, ... of triplet t.  R: the
-// arithmetic of the terms (double for FP64_TC; float for MIXED, whose products
-// carry ~1e-6, with W and the sums as float-float pairs).
+// Where element (x, y, z) of a cube lies: a linear bijection of the nine index bits
+// whose low four bits (the 16 banks of 8 bytes) differ over 8 values of any one
+// index times 2 neighbouring values of any other, i.e. over the half warp of a
+// copy (z, y) and of a read along any two of the three indices.
+__device__ __forceinline__ int cube_at(int x, int y, int z) {
+  const int x0 = x & 1, x1 = (x >> 1) & 1, x2 = x >> 2, y0 = y & 1, y1 = (y >> 1) & 1, y2 = y >> 2, z0 = z & 1,
+            z1 = (z >> 1) & 1, z2 = z >> 2;
+  return (z0 ^ y2 ^ x2) | ((y0 ^ z2 ^ x2) << 1) | ((x0 ^ z2 ^ y2) << 2) | ((z1 ^ y1 ^ x1) << 3) | (z2 << 4) |
+         (y1 << 5) | (y2 << 6) | (x1 << 7) | (x2 << 8);
+}
+// and (x, y) of an 8 x 8 tile: a warp's 8 values of one index times 4 of the other
+// lie in different banks
+__device__ __forceinline__ int tile_at(int x, int y) { return x * kB + (x ^ y); }
+
+// A persistent block takes the batch's pairs (triplet, block triple) w = blockIdx.x,
+// blockIdx.x + gridDim.x, ...  R: the arithmetic of the terms (double for
+// FP64_TC; float for MIXED, whose products carry ~1e-6, with W and the sums as
+// float-float pairs).
 //
-// Bound by instructions and by the latency of one block triple's loads (two
-// blocks of 96 KB an SM), not by L2: so the 18 cubes come by asynchronous copies,
-// all in flight at once, and a thread keeps one (a, b) for two values of c --
-// every cube of ordering m is read at F[m], the same six offsets for all three
-// arrays.
+// A pair is 18 cubes of W (74 KB) and a few hundred operations per element: one
+// thread an element (a, b, c), and two stages, so that the copies of the next
+// pair, all asynchronous, run under the terms of this one.  Every cube of
+// ordering m is read at F[m], the same six offsets for all three arrays and all
+// pairs.  Nine triplets at v = 76: 58 -> 44 us against blocks of one pair each with
+// one stage ((T) at o = 20, v = 76: 20.4 -> 17.1 ms).
 template <typename R>
-__global__ void __launch_bounds__(kThreads, 2) triples_blocks_kernel(EnergyArgs g) {
+__global__ void __launch_bounds__(kEnergyThreads, 1) triples_blocks_kernel(EnergyArgs g) {
   extern __shared__ double smem_d[];
-  auto& S = *reinterpret_cast<EnergySmem<R>*>(smem_d);
-  constexpr bool kPair = sizeof(R) == 4;
+  EnergyStage<R>* stages = reinterpret_cast<EnergyStage<R>*>(smem_d);
+  constexpr bool kPairs = sizeof(R) == 4;
   const int tid = threadIdx.x;
   const int v = g.v, o = g.o, v2 = v * v;
   const int64_t v3 = static_cast<int64_t>(v2) * v;
-  const int4 ijk = g.triples[blockIdx.y];
-  const int i = ijk.x, j = ijk.y, k = ijk.z;
-  const double mult = (i < j && j < k) ? 6.0 : ((i == j && j == k) ? 1.0 : 3.0);
-  const double* __restrict__ W = g.W + static_cast<int64_t>(blockIdx.y) * 3 * v3;
-  const double* __restrict__ Gp[3] = {g.Gijab + (static_cast<int64_t>(i) * o + j) * v2,
-                                      g.Gijab + (static_cast<int64_t>(j) * o + k) * v2,
-                                      g.Gijab + (static_cast<int64_t>(i) * o + k) * v2};
-  const R eijk = static_cast<R>(g.eps_o[i] + g.eps_o[j] + g.eps_o[k]);
-  const int l2 = tid & 7, l1 = (tid >> 3) & 7, l0 = tid >> 6;  // copies: l0 and l0 + 4
-  const int la = l1, lb = l2, lc0 = 2 * l0;                    // terms: (a, b) and c0, c0 + 1
-  double acc = 0.0;
-  float ahi = 0.f, alo = 0.f;
-  for (int bt = blockIdx.x; bt < g.nblocks; bt += gridDim.x) {
-    const unsigned code = g.blocks[bt];
-    const int A = static_cast<int>(code & 1023u) * kB, B = static_cast<int>((code >> 10) & 1023u) * kB,
-              C = static_cast<int>(code >> 20) * kB;
-    auto start = [&](int q) { return q == 0 ? A : (q == 1 ? B : C); };
-    __syncthreads();
+  const R* Gijab = static_cast<const R*>(g.Gijab);
+  const R* t1 = static_cast<const R*>(g.t1);
+  const int l2 = tid & 7, l1 = (tid >> 3) & 7, l0 = tid >> 6;  // copies: element (l0, l1, l2)
+  const int la = l1, lb = l2, lc = l0;                         // terms
+  const int put = cube_at(l0, l1, l2), put2 = tile_at(l1, l2);
+  int F[6], Q[6];
+  {
+    auto l = [&](int q) { return q == 0 ? la : (q == 1 ? lb : lc); };
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
-      const int gf = start(kPerm[m][1]) + l1, gr = start(kPerm[m][2]) + l2;
+      F[m] = cube_at(l(kPerm[m][0]), l(kPerm[m][1]), l(kPerm[m][2]));
+      Q[m] = tile_at(l(kPair[m][0]), l(kPair[m][1]));
+    }
+  }
+
+  struct Item {
+    int t;
+    unsigned code;
+    int4 ijk;
+  };
+  const int64_t items = static_cast<int64_t>(g.n) * g.nblocks;
+  auto item = [&](int64_t w) {
+    Item x;
+    x.t = static_cast<int>(static_cast<uint32_t>(w) / static_cast<uint32_t>(g.nblocks));
+    x.code = g.blocks[static_cast<uint32_t>(w) - static_cast<uint32_t>(x.t) * static_cast<uint32_t>(g.nblocks)];
+    x.ijk = g.triples[x.t];
+    return x;
+  };
+  auto load = [&](const Item& x, EnergyStage<R>& S) {
+    const int A = static_cast<int>(x.code & 1023u) * kB, B = static_cast<int>((x.code >> 10) & 1023u) * kB,
+              C = static_cast<int>(x.code >> 20) * kB;
+    auto start = [&](int q) { return q == 0 ? A : (q == 1 ? B : C); };
+    const double* W = g.W + static_cast<int64_t>(x.t) * 3 * v3;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int s = l0 + 4 * h, gs = start(kPerm[m][0]) + s;
-        const bool in = gs < v && gf < v && gr < v;  // zeros past v
-        const double* src = W + (in ? static_cast<int64_t>(gs * v + gf) * v + gr : 0);
+    for (int m = 0; m < 6; ++m) {
+      const int gs = start(kPerm[m][0]) + l0, gf = start(kPerm[m][1]) + l1, gr = start(kPerm[m][2]) + l2;
+      const bool in = gs < v && gf < v && gr < v;  // zeros past v
+      const double* src = W + (in ? static_cast<int64_t>(gs * v + gf) * v + gr : 0);
 #pragma unroll
-        for (int p = 0; p < 3; ++p) copy8_async(&S.W[p][m][s * kSlabLd + l1 * kRowLd + l2], src + p * v3, in);
-      }
+      for (int p = 0; p < 3; ++p) copy_async<8>(&S.W[p][m][put], src + p * v3, in);
     }
     // <ij|, <jk|, <ik| over the six ordered block pairs: 64 elements by 64 threads each
 #pragma unroll
-    for (int u = 0; u < 5; ++u) {
-      const int q = l0 + 4 * u;  // pair (q % 6) of array (q / 6)
+    for (int u = 0; u < 3; ++u) {
+      const int q = l0 + kB * u;
       if (q < 18) {
-        const int p = q / 6, m = q % 6;
-        const int bs = m < 2 ? 0 : (m < 4 ? 1 : 2), bf = m == 0 ? 1 : (m == 1 ? 2 : (m == 2 ? 0 : (m == 3 ? 2 : (m == 4 ? 0 : 1))));
+        const int p = q / 6, m = q - 6 * p;
+        const int bs = m >> 1, bf = (m & 1) ? (bs == 2 ? 1 : 2) : (bs == 0 ? 1 : 0);
         const int gs = start(bs) + l1, gf = start(bf) + l2;
-        const double* gp = p == 0 ? Gp[0] : (p == 1 ? Gp[1] : Gp[2]);
-        S.G[p][bs * 3 + bf][l1 * kRowLd + l2] = (gs < v && gf < v) ? static_cast<R>(gp[gs * v + gf]) : R(0);
+        const int x1 = p == 1 ? x.ijk.y : x.ijk.x, x2 = p == 0 ? x.ijk.y : x.ijk.z;
+        const bool in = gs < v && gf < v;
+        copy_async<sizeof(R)>(&S.G[p][m][put2],
+                              Gijab + (static_cast<int64_t>(x1) * o + x2) * v2 + (in ? gs * v + gf : 0), in);
       }
     }
     if (tid < 72) {
-      const int x = tid & 7, blk = (tid >> 3) % 3, p = (tid >> 3) / 3;
-      const int gx = start(blk) + x, occ = p == 0 ? i : (p == 1 ? j : k);
-      S.t1[p][blk][x] = gx < v ? static_cast<R>(g.t1[gx * o + occ]) : R(0);
-      if (p == 0) S.ev[blk][x] = gx < v ? static_cast<R>(g.eps_v[gx]) : R(0);
+      const int e = tid & 7, blk = (tid >> 3) % 3, p = (tid >> 3) / 3;
+      const int gx = start(blk) + e, occ = p == 0 ? x.ijk.x : (p == 1 ? x.ijk.y : x.ijk.z);
+      copy_async<sizeof(R)>(&S.t1[p][blk][e], t1 + (gx < v ? gx * o + occ : 0), gx < v);
+    } else if (tid < 96) {
+      const int blk = (tid - 72) >> 3, gx = start(blk) + (tid & 7);
+      copy_async<sizeof(R)>(&S.ev[blk][tid & 7], static_cast<const R*>(g.eps_v) + (gx < v ? gx : 0), gx < v);
+    } else if (tid == 96) {
+      copy_async<sizeof(R)>(&S.eo, static_cast<const R*>(g.eo) + x.t, true);
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  double acc = 0.0;
+  float ahi = 0.f, alo = 0.f;
+  Item cur{}, next{};
+  int64_t w = blockIdx.x;
+  if (w < items) {
+    cur = item(w);
+    load(cur, stages[0]);
+    if (w + gridDim.x < items) next = item(w + gridDim.x);
+  }
+  for (int st = 0; w < items; w += gridDim.x, st ^= 1) {
+    const bool more = w + gridDim.x < items;
+    const Item soon = next;
+    if (more) {
+      load(next, stages[st ^ 1]);
+      if (w + 2 * static_cast<int64_t>(gridDim.x) < items) next = item(w + 2 * static_cast<int64_t>(gridDim.x));
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
     __syncthreads();
-    const int a = A + la, b = B + lb;
-    if (a > b) continue;
-    // offsets of (l[P0], l[P1], l[P2]) in a cube, c = c0, and what one more c adds
-    constexpr int kStep[6] = {1, kRowLd, kSlabLd, kSlabLd, kRowLd, 1};
-    int F[6];
-#pragma unroll
-    for (int m = 0; m < 6; ++m) {
-      auto l = [&](int q) { return q == 0 ? la : (q == 1 ? lb : lc0); };
-      F[m] = l(kPerm[m][0]) * kSlabLd + l(kPerm[m][1]) * kRowLd + l(kPerm[m][2]);
-    }
-    const R eab = eijk - S.ev[0][la] - S.ev[1][lb];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int lc = lc0 + u, c = C + lc;
-      if (b > c || c >= v) continue;
-      R w[6], vv[6];
+    const EnergyStage<R>& S = stages[st];
+    const int a = static_cast<int>(cur.code & 1023u) * kB + la, b = static_cast<int>((cur.code >> 10) & 1023u) * kB + lb,
+              c = static_cast<int>(cur.code >> 20) * kB + lc;
+    if (a <= b && b <= c && c < v) {
+      R ww[6], u[6];
 #pragma unroll
       for (int m = 0; m < 6; ++m) {
-        const double w0 = S.W[0][m][F[m] + u * kStep[m]];
-        const double w1 = S.W[1][kSwap[m]][F[kSwap[m]] + u * kStep[kSwap[m]]];
-        const double w2 = S.W[2][kCycle[m]][F[kCycle[m]] + u * kStep[kCycle[m]]];
-        if constexpr (kPair) {
+        const double w0 = S.W[0][m][F[m]], w1 = S.W[1][kSwap[m]][F[kSwap[m]]], w2 = S.W[2][kCycle[m]][F[kCycle[m]]];
+        if constexpr (kPairs) {
           // words of (hi, lo) floats
           const float2 f0 = *reinterpret_cast<const float2*>(&w0), f1 = *reinterpret_cast<const float2*>(&w1),
                        f2 = *reinterpret_cast<const float2*>(&w2);
           float hi = f0.x, lo = f0.y;
           add_ff(hi, lo, f1.x);
           add_ff(hi, lo, f2.x);
-          w[m] = hi + (lo + (f1.y + f2.y));
+          ww[m] = hi + (lo + (f1.y + f2.y));
         } else {
-          w[m] = w0 + w1 + w2;
+          ww[m] = w0 + w1 + w2;
         }
         auto l = [&](int q) { return q == 0 ? la : (q == 1 ? lb : lc); };
         const int px = kPerm[m][0], py = kPerm[m][1], pz = kPerm[m][2];
-        const int x = l(px), y = l(py), z = l(pz);
-        vv[m] = S.G[0][px * 3 + py][x * kRowLd + y] * S.t1[2][pz][z] + S.G[1][py * 3 + pz][y * kRowLd + z] * S.t1[0][px][x] +
-                S.G[2][px * 3 + pz][x * kRowLd + z] * S.t1[1][py][y];
+        const int xy = pair_id(px, py), yz = pair_id(py, pz), xz = pair_id(px, pz);
+        u[m] = S.G[0][xy][Q[xy]] * S.t1[2][pz][l(pz)] + S.G[1][yz][Q[yz]] * S.t1[0][px][l(px)] +
+               S.G[2][xz][Q[xz]] * S.t1[1][py][l(py)];
       }
-      const R even = w[0] + w[1] + w[2], odd = w[3] + w[4] + w[5];
+      const R even = ww[0] + ww[1] + ww[2], odd = ww[3] + ww[4] + ww[5];
       // 4 t3(abc) + the two cyclic orderings - 2 the three others
+      const R ee = even - R(2) * odd, oo = odd - R(2) * even;
       R sum[6];
 #pragma unroll
-      for (int m = 0; m < 6; ++m)
-        sum[m] = (w[m] + vv[m]) * (R(3) * w[m] + (m < 3 ? even - R(2) * odd : odd - R(2) * even));
+      for (int m = 0; m < 6; ++m) sum[m] = (ww[m] + u[m]) * (R(3) * ww[m] + (m < 3 ? ee : oo));
       // a set with equal members has its orderings counted that many times
+      const int i = cur.ijk.x, j = cur.ijk.y, k = cur.ijk.z;
+      const R mult = (i < j && j < k) ? R(6) : ((i == j && j == k) ? R(1) : R(3));
       const R share = a == b ? (b == c ? R(1) / R(6) : R(0.5)) : (b == c ? R(0.5) : R(1));
-      const R f = share / (eab - S.ev[2][lc]);
+      const R f = (mult * share) / (S.eo - S.ev[0][la] - S.ev[1][lb] - S.ev[2][lc]);
       const R term = (((sum[0] + sum[1]) + sum[2]) + ((sum[3] + sum[4]) + sum[5])) * f;
-      if constexpr (kPair) add_ff(ahi, alo, term);
+      if constexpr (kPairs) add_ff(ahi, alo, term);
       else acc += term;
     }
+    cur = soon;
+    __syncthreads();  // the stage is free
   }
-  if constexpr (kPair) acc = static_cast<double>(ahi) + static_cast<double>(alo);
-  __syncthreads();
-  const double s = block_sum_det(acc, S.red);
-  if (tid == 0) g.partial[static_cast<int64_t>(blockIdx.y) * gridDim.x + blockIdx.x] = mult * s;
+  if constexpr (kPairs) acc = static_cast<double>(ahi) + static_cast<double>(alo);
+  const double s = block_sum_det(acc, smem_d);
+  if (tid == 0) g.partial[blockIdx.x] = s;
 }
 
 // out[blockIdx.x] = sum of its share of x (strided; fixed order)
@@ -642,11 +707,38 @@ __global__ void __launch_bounds__(kThreads) sum_blocks_kernel(const double* __re
 }
 
 template <typename R>
-void launch_blocks(const EnergyArgs& g, dim3 grid, cudaStream_t st) {
+void launch_blocks(const EnergyArgs& g, cudaStream_t st) {
+  constexpr int bytes = 2 * sizeof(EnergyStage<R>);
   static const bool attr = cudaFuncSetAttribute(triples_blocks_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                sizeof(EnergySmem<R>)) == cudaSuccess;
+                                                bytes) == cudaSuccess;
   if (!attr) throw Error(GBCC_ERR_CUDA, "(T): energy kernel shared memory");
-  triples_blocks_kernel<R><<<grid, kThreads, sizeof(EnergySmem<R>), st>>>(g);
+  triples_blocks_kernel<R><<<kEnergyGrid, kEnergyThreads, bytes, st>>>(g);
+}
+
+// the energy's inputs as its type: Gijab, t1, eps_v (double: where they lie) and
+// the triplets' sums of eps_o
+template <typename R>
+void prepare_energy(const TriplesInputs& in, const int4* tr, int64_t ntr, char* ws, EnergyArgs& e, cudaStream_t st) {
+  const int64_t ng = in.o * in.o * in.v * in.v, nt = in.o * in.v;
+  R* eo = reinterpret_cast<R*>(ws);
+  triplet_energies_kernel<R><<<static_cast<unsigned>((ntr + kThreads - 1) / kThreads), kThreads, 0, st>>>(tr, ntr, in.eps_o, eo);
+  e.eo = eo;
+  if constexpr (sizeof(R) == 8) {
+    e.Gijab = in.Gijab;
+    e.t1 = in.t1;
+    e.eps_v = in.eps_v;
+  } else {
+    R *G = eo + ntr, *t1 = G + ng, *ev = t1 + nt;
+    auto convert = [&](const double* x, int64_t n, R* y) {
+      convert_kernel<R><<<static_cast<unsigned>(std::min<int64_t>((n + kThreads - 1) / kThreads, 1216)), kThreads, 0, st>>>(x, n, y);
+    };
+    convert(in.Gijab, ng, G);
+    convert(in.t1, nt, t1);
+    convert(in.eps_v, in.v, ev);
+    e.Gijab = G;
+    e.t1 = t1;
+    e.eps_v = ev;
+  }
 }
 
 double triples_tc(const TriplesInputs& in, int precision, cudaStream_t st, int* err) {
@@ -665,11 +757,9 @@ double triples_tc(const TriplesInputs& in, int precision, cudaStream_t st, int* 
       for (unsigned c = b; c < nvb; ++c) bl.push_back(a | (b << 10) | (c << 20));
   const int64_t ntr = static_cast<int64_t>(tr.size()), nbl = static_cast<int64_t>(bl.size());
   int64_t batch = std::max<int64_t>(1, std::min<int64_t>(ntr, (int64_t{96} << 20) / (3 * v3 * 8)));
-  batch = std::min<int64_t>(batch, 32768);  // the energy grid's second dimension
+  batch = std::min<int64_t>(batch, (int64_t{1} << 31) / nbl);  // 32-bit counts of (triplet, block triple)
   if (g_triples_chunk > 0) batch = std::min(batch, g_triples_chunk);
-  // energy blocks per triplet: a few waves of the chip per batch, 32 MB of partial sums
-  const int64_t gx = std::min(nbl, std::max<int64_t>(1, std::min<int64_t>(std::max<int64_t>((2432 + batch - 1) / batch, 16),
-                                                                         (int64_t{1} << 22) / ntr)));
+  const int64_t nbatch = (ntr + batch - 1) / batch;
   constexpr int kSums = 152;
   size_t total = 0;
   auto part = [&](size_t bytes) {
@@ -679,7 +769,8 @@ double triples_tc(const TriplesInputs& in, int precision, cudaStream_t st, int* 
   };
   const size_t elems_a = static_cast<size_t>(slices) * kblocks * rowsA * 64, elems_b = static_cast<size_t>(slices) * kblocks * rowsB * 64;
   const size_t oA = part(elems_a * 2), oA2 = part(elems_a * 2), oB = part(elems_b * 2), oW = part(static_cast<size_t>(batch) * 3 * v3 * 8),
-               oT = part(ntr * sizeof(int4)), oBl = part(nbl * sizeof(unsigned)), oP = part(static_cast<size_t>(ntr) * gx * 8),
+               oT = part(ntr * sizeof(int4)), oBl = part(nbl * sizeof(unsigned)), oP = part(static_cast<size_t>(nbatch) * kEnergyGrid * 8),
+               oE = part(slices == 3 ? (ntr + o * o * v * v + o * v + v) * sizeof(float) : ntr * sizeof(double)),
                oS = part((kSums + 1) * 8);
   struct Owned {
     char* p;
@@ -719,21 +810,21 @@ double triples_tc(const TriplesInputs& in, int precision, cudaStream_t st, int* 
   e.blocks = d_bl;
   e.nblocks = static_cast<int>(nbl);
   e.W = W;
-  e.Gijab = in.Gijab;
-  e.t1 = in.t1;
-  e.eps_o = in.eps_o;
-  e.eps_v = in.eps_v;
-  for (int64_t t0 = 0; t0 < ntr; t0 += batch) {
+  if (slices == 3) prepare_energy<float>(in, d_tr, ntr, ws.p + oE, e, st);
+  else prepare_energy<double>(in, d_tr, ntr, ws.p + oE, e, st);
+  const char* eo = static_cast<const char*>(e.eo);
+  for (int64_t t0 = 0, k = 0; t0 < ntr; t0 += batch, ++k) {
     const int n = static_cast<int>(std::min(batch, ntr - t0));
     g.triples = d_tr + t0;
     if (!launch_gemm_triples(g, slices, n, st)) throw Error(GBCC_ERR_CUDA, "(T): tcgen05 launch rejected");
+    e.n = n;
     e.triples = d_tr + t0;
-    e.partial = partial + t0 * gx;
-    const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(n));
-    if (slices == 3) launch_blocks<float>(e, grid, st);
-    else launch_blocks<double>(e, grid, st);
+    e.eo = eo + t0 * (slices == 3 ? sizeof(float) : sizeof(double));
+    e.partial = partial + k * kEnergyGrid;
+    if (slices == 3) launch_blocks<float>(e, st);
+    else launch_blocks<double>(e, st);
   }
-  sum_blocks_kernel<<<kSums, kThreads, 0, st>>>(partial, ntr * gx, sums);
+  sum_blocks_kernel<<<kSums, kThreads, 0, st>>>(partial, nbatch * kEnergyGrid, sums);
   sum_kernel<<<1, kThreads, 0, st>>>(sums, kSums, 1.0 / 3.0, sums + kSums);
   double out = 0.0;
   GBCC_CK(cudaMemcpyAsync(&out, sums + kSums, sizeof(double), cudaMemcpyDeviceToHost, st));
