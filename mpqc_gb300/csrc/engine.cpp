@@ -1031,9 +1031,12 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
         PM.kord = order_by(kset, ref.lab);
       }
     } else {
-      // pack reads are cheapest along the storage order of the per-iteration operand
+      // pack reads are cheapest along the storage order of the per-iteration operand;
+      // a vector's order is free and lets a contraction name the order of a pack
+      // that another one makes
       const Ix* ref = nullptr;
-      if (!constM && !constN) ref = bigM.t->size() >= bigN.t->size() ? &bigM : &bigN;
+      if (!constM && !constN && p.N == 1) ref = &bigN;
+      else if (!constM && !constN) ref = bigM.t->size() >= bigN.t->size() ? &bigM : &bigN;
       else if (!constM) ref = &bigM;
       else if (!constN) ref = &bigN;
       else ref = &bigM;
@@ -1162,6 +1165,15 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
         op.Kpad = Kpad;
         // (the FP64_TC kernel's tensor maps end at the last row)
         op.rows_pad = emu ? op.rows : (side == 0 ? round_up(op.rows, kTcBM) : npanel);
+        if (!emu && side == 0 && p.N == 1) {
+          // the matrix of a vector product is padded as on the N side of a wide
+          // product, whose pack it can then share
+          int wbns[4];
+          const int nw = gemm_tc_bn_candidates(op.rows, true, wbns);
+          int64_t wide_rows = op.rows_pad;
+          for (int c = 0; c < nw; ++c) wide_rows = std::max(wide_rows, round_up(op.rows, wbns[c]));
+          op.rows_pad = round_up(wide_rows, kTcBM);
+        }
         GatherArgs& g = op.gather;
         g.Rpad = op.rows_pad;
         g.Cpad = Kpad;
@@ -1180,17 +1192,25 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
         const size_t need = static_cast<size_t>(slices) * op.rows_pad * Kpad;
         if (!op.constant) {
           bool frozen = true;
+          // labels by their place among rows and columns, so that packs of the same
+          // elements match whatever their contractions call the indices
+          auto place = [&](const std::string& lab) {
+            const std::string order = op.ext + op.kord;
+            std::string out;
+            for (char ch : lab) out += static_cast<char>('A' + order.find(ch));
+            return out;
+          };
           std::string sig;
           for (const auto& l : op.terms) {
             frozen = frozen && frozen_.count(l.x.t) > 0 && (!l.y.t || frozen_.count(l.y.t) > 0);
             // a single one-factor term is packed unscaled (plain copy)
             const double coef = (op.terms.size() == 1 && !l.y.t) ? 1.0 : l.coef;
-            sig += l.x.t->name + "(" + l.x.lab + ")";
-            if (l.y.t) sig += l.y.t->name + "(" + l.y.lab + ")";
+            sig += l.x.t->name + "(" + place(l.x.lab) + ")";
+            if (l.y.t) sig += l.y.t->name + "(" + place(l.y.lab) + ")";
             sig += "*" + std::to_string(coef) + ";";
           }
           if (frozen) {
-            op.sig = sig + op.ext + "|" + op.kord + "|" + (emu ? "fixed" : "float") + std::to_string(slices) + "|" +
+            op.sig = sig + std::to_string(op.ext.size()) + "|" + (emu ? "fixed" : "float") + std::to_string(slices) + "|" +
                      std::to_string(op.rows_pad) + "|" + std::to_string(Kpad);
             op.pack_elems = need;
             pack_uses_[op.sig].push_back(&op);
