@@ -138,8 +138,11 @@ void CcsdTensors::create(Engine& E, int64_t o, int64_t v, int64_t naux_df, int64
     Xai = &E.tensor("Xai", {naux, v, o}, true);
     Xab = &E.tensor("Xab", {naux, v, v}, true);
     Xac = &E.tensor("Xac", {v, v, naux});
-    // blocks of a: Gblk[a - a0][b][c][d] of at most ~4 GB
-    int64_t blk = std::max<int64_t>(1, std::min<int64_t>(v, (int64_t{1} << 29) / std::max<int64_t>(1, v * v * v)));
+    // blocks of a: Gblk[a - a0][b >= a0][c][d] of at most ~4 GB, and at least two: the
+    // second needs b from its own rows on, so two blocks form 3/4 of <ab|cd>.  v = 131:
+    // one block 6.51 ms a residual, two 6.18, three 6.35, four 6.45 (more, smaller
+    // pair products); v = 100: one 2.88, two 2.80, three or four 2.9 to 3.0
+    int64_t blk = std::max<int64_t>(1, std::min<int64_t>((v + 1) / 2, (int64_t{1} << 29) / std::max<int64_t>(1, v * v * v)));
     if (g_df_block_rows > 0) blk = std::min(v, g_df_block_rows);
     const int64_t rows_p_max = pairs_before(blk, v), rows_m_max = std::max<int64_t>(1, anti_before(blk, v));
     Tensor& gblk = E.tensor("df_gblk", {blk, v, v, v});

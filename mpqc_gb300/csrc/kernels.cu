@@ -145,11 +145,19 @@ __global__ void __launch_bounds__(kThreads) build_gpm_kernel(int64_t rows_v, int
 // The rows a in [a0, a1) of G+ / G- (pairs a <= b / a < b), from the block
 // Gblk[a - a0][b - a0][c][d] = <ab|cd> (b >= a0 only); output rows counted
 // from the block's first pair: sym(a,b) - sym(a0,a0) and anti(a,b) - anti(a0,a0+1).
+// Bound by memory (the block's rows a <= b read once, G+ and G- written once).  Both
+// <ab|cd> and <ab|dc> of a pair of 32 x 32 tiles (C, D), (D, C), C <= D, come from
+// shared memory, so every element is read once, along d: reading <ab|dc> down a
+// column fetched each 32-byte sector several times (v = 131, one block: 0.84 ->
+// 0.80 ms, 3 TB/s; the packed rows start at any multiple of 8 bytes).
 __global__ void __launch_bounds__(kThreads) build_gpm_rows_kernel(int64_t a0, int64_t a1, int64_t v,
                                                                   const double* __restrict__ Gblk,
                                                                   double* __restrict__ Gp, double* __restrict__ Gm) {
+  __shared__ double sx[32][33];  // [c][d] of tile (C, D)
+  __shared__ double sy[32][33];  // [d][c] of tile (D, C)
   const int64_t np = v * (v + 1) / 2, nm = v * (v - 1) / 2, w = v - a0;
   const int64_t p0 = pair_sym(a0, a0, v), m0 = a0 * (v - 1) - a0 * (a0 - 1) / 2;
+  const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
   for (int64_t row = blockIdx.x; row < (a1 - a0) * w; row += gridDim.x) {
     int64_t al, bl;
     divmod32(row, w, al, bl);
@@ -158,11 +166,26 @@ __global__ void __launch_bounds__(kThreads) build_gpm_rows_kernel(int64_t a0, in
     double* gp = Gp + (pair_sym(a, b, v) - p0) * np;
     double* gm = a < b ? Gm + (pair_anti(a, b, v) - m0) * nm : nullptr;
     const double* g = Gblk + row * v * v;
-    for (int64_t c = 0; c < v; ++c) {
-      for (int64_t d = c + threadIdx.x; d < v; d += blockDim.x) {
-        const double x = g[c * v + d], y = g[d * v + c];
-        gp[pair_sym(c, d, v)] = c < d ? x + y : x;
-        if (gm && c < d) gm[pair_anti(c, d, v)] = x - y;
+    for (int64_t C = 0; C < v; C += 32) {
+      for (int64_t D = C; D < v; D += 32) {
+#pragma unroll
+        for (int k = 0; k < 32; k += 8) {
+          const int64_t c = C + ty + k, d = D + tx;
+          if (c < v && d < v) sx[ty + k][tx] = g[c * v + d];
+          const int64_t d2 = D + ty + k, c2 = C + tx;
+          if (c2 < v && d2 < v) sy[ty + k][tx] = g[d2 * v + c2];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 32; k += 8) {
+          const int64_t c = C + ty + k, d = D + tx;
+          if (d < v && c <= d) {
+            const double x = sx[ty + k][tx], y = sy[tx][ty + k];
+            gp[pair_sym(c, d, v)] = c < d ? x + y : x;
+            if (gm && c < d) gm[pair_anti(c, d, v)] = x - y;
+          }
+        }
+        __syncthreads();
       }
     }
   }
