@@ -76,10 +76,10 @@ int gbcc_testing_fixed_split(const double* x, int64_t rows, int64_t cols, int ns
                              uint32_t* rowexp);
 
 /* C[M][N] = A[M][K] B[N][K]^T through the FP64-grade tensor-core path: six
- * fixed-point slices per operand row, one tcgen05 launch per weight class
- * (bn 0: the heuristic tile width; 32, 64 or 128), K split over CTAs when
- * ksplit > 1, CTA pairs (cta_group::2, 256-row tiles; bn 64 or 128) when
- * cta2.  *ms: the time of one product (all class launches). */
+ * fixed-point slices per operand row; one launch of gemm_multi_kernel (bn 0: the
+ * heuristic tile width; 32 or 64), K split over CTAs when ksplit > 1.  bn 128 or
+ * cta2 (CTA pairs, 256-row tiles; bn 64 or 128): one launch of gemm_tc_kernel
+ * per weight class.  *ms: the time of one product. */
 int gbcc_testing_gemm_fp64tc(int64_t M, int64_t N, int64_t K, const double* A, const double* B, double* C,
                              int bn, int ksplit, int cta2, int repeat, float* ms);
 
@@ -93,8 +93,8 @@ int gbcc_testing_gemm_fp64tc(int64_t M, int64_t N, int64_t K, const double* A, c
 int gbcc_testing_gemm_timeout(int64_t M, int64_t N, int64_t K, const double* A, const double* B, double* C,
                               uint64_t wait_ns, int64_t skip_stage, int* first, int* second);
 
-/* Triplets per (T) batch for calls from now on (0: the default, as many as
- * keep the batch's slice of t3 in L2). */
+/* Triplets per (T) batch for calls from now on (0: the default, 96 MB of t3 or,
+ * in FP64, 8 GB). */
 int gbcc_testing_triples_chunk(int64_t k);
 
 /* Peak probe: FP64 tensor-core throughput (mma.sync m8n8k4 .f64, DMMA) in
@@ -120,7 +120,7 @@ int gbcc_testing_r2_assemble(int64_t o, int64_t v, const double* r2u, const doub
 int gbcc_testing_fail_alloc(int64_t after, int64_t* count);
 
 /* Rows a per block of the density-fitted ladder for handles whose inputs are
- * set from now on (0: the default size, a block of (ab|cd) of at most 4 GB). */
+ * set from now on (0: the default, half of them, at most 4 GB of (ab|cd)). */
 int gbcc_testing_df_block_rows(int64_t rows);
 
 /* Symmetric eigensolver of the RHF driver (host code, no GPU needed):

@@ -57,7 +57,7 @@ int64_t anti_before(int64_t a, int64_t v) { return a * (v - 1) - a * (a - 1) / 2
 }  // namespace
 
 // rows a per block of the density-fitted ladder for handles set up from now
-// on (0: the default, Gblk of at most 4 GB); a test hook
+// on (0: the default, half of them, Gblk of at most 4 GB); a test hook
 int64_t g_df_block_rows = 0;
 
 void CcsdTensors::create(Engine& E, int64_t o, int64_t v, int64_t naux_df, int64_t nao_direct) {

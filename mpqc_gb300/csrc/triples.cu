@@ -21,7 +21,7 @@
 // columns a.  Each pair is one product over 2 K (gemm_multi.cu), written once
 // to its own array, in its own order; the energy kernel adds the three as it
 // reads them.  (Six read-modify-write passes of W through scattered offsets, one
-// per term and pair i, j, took 112 ms at o = 20, v = 76; this takes 20 ms.)  A
+// per term and pair i, j, took 112 ms at o = 20, v = 76; this takes 17 ms.)  A
 // batch is as many triplets as keep the three arrays in about 96 MB, most of
 // L2.  The energy kernel takes 8 x 8 x 8 blocks of a <= b <= c: all six
 // orderings of a set {a, b, c} are read once and give all six permuted W
