@@ -143,6 +143,11 @@ int gbcc_testing_profile_residual(struct gbcc_handle* h, int precision, int max_
  * calibration and tile tuning included (for choosing an ncu launch to skip to). */
 int gbcc_testing_tc_launches_total(gbcc_handle* h, int64_t* launches);
 
+/* 1 if gbcc_energy on a handle of `device` reads the n doubles at src where they
+ * lie, 0 if it copies them first (host arrays, another device's, an address that
+ * is no multiple of 8, or n past the end of the allocation). */
+int gbcc_testing_reads_in_place(const void* src, int64_t n, int device);
+
 /* Kernel launches of the last residual (every kernel of this library). */
 int gbcc_testing_last_launches(struct gbcc_handle* h, int* launches);
 

@@ -17,6 +17,8 @@
 #include <thread>
 #include <vector>
 
+#include <cuda.h>
+
 #include "../../include/gbcc.h"
 #include "triples.h"
 #include "../../include/gbcc_testing.h"
@@ -126,6 +128,34 @@ void create_tensors(gbcc_handle* h, int64_t naux, int64_t nao) {
 
 void copy_in(double* dst, const double* src, int64_t n, cudaStream_t st) {
   GBCC_CK(cudaMemcpyAsync(dst, src, static_cast<size_t>(n) * sizeof(double), cudaMemcpyDefault, st));
+}
+
+// Whether a kernel on `device` may read n doubles at src where they lie: memory
+// of that device, at a double's alignment, all n within its allocation.  What a
+// copy takes at any byte address, or refuses for running past its allocation,
+// a kernel would fault on.
+bool reads_in_place(const void* src, int64_t n, int device) {
+  if (reinterpret_cast<uintptr_t>(src) % alignof(double) != 0) return false;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, src) != cudaSuccess || at.type != cudaMemoryTypeDevice || at.device != device) {
+    cudaGetLastError();
+    return false;
+  }
+  using Range = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+  static const Range range = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const bool ok = cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &p, 12000, cudaEnableDefault, &q) ==
+                        cudaSuccess &&
+                    q == cudaDriverEntryPointSuccess;
+    if (!ok) cudaGetLastError();
+    return ok ? reinterpret_cast<Range>(p) : nullptr;
+  }();
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const auto at0 = reinterpret_cast<CUdeviceptr>(src);
+  if (!range || range(&base, &size, at0) != CUDA_SUCCESS || at0 < base) return false;
+  return at0 - base + static_cast<size_t>(n) * sizeof(double) <= size;
 }
 
 void copy_out(double* dst, const double* src, int64_t n, cudaStream_t st) {
@@ -649,6 +679,10 @@ void commit_inputs(gbcc_handle* h) {
 
 }  // namespace
 
+extern "C" int gbcc_testing_reads_in_place(const void* src, int64_t n, int device) {
+  return src && n > 0 && reads_in_place(src, n, device) ? 1 : 0;
+}
+
 // Thread-local message read by gbcc_last_error(NULL) (handle-free entry points).
 void gbcc_set_thread_error(const std::string& msg) { g_create_error = msg; }
 
@@ -936,14 +970,10 @@ gbcc_status gbcc_energy(gbcc_handle* h, const double* t1_ai, const double* t2_ab
     if (!t1_ai || !t2_abij || !r1_ai || !r2_abij)
       throw Error(GBCC_ERR_INVALID_ARG, "gbcc_energy: NULL argument");
     h->have_solution = false;
-    // device arrays are read where they are; host arrays through the handle's own
+    // device arrays are read where they are; the others through the handle's own
     gbcc::EnergyTermsArgs e = energy_args(h);
     auto on_device = [&](const double* src, gbcc::Tensor* own, int64_t n) -> const double* {
-      cudaPointerAttributes at{};
-      if (cudaPointerGetAttributes(&at, src) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
-          at.device == h->cfg.device)
-        return src;
-      cudaGetLastError();
+      if (reads_in_place(src, n, h->cfg.device)) return src;
       copy_in(own->d, src, n, h->stream);
       return own->d;
     };
