@@ -143,6 +143,13 @@ int gbcc_testing_profile_residual(struct gbcc_handle* h, int precision, int max_
  * calibration and tile tuning included (for choosing an ncu launch to skip to). */
 int gbcc_testing_tc_launches_total(gbcc_handle* h, int64_t* launches);
 
+/* The operation `site` (counted from 0) of the next residual pass that reaches it
+ * fails on the host instead of being launched, once (-1: none). */
+int gbcc_testing_fail_site(int64_t site);
+
+/* Lanes of handle h, beside its stream, that are still running kernels. */
+int gbcc_testing_lanes_busy(struct gbcc_handle* h, int* busy);
+
 /* 1 if gbcc_energy on a handle of `device` reads the n doubles at src where they
  * lie, 0 if it copies them first (host arrays, another device's, an address that
  * is no multiple of 8, or n past the end of the allocation). */

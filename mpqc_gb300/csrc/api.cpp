@@ -232,6 +232,19 @@ int hi_prec(const gbcc_handle* h) {
 // whether the handle's plan includes the FP64_TC contractions
 bool uses_fp64_tc(const gbcc_handle* h) { return hi_prec(h) == GBCC_PREC_FP64_TC; }
 
+// One EXEC pass of the residual program; if it fails midway, nothing of it is
+// still running when the exception leaves.
+void exec_residual(gbcc_handle* h, int precision) {
+  try {
+    h->eng->begin(gbcc::Mode::kExec, precision);
+    gbcc::residual_program(*h->eng, h->S);
+    h->eng->end();
+  } catch (...) {
+    h->eng->abandon();
+    throw;
+  }
+}
+
 // r1, r2 of the device-resident t1, t2, tau.  The first evaluation in each
 // precision is captured into a CUDA graph (every launch of the EXEC pass has
 // fixed pointers, sizes and tensor maps once the plan is finalised); later
@@ -239,9 +252,7 @@ bool uses_fp64_tc(const gbcc_handle* h) { return hi_prec(h) == GBCC_PREC_FP64_TC
 int enqueue_residual_program(gbcc_handle* h, int precision) {
   h->eng->prepack(precision);  // once per plan; no workspace changes
   auto direct = [&]() {
-    h->eng->begin(gbcc::Mode::kExec, precision);
-    gbcc::residual_program(*h->eng, h->S);
-    h->eng->end();
+    exec_residual(h, precision);
     return h->eng->kernel_launches();
   };
   if (!h->cfg.use_graphs || h->profiling || h->calibrating) return direct();
@@ -325,9 +336,7 @@ cudaGraph_t capture_residual_graph(gbcc_handle* h, int precision) {
   cudaGraph_t g = nullptr;
   GBCC_CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   try {
-    h->eng->begin(gbcc::Mode::kExec, precision);
-    gbcc::residual_program(*h->eng, h->S);
-    h->eng->end();
+    exec_residual(h, precision);
   } catch (...) {
     cudaStreamEndCapture(h->stream, &g);
     if (g) cudaGraphDestroy(g);
@@ -678,6 +687,12 @@ void commit_inputs(gbcc_handle* h) {
 }
 
 }  // namespace
+
+extern "C" int gbcc_testing_lanes_busy(gbcc_handle* h, int* busy) {
+  if (!h || !busy) return GBCC_ERR_INVALID_ARG;
+  *busy = h->eng->lanes_busy();
+  return GBCC_OK;
+}
 
 extern "C" int gbcc_testing_reads_in_place(const void* src, int64_t n, int device) {
   return src && n > 0 && reads_in_place(src, n, device) ? 1 : 0;

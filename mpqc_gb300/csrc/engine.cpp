@@ -73,6 +73,10 @@ void tune_clear() {
 std::atomic<int64_t> g_alloc_count{0};
 std::atomic<int64_t> g_fail_alloc_after{-1};
 
+// test hook (gbcc_testing_fail_site): the operation of an EXEC pass that fails
+// instead of being launched, once (-1: none)
+std::atomic<int64_t> g_fail_site{-1};
+
 void* dev_alloc(size_t bytes) {
   if (bytes == 0) bytes = 256;
   ++g_alloc_count;
@@ -407,6 +411,26 @@ void Engine::wait(int k, int m) {
   if (mode_ == Mode::kExec && concurrent()) GBCC_CK(cudaStreamWaitEvent(lane_ws_[k].stream, marks_.at(m), 0));
 }
 
+void Engine::abandon() noexcept {
+  for (int k = 1; k < nlanes_; ++k) {
+    cudaStream_t s = lane_ws_[k].stream;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (s && cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+      cudaStreamSynchronize(s);
+  }
+  cudaGetLastError();
+  lane_ = 0;
+  run_ = stream_;
+  ws_ = &lane_ws_[0];
+}
+
+int Engine::lanes_busy() const {
+  int n = 0;
+  for (int k = 1; k < nlanes_; ++k)
+    if (lane_ws_[k].stream && cudaStreamQuery(lane_ws_[k].stream) == cudaErrorNotReady) ++n;
+  return n;
+}
+
 Tensor& Engine::tensor(const std::string& name, std::initializer_list<int64_t> dims, bool constant) {
   auto it = tensors_.find(name);
   if (it != tensors_.end()) {
@@ -508,6 +532,10 @@ Site& Engine::site() {
     return *sites_.back();
   }
   if (cursor_ >= sites_.size()) throw Error(GBCC_ERR_STATE, "engine: program longer than its plan");
+  if (g_fail_site.load() == static_cast<int64_t>(cursor_)) {
+    g_fail_site.store(-1);
+    throw Error(GBCC_ERR_CUDA, "operation not launched: injected failure (test hook)");
+  }
   Site& s = *sites_[cursor_++];
   ws_ = &lane_ws_[s.lane];
   run_ = concurrent() ? ws_->stream : stream_;
@@ -1371,6 +1399,12 @@ void Engine::prepack(int precision) {
 }
 
 }  // namespace gbcc
+
+extern "C" int gbcc_testing_fail_site(int64_t site) {
+  if (site < -1) return GBCC_ERR_INVALID_ARG;
+  gbcc::g_fail_site.store(site);
+  return GBCC_OK;
+}
 
 extern "C" int gbcc_testing_fail_alloc(int64_t after, int64_t* count) {
   if (after < -1) return GBCC_ERR_INVALID_ARG;

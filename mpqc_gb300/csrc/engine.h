@@ -218,6 +218,11 @@ class Engine {
   int mark(int k);
   void wait(int k, int m);
   void set_lanes(bool on) { lanes_on_ = on; }
+  // After an EXEC pass that ended in an exception: waits for what its lanes have
+  // been given (end() did not join them), so that nothing of it still runs beside
+  // what the stream is given next.  Lanes in a capture have nothing running.
+  void abandon() noexcept;
+  int lanes_busy() const;  // lanes beside the stream that are still running
 
   // Statistics of the last EXEC pass (FLOPs of the contractions as planned).
   double flops() const { return flops_; }
