@@ -763,10 +763,11 @@ void Engine::launch_fixed(const GemmPlan& p, __nv_bfloat16* const panel[2]) {
   t.hb_per_split = static_cast<int>(p.k_per_split);
   t.partial = ws_->wpart;
   t.err = err_;
-  if (!launch_gemm_fixed(t, run_)) throw Error(GBCC_ERR_CUDA, "tcgen05 GEMM launch rejected (tensor map or size)");
-  ++n_tc_;
-  ++tc_total_;
-  ++n_launch_;
+  const int n = launch_gemm_fixed(t, run_);
+  if (n < 1) throw Error(GBCC_ERR_CUDA, "tcgen05 GEMM launch rejected (tensor map or size)");
+  n_tc_ += n;
+  tc_total_ += n;
+  n_launch_ += n;
   if (p.ksplit > 1) {
     launch_splitk_reduce(p.M, p.N, p.ksplit, ws_->wpart, round_up(p.M, kTcBM), round_up(p.N, p.bn), p.C, p.cm, p.cn,
                          p.alpha, p.beta, run_);

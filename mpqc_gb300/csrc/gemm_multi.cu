@@ -19,8 +19,18 @@
 // accumulators of BN <= 64 columns, two more than a chunk needs: the MMAs of
 // the next chunk start while the epilogue still drains this one.  The epilogue
 // adds the finished sums to two float-float pairs per output, classes 0-2 and
-// 3-5: the units of a pair's classes span 16 bits, so its TwoSums are exact up
-// to K = 2^18 (30 + log2 K <= 48 bits), and the pairs meet in FP64.
+// 3-5, and the pairs meet in FP64.  A pair is exact while its low word holds every
+// rounding error of its high one.  In units of class 2 the sum of classes 0-2 over
+// K elements is at most 2^14 (2^16 + 2 2^8 + 3) K, below 2^45 for K <= 32000, so an
+// addition to the high word errs by at most 2^20 units.  The pair is renormalised
+// every four chunks, and a low word of 2^20 with twelve more errors is within the
+// 2^24 units that FP32 holds: exact.  Of classes 3-5, sixteen bits further down,
+// an addition then loses two units of class 5 at most, 2^-53 of a largest product,
+// 10^-4 of what the classes left out (6 on) may hold.  K beyond that runs in
+// windows of 32000 elements, a launch each, added to C (or to the partial tiles)
+// in FP64.  (Never renormalised and in one window, sums of one sign were off by
+// 1.5e-12 at K = 65536 and 3.6e-12 at 262144.  Renormalising every chunk instead
+// cost 5 %, windows of 8000 12 % of 4096 x 528 x 51360.)
 //
 // Three slices (the BF16 split; (T) only): one accumulator per stage (12 MMAs,
 // no longer than the 16 of gemm_tc_kernel), summed per segment in FP32
@@ -100,6 +110,9 @@ struct MultiCfg {
   static constexpr int kOut = BN / (kEpiWarps / 4);  // columns per epilogue thread
 };
 
+constexpr int kWindow = 1000;  // stages of a tile in one launch (six slices): 200 chunks
+constexpr int kRenorm = 4;     // chunks between renormalisations
+
 // one output tile: where its operand segments and its output lie
 struct Tile {
   int nseg;
@@ -148,8 +161,9 @@ __device__ __forceinline__ Tile decode(const GemmMultiArgs& g, int t, int BN) {
     T.row0 = mt * BM;
     T.n0 = nt * BN;
     T.b_row[0] = T.n0;
-    T.hb0 = T.split * g.hb_per_split;
-    T.hb1 = min(g.hbs, T.hb0 + g.hb_per_split);
+    const int end = min(g.hbs, (T.split + 1) * g.hb_per_split);
+    T.hb0 = min(end, T.split * g.hb_per_split + g.hb_first);
+    T.hb1 = min(end, T.hb0 + kWindow);
   }
   return T;
 }
@@ -315,6 +329,7 @@ __global__ void __launch_bounds__(MultiCfg<SL, BN>::kThreads, 1)
         x2[SL == 3 ? 0 : j] = x3[SL == 3 ? 0 : j] = 0.f;
       }
       const int nchunks = (T.hb1 - T.hb0 + Cfg::kChunk - 1) / Cfg::kChunk;
+      int unnorm = 0;  // chunks since the pairs were renormalised
       for (int seg = 0; seg < T.nseg && ok; ++seg) {
         if constexpr (SL == 3) {
           if (seg == 1) {
@@ -360,6 +375,16 @@ __global__ void __launch_bounds__(MultiCfg<SL, BN>::kThreads, 1)
           __syncwarp();
           if (lane == 0) mbar_arrive(&acc_empty[b]);
         };
+        auto renormalise = [&](auto& hi, auto& lo) {
+#pragma unroll
+          for (int j = 0; j < OUT; ++j) {
+            const float h = hi[j];
+            hi[j] = __fadd_rn(h, lo[j]);
+            // the rounding error of that sum (TwoSum)
+            const float v = __fsub_rn(hi[j], h);
+            lo[j] = __fadd_rn(__fsub_rn(h, __fsub_rn(hi[j], v)), __fsub_rn(lo[j], v));
+          }
+        };
         for (int ch = 0; ch < nchunks && ok; ++ch, q += NC) {
           if constexpr (SL == 3) {
             drain(0, x0, x1);
@@ -368,6 +393,11 @@ __global__ void __launch_bounds__(MultiCfg<SL, BN>::kThreads, 1)
             for (int c = 0; c < SL / 2 && ok; ++c) drain(c, x2, x3);  // classes 5, 4, 3
 #pragma unroll 1
             for (int c = SL / 2; c < SL && ok; ++c) drain(c, x0, x1);  // classes 2, 1, 0
+            if (++unnorm == kRenorm) {
+              unnorm = 0;
+              renormalise(x2, x3);
+              renormalise(x0, x1);
+            }
           }
         }
       }
@@ -447,7 +477,8 @@ __global__ void __launch_bounds__(MultiCfg<SL, BN>::kThreads, 1)
 #pragma unroll
             for (int r = 0; r < SC; ++r) {
               const int rr = rj + RP * r;
-              P[(static_cast<int64_t>(T.row0) + qd * 32 + rr) * g.Npad] = s8[rr * LD + cj];
+              double* at = P + (static_cast<int64_t>(T.row0) + qd * 32 + rr) * g.Npad;
+              *at = g.hb_first ? *at + s8[rr * LD + cj] : s8[rr * LD + cj];
             }
           } else if (n < g.N) {
             const int64_t on = g.cn[n];
@@ -534,9 +565,10 @@ int triples_bn(int slices, int64_t v) {
   return static_cast<int>(slices == 3 ? std::max<int64_t>(bn, 32) : (bn <= 32 ? 32 : 64));
 }
 
-bool launch_gemm_fixed(GemmMultiArgs g, cudaStream_t st) {
-  if (g.M <= 0 || g.N <= 0) return true;
-  if (g.K < 1 || (g.bn != 32 && g.bn != 64) || g.kblocks * 64 < g.K || g.a_rows < g.M || g.b_rows < g.N) return false;
+int launch_gemm_fixed(GemmMultiArgs g, cudaStream_t st) {
+  if (g.M < 1 || g.N < 1 || g.K < 1 || (g.bn != 32 && g.bn != 64) || g.kblocks * 64 < g.K || g.a_rows < g.M ||
+      g.b_rows < g.N)
+    return 0;
   g.hbs = static_cast<int>((g.K + HB - 1) / HB);
   g.last_k16 = (g.K - 1) % HB < 16 ? 1 : 2;
   const int64_t ntm = (g.M + BM - 1) / BM, ntn = (g.N + g.bn - 1) / g.bn;
@@ -545,17 +577,23 @@ bool launch_gemm_fixed(GemmMultiArgs g, cudaStream_t st) {
   if (g.ksplit > 1 && (!g.partial || g.hb_per_split < 1 ||
                        static_cast<int64_t>(g.ksplit - 1) * g.hb_per_split >= g.hbs ||
                        static_cast<int64_t>(g.ksplit) * g.hb_per_split < g.hbs))
-    return false;
+    return 0;
   const int64_t tiles = ntm * ntn * g.ksplit;
-  if (tiles > (1LL << 30) || g.M > (1LL << 30) || g.N > (1LL << 30)) return false;
+  if (tiles > (1LL << 30) || g.M > (1LL << 30) || g.N > (1LL << 30)) return 0;
   g.ntm = static_cast<int>(ntm);
   g.ntn = static_cast<int>(ntn);
   g.tiles = static_cast<int>(tiles);
   g.Mpad = ntm * BM;
   g.Npad = ntn * g.bn;
   CUtensorMap a;
-  if (!panel_map(&a, g.A, kFixedSlices, g.a_rows, g.kblocks, BM)) return false;
-  return g.bn == 32 ? launch<kFixedSlices, 32, false>(g, a, a, st) : launch<kFixedSlices, 64, false>(g, a, a, st);
+  if (!panel_map(&a, g.A, kFixedSlices, g.a_rows, g.kblocks, BM)) return 0;
+  int n = 0;
+  for (g.hb_first = 0; g.hb_first < g.hb_per_split; g.hb_first += kWindow, ++n) {
+    if (!(g.bn == 32 ? launch<kFixedSlices, 32, false>(g, a, a, st) : launch<kFixedSlices, 64, false>(g, a, a, st)))
+      return 0;
+    g.beta = 1.0;
+  }
+  return n;
 }
 
 bool launch_gemm_triples(GemmMultiArgs g, int slices, int ntriples, cudaStream_t st) {

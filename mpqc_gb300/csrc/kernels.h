@@ -296,13 +296,14 @@ struct GemmMultiArgs {
   const int4* triples;
   int o, v;
   double* W;
-  // set by the launchers
-  int hbs, last_k16, ntm, ntn, nts, ntf, tiles;
+  // set by the launchers; hb_first: first stage of each K split in this launch
+  int hb_first, hbs, last_k16, ntm, ntn, nts, ntf, tiles;
   int64_t Mpad, Npad;
 };
 // FP64-grade product of fixed-point panels (kFixedSlices slices); bn 32 or 64
-// (gemm_multi_bn).  false: nothing launched (bad size or tensor map).
-bool launch_gemm_fixed(GemmMultiArgs g, cudaStream_t st);
+// (gemm_multi_bn).  Returns the kernels launched, one per window of 32000 elements
+// of a K split; 0 for a bad size or tensor map.
+int launch_gemm_fixed(GemmMultiArgs g, cudaStream_t st);
 int gemm_multi_bn(int64_t N);
 // The three sums of two (T) permutation terms of each triple (triples.cu);
 // A, A2: rows (x, p, q) and (x, q, p) of o v^2, B: rows (y, z, r) of o^2 v

@@ -548,7 +548,7 @@ extern "C" int gbcc_testing_gemm_fp64tc(int64_t M, int64_t N, int64_t K, const d
     }
     auto run = [&]() {
       if (multi) {
-        if (!launch_gemm_fixed(u, st)) throw Error(GBCC_ERR_CUDA, "tcgen05 launch rejected");
+        if (launch_gemm_fixed(u, st) < 1) throw Error(GBCC_ERR_CUDA, "tcgen05 launch rejected");
         if (u.ksplit > 1) launch_splitk_reduce(M, N, u.ksplit, u.partial, Mpad, Npad, dC, cm, cn, 1.0, 0.0, st);
         return;
       }
