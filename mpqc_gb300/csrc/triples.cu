@@ -479,8 +479,8 @@ struct EnergyStage {
   double W[3][6][kCube];           // float2 (three slices) or double words
   R G[3][6][kB * kB];              // <ij|, <jk|, <ik| over ordered block pairs
   R t1[3][3][kB];                  // t1 of i, j, k over the blocks
-  R ev[3][kB];
-  R eo;                            // eps_i + eps_j + eps_k
+  double ev[3][kB];
+  double eo;                       // eps_i + eps_j + eps_k
 };
 
 struct EnergyArgs {
@@ -490,10 +490,10 @@ struct EnergyArgs {
   const unsigned* blocks;     // block triples A <= B <= C, 10 bits each
   int nblocks;
   const double* W;            // [triplet][3][v][v][v]
-  const void* Gijab;          // of type R, as the rest
+  const void* Gijab;          // of type R, as t1
   const void* t1;
-  const void* eps_v;
-  const void* eo;             // per triplet of this batch
+  const double* eps_v;
+  const double* eo;           // per triplet of this batch
   double* partial;            // [gridDim.x]
 };
 
@@ -505,11 +505,11 @@ __global__ void __launch_bounds__(kThreads) convert_kernel(const double* __restr
     y[e] = static_cast<R>(x[e]);
 }
 
-template <typename R>
 __global__ void __launch_bounds__(kThreads) triplet_energies_kernel(const int4* __restrict__ tr, int64_t n,
-                                                                    const double* __restrict__ eps_o, R* __restrict__ eo) {
+                                                                    const double* __restrict__ eps_o,
+                                                                    double* __restrict__ eo) {
   const int64_t t = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
-  if (t < n) eo[t] = static_cast<R>(eps_o[tr[t].x] + eps_o[tr[t].y] + eps_o[tr[t].z]);
+  if (t < n) eo[t] = eps_o[tr[t].x] + eps_o[tr[t].y] + eps_o[tr[t].z];
 }
 
 // hi + lo += x (TwoSum), for sums of many FP32 terms
@@ -541,8 +541,11 @@ __device__ __forceinline__ int tile_at(int x, int y) { return x * kB + (x ^ y); 
 
 // A persistent block takes the batch's pairs (triplet, block triple) w = blockIdx.x,
 // blockIdx.x + gridDim.x, ...  R: the arithmetic of the terms (double for
-// FP64_TC; float for MIXED, whose products carry ~1e-6, with W and the sums as
-// float-float pairs).
+// FP64_TC; float for MIXED, whose products carry ~1e-6: FP32 rounds W, a term and
+// its weight, and nothing that is summed -- the arrays of W, the six orderings of a
+// set and the running sum are float-float sums, the denominators FP64.  With plain
+// FP32 sums of the orderings and denominators (T) at o = 20, v = 76 took 16.97 ms,
+// so 17.33, with the running sum in FP64 17.66).
 //
 // A pair is 18 cubes of W (74 KB) and a few hundred operations per element: one
 // thread an element (a, b, c), and two stages, so that the copies of the next
@@ -619,9 +622,9 @@ __global__ void __launch_bounds__(kEnergyThreads, 1) triples_blocks_kernel(Energ
       copy_async<sizeof(R)>(&S.t1[p][blk][e], t1 + (gx < v ? gx * o + occ : 0), gx < v);
     } else if (tid < 96) {
       const int blk = (tid - 72) >> 3, gx = start(blk) + (tid & 7);
-      copy_async<sizeof(R)>(&S.ev[blk][tid & 7], static_cast<const R*>(g.eps_v) + (gx < v ? gx : 0), gx < v);
+      copy_async<8>(&S.ev[blk][tid & 7], g.eps_v + (gx < v ? gx : 0), gx < v);
     } else if (tid == 96) {
-      copy_async<sizeof(R)>(&S.eo, static_cast<const R*>(g.eo) + x.t, true);
+      copy_async<8>(&S.eo, g.eo + x.t, true);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -681,16 +684,25 @@ __global__ void __launch_bounds__(kEnergyThreads, 1) triples_blocks_kernel(Energ
       const int i = cur.ijk.x, j = cur.ijk.y, k = cur.ijk.z;
       const R mult = (i < j && j < k) ? R(6) : ((i == j && j == k) ? R(1) : R(3));
       const R share = a == b ? (b == c ? R(1) / R(6) : R(0.5)) : (b == c ? R(0.5) : R(1));
-      const R f = (mult * share) / (S.eo - S.ev[0][la] - S.ev[1][lb] - S.ev[2][lc]);
-      const R term = (((sum[0] + sum[1]) + sum[2]) + ((sum[3] + sum[4]) + sum[5])) * f;
-      if constexpr (kPairs) add_ff(ahi, alo, term);
-      else acc += term;
+      const double d = S.eo - S.ev[0][la] - S.ev[1][lb] - S.ev[2][lc];
+      const R f = (mult * share) / static_cast<R>(d);
+      if constexpr (kPairs) {
+        float hi[3] = {sum[0], sum[2], sum[4]}, lo[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) add_ff(hi[q], lo[q], sum[2 * q + 1]);
+        add_ff(hi[0], lo[0], hi[1]);
+        add_ff(hi[0], lo[0], hi[2]);
+        const float p = hi[0] * f;
+        add_ff(ahi, alo, p);
+        alo += fmaf(hi[0], f, -p) + (lo[0] + (lo[1] + lo[2])) * f;
+      } else {
+        acc += (((sum[0] + sum[1]) + sum[2]) + ((sum[3] + sum[4]) + sum[5])) * f;
+      }
     }
     cur = soon;
     __syncthreads();  // the stage is free
   }
-  if constexpr (kPairs) acc = static_cast<double>(ahi) + static_cast<double>(alo);
-  const double s = block_sum_det(acc, smem_d);
+  const double s = block_sum_det(acc + static_cast<double>(ahi) + static_cast<double>(alo), smem_d);
   if (tid == 0) g.partial[blockIdx.x] = s;
 }
 
@@ -715,29 +727,27 @@ void launch_blocks(const EnergyArgs& g, cudaStream_t st) {
   triples_blocks_kernel<R><<<kEnergyGrid, kEnergyThreads, bytes, st>>>(g);
 }
 
-// the energy's inputs as its type: Gijab, t1, eps_v (double: where they lie) and
+// the energy's inputs: Gijab and t1 as its type (double: where they lie), eps_v and
 // the triplets' sums of eps_o
 template <typename R>
 void prepare_energy(const TriplesInputs& in, const int4* tr, int64_t ntr, char* ws, EnergyArgs& e, cudaStream_t st) {
   const int64_t ng = in.o * in.o * in.v * in.v, nt = in.o * in.v;
-  R* eo = reinterpret_cast<R*>(ws);
-  triplet_energies_kernel<R><<<static_cast<unsigned>((ntr + kThreads - 1) / kThreads), kThreads, 0, st>>>(tr, ntr, in.eps_o, eo);
+  double* eo = reinterpret_cast<double*>(ws);
+  triplet_energies_kernel<<<static_cast<unsigned>((ntr + kThreads - 1) / kThreads), kThreads, 0, st>>>(tr, ntr, in.eps_o, eo);
   e.eo = eo;
+  e.eps_v = in.eps_v;
   if constexpr (sizeof(R) == 8) {
     e.Gijab = in.Gijab;
     e.t1 = in.t1;
-    e.eps_v = in.eps_v;
   } else {
-    R *G = eo + ntr, *t1 = G + ng, *ev = t1 + nt;
+    R *G = reinterpret_cast<R*>(eo + ntr), *t1 = G + ng;
     auto convert = [&](const double* x, int64_t n, R* y) {
       convert_kernel<R><<<static_cast<unsigned>(std::min<int64_t>((n + kThreads - 1) / kThreads, 1216)), kThreads, 0, st>>>(x, n, y);
     };
     convert(in.Gijab, ng, G);
     convert(in.t1, nt, t1);
-    convert(in.eps_v, in.v, ev);
     e.Gijab = G;
     e.t1 = t1;
-    e.eps_v = ev;
   }
 }
 
@@ -770,7 +780,7 @@ double triples_tc(const TriplesInputs& in, int precision, cudaStream_t st, int* 
   const size_t elems_a = static_cast<size_t>(slices) * kblocks * rowsA * 64, elems_b = static_cast<size_t>(slices) * kblocks * rowsB * 64;
   const size_t oA = part(elems_a * 2), oA2 = part(elems_a * 2), oB = part(elems_b * 2), oW = part(static_cast<size_t>(batch) * 3 * v3 * 8),
                oT = part(ntr * sizeof(int4)), oBl = part(nbl * sizeof(unsigned)), oP = part(static_cast<size_t>(nbatch) * kEnergyGrid * 8),
-               oE = part(slices == 3 ? (ntr + o * o * v * v + o * v + v) * sizeof(float) : ntr * sizeof(double)),
+               oE = part(ntr * sizeof(double) + (slices == 3 ? (o * o * v * v + o * v) * sizeof(float) : 0)),
                oS = part((kSums + 1) * 8);
   struct Owned {
     char* p;
@@ -812,14 +822,14 @@ double triples_tc(const TriplesInputs& in, int precision, cudaStream_t st, int* 
   e.W = W;
   if (slices == 3) prepare_energy<float>(in, d_tr, ntr, ws.p + oE, e, st);
   else prepare_energy<double>(in, d_tr, ntr, ws.p + oE, e, st);
-  const char* eo = static_cast<const char*>(e.eo);
+  const double* eo = e.eo;
   for (int64_t t0 = 0, k = 0; t0 < ntr; t0 += batch, ++k) {
     const int n = static_cast<int>(std::min(batch, ntr - t0));
     g.triples = d_tr + t0;
     if (!launch_gemm_triples(g, slices, n, st)) throw Error(GBCC_ERR_CUDA, "(T): tcgen05 launch rejected");
     e.n = n;
     e.triples = d_tr + t0;
-    e.eo = eo + t0 * (slices == 3 ? sizeof(float) : sizeof(double));
+    e.eo = eo + t0;
     e.partial = partial + k * kEnergyGrid;
     if (slices == 3) launch_blocks<float>(e, st);
     else launch_blocks<double>(e, st);
