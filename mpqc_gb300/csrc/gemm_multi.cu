@@ -437,12 +437,12 @@ __global__ void __launch_bounds__(MultiCfg<SL, BN>::kThreads, 1)
       // neighbouring lanes write neighbouring columns
       constexpr int SC = Cfg::kStgCols, LD = Cfg::kStgLd, RP = 32 / SC;  // RP rows per store
       const int cj = lane % SC, rj = lane / SC;
-      int roff[SC];  // (T): offsets of this lane's rows in the sum array, -1 past v
+      int rrow[SC];  // (T): this lane's rows (slow, fast) of the sum array, -1 past v
       if constexpr (TRIPLES) {
 #pragma unroll
         for (int r = 0; r < SC; ++r) {
           const int lr = qd * 32 + rj + RP * r, slow = T.row0 + lr / 16, fast = T.fast0 + lr % 16;
-          roff[r] = (slow < g.v && fast < g.v) ? (slow * g.v + fast) * g.v : -1;
+          rrow[r] = (slow < g.v && fast < g.v) ? slow * g.v + fast : -1;
         }
       }
 #pragma unroll
@@ -468,7 +468,8 @@ __global__ void __launch_bounds__(MultiCfg<SL, BN>::kThreads, 1)
             double* out = g.W + T.out + n;
 #pragma unroll
             for (int r = 0; r < SC; ++r)
-              if (roff[r] >= 0) out[roff[r]] = reinterpret_cast<const double*>(stg)[(rj + RP * r) * LD + cj];
+              if (rrow[r] >= 0)
+                out[static_cast<int64_t>(rrow[r]) * g.v] = reinterpret_cast<const double*>(stg)[(rj + RP * r) * LD + cj];
           }
         } else {
           const double* s8 = reinterpret_cast<const double*>(stg);
@@ -606,8 +607,9 @@ bool launch_gemm_triples(GemmMultiArgs g, int slices, int ntriples, cudaStream_t
   g.ntf = (g.v + 15) / 16;
   g.ntn = (g.v + g.bn - 1) / g.bn;
   const int64_t tiles = static_cast<int64_t>(ntriples) * 3 * g.nts * g.ntf * g.ntn;
+  // (32-bit rows of B, virtual pairs and tiles; offsets in the sums are 64-bit)
   if (tiles > (1LL << 30) || static_cast<int64_t>(g.o) * g.o * g.v > (1LL << 30) ||
-      static_cast<int64_t>(g.v) * g.v * g.v > (1LL << 30))
+      static_cast<int64_t>(g.v) * g.v > (1LL << 30))
     return false;
   g.tiles = static_cast<int>(tiles);
   g.b_rows = static_cast<int64_t>(g.o) * g.o * g.v;
