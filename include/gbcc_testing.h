@@ -147,6 +147,17 @@ int gbcc_testing_tc_launches_total(gbcc_handle* h, int64_t* launches);
  * fails on the host instead of being launched, once (-1: none). */
 int gbcc_testing_fail_site(int64_t site);
 
+/* Lanes of plans made from now on: -1 as the library decides, 0 one, 1 the
+ * program's four.  The results of a residual do not depend on it. */
+int gbcc_testing_lanes_mode(int mode);
+
+/* The free device memory that the decision on lanes is told of from now on, in
+ * bytes (-1: the device's own). */
+int gbcc_testing_free_bytes(int64_t bytes);
+
+/* The lanes of handle h's plan and the bytes of their workspaces. */
+int gbcc_testing_lanes(struct gbcc_handle* h, int* lanes, int64_t* workspace_bytes);
+
 /* Lanes of handle h, beside its stream, that are still running kernels. */
 int gbcc_testing_lanes_busy(struct gbcc_handle* h, int* busy);
 

@@ -566,12 +566,24 @@ void check_pair_symmetric(gbcc_handle* h) {
   finish_pair_check(h);
 }
 
+// What later calls on the handle may allocate: a calibration's residuals, the DIIS
+// vectors and seeds of a solve, (ab|cd) for a refill, and (T)'s operands and sums.
+size_t later_bytes(const gbcc_handle* h) {
+  const size_t n = static_cast<size_t>(n1_of(h) + n2_of(h)) * sizeof(double);
+  size_t need = n;
+  if (!h->x1) need += 2 * static_cast<size_t>(h->cfg.n_diis) * n;
+  if (!h->seed1) need += n;
+  if (h->S.Gabcd && !h->S.Gabcd->d) need += static_cast<size_t>(h->S.Gabcd->size()) * sizeof(double);
+  return need + gbcc::triples_bytes(h->cfg.o, h->cfg.v);
+}
+
 void plan_residual(gbcc_handle* h) {
   drop_graphs(h);
   h->eng->reset_plans();
   h->eng->set_slices(h->slices_used[0], h->slices_used[1], h->slices_used[2]);
   h->eng->set_frozen({h->S.t1, h->S.t2, h->S.tau});
   h->eng->set_emulation(uses_fp64_tc(h));
+  h->eng->set_reserve(later_bytes(h));
   h->eng->begin(gbcc::Mode::kPlan, GBCC_PREC_FP64);
   gbcc::residual_program(*h->eng, h->S);
   h->eng->end();
@@ -687,6 +699,13 @@ void commit_inputs(gbcc_handle* h) {
 }
 
 }  // namespace
+
+extern "C" int gbcc_testing_lanes(gbcc_handle* h, int* lanes, int64_t* workspace_bytes) {
+  if (!h || !lanes || !workspace_bytes) return GBCC_ERR_INVALID_ARG;
+  *lanes = h->eng->lanes();
+  *workspace_bytes = static_cast<int64_t>(h->eng->workspace_bytes());
+  return GBCC_OK;
+}
 
 extern "C" int gbcc_testing_lanes_busy(gbcc_handle* h, int* busy) {
   if (!h || !busy) return GBCC_ERR_INVALID_ARG;
@@ -1248,7 +1267,14 @@ gbcc_status gbcc_triples(gbcc_handle* h, int32_t precision, const double* t1_ai,
     in.Giabc = S.Giabc->d;
     in.eps_o = S.eps_o->d;
     in.eps_v = S.eps_v->d;
-    *e_t = gbcc::triples_energy(in, precision, h->stream, h->d_err);
+    try {
+      *e_t = gbcc::triples_energy(in, precision, h->stream, h->d_err);
+    } catch (const Error& e) {
+      // short of memory: the residual's workspaces hold nothing between calls
+      if (e.status != GBCC_ERR_OOM || !h->eng->release_scratch()) throw;
+      drop_graphs(h);
+      *e_t = gbcc::triples_energy(in, precision, h->stream, h->d_err);
+    }
     sync_check(h);
     return GBCC_OK;
   });

@@ -225,10 +225,10 @@ void residual_program(Engine& E, const CcsdTensors& S) {
   //   1  K, g_ac, tmp
   //   2  the pair ladders (integral-direct: the U intermediate)
   //   3  tmp2, the small products, r1
-  // Mixed residual at o = 13, v = 57: 1.14 -> 0.75 ms; at o = 30, v = 120: 5.17 ->
-  // 4.69; at o = 50, v = 190 (every product fills the chip): 37.3 -> 37.8; FP64
-  // solve at o = 5, v = 19: 5.5 -> 3.65 ms.
-
+  // Mixed residual in one lane and in four: o = 20, v = 76 1.70 and 1.29 ms; o = 30,
+  // v = 120 4.68 and 4.26; o = 50, v = 190 38.2 and 37.4 (untuned); o = 32, v = 320
+  // 44.0 and 42.6; integral-direct o = 16, v = 80 1.86 and 1.30; FP64_TC o = 21,
+  // v = 83 5.47 and 4.35.  The results are the same bits.
   E.lane(2);
   int tmp2_done = -1;
   if (direct) {

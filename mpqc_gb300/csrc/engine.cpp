@@ -73,6 +73,23 @@ void tune_clear() {
 std::atomic<int64_t> g_alloc_count{0};
 std::atomic<int64_t> g_fail_alloc_after{-1};
 
+// test hooks: lanes of plans made from now on (gbcc_testing_lanes_mode: -1 as
+// finalize() decides, 0 one, 1 the program's), and the free bytes that lanes_fit
+// is told of (gbcc_testing_free_bytes, -1: the device's)
+std::atomic<int> g_lanes_mode{-1};
+std::atomic<int64_t> g_free_bytes{-1};
+
+size_t device_bytes_free() {
+  const int64_t told = g_free_bytes.load();
+  if (told >= 0) return static_cast<size_t>(told);
+  size_t free = 0, total = 0;
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return free;
+}
+
 // test hook (gbcc_testing_fail_site): the operation of an EXEC pass that fails
 // instead of being launched, once (-1: none)
 std::atomic<int64_t> g_fail_site{-1};
@@ -378,6 +395,8 @@ Engine::~Engine() {
 // every pointer is cleared before any new allocation: one that fails leaves no
 // pointer to freed memory behind
 void Engine::free_workspaces() {
+  if (scratch_) bytes_ -= workspace_bytes();
+  scratch_ = false;
   for (Lane& w : lane_ws_) {
     for (void** p : {reinterpret_cast<void**>(&w.w64a), reinterpret_cast<void**>(&w.w64b),
                      reinterpret_cast<void**>(&w.wbfa), reinterpret_cast<void**>(&w.wbfb),
@@ -386,6 +405,31 @@ void Engine::free_workspaces() {
       *p = nullptr;
     }
   }
+}
+
+void Engine::alloc_workspaces() {
+  free_workspaces();
+  for (int k = 0; k < nlanes_; ++k) {
+    Lane& w = lane_ws_[k];
+    if (k > 0 && !w.stream) GBCC_CK(cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking));
+    w.w64a = static_cast<double*>(dev_alloc(w.n64a * sizeof(double)));
+    w.w64b = static_cast<double*>(dev_alloc(w.n64b * sizeof(double)));
+    w.wbfa = static_cast<__nv_bfloat16*>(dev_alloc(w.nbfa * sizeof(__nv_bfloat16)));
+    w.wbfb = static_cast<__nv_bfloat16*>(dev_alloc(w.nbfb * sizeof(__nv_bfloat16)));
+    w.wpart = static_cast<double*>(dev_alloc(w.npart * sizeof(double)));
+    w.wcount = static_cast<unsigned*>(dev_alloc(w.ncount * sizeof(unsigned)));
+    GBCC_CK(cudaMemsetAsync(w.wcount, 0, std::max<size_t>(w.ncount, 1) * sizeof(unsigned), stream_));
+  }
+  bytes_ += workspace_bytes();
+  scratch_ = true;
+}
+
+bool Engine::release_scratch() {
+  if (!scratch_ || workspace_bytes() == 0) return false;
+  abandon();
+  GBCC_CK(cudaStreamSynchronize(stream_));
+  free_workspaces();
+  return true;
 }
 
 void Engine::lane(int k) {
@@ -422,6 +466,58 @@ void Engine::abandon() noexcept {
   lane_ = 0;
   run_ = stream_;
   ws_ = &lane_ws_[0];
+}
+
+size_t Engine::lane_bytes(const Lane& w) {
+  return w.ncount * sizeof(unsigned) + (w.n64a + w.n64b + w.npart) * sizeof(double) +
+         (w.nbfa + w.nbfb) * sizeof(__nv_bfloat16);
+}
+
+size_t Engine::workspace_bytes() const {
+  size_t n = 0;
+  for (int k = 0; k < nlanes_; ++k) n += lane_bytes(lane_ws_[k]);
+  return n;
+}
+
+// one workspace that serves every lane's operations in turn
+Engine::Lane Engine::merged_lane() const {
+  Lane m = lane_ws_[0];
+  for (int k = 1; k < nlanes_; ++k) {
+    const Lane& w = lane_ws_[k];
+    m.n64a = std::max(m.n64a, w.n64a);
+    m.n64b = std::max(m.n64b, w.n64b);
+    m.nbfa = std::max(m.nbfa, w.nbfa);
+    m.nbfb = std::max(m.nbfb, w.nbfb);
+    m.npart = std::max(m.npart, w.npart);
+    m.ncount = std::max(m.ncount, w.ncount);
+  }
+  return m;
+}
+
+void Engine::merge_lanes() {
+  lane_ws_[0] = merged_lane();
+  for (int k = 1; k < nlanes_; ++k) {
+    Lane& w = lane_ws_[k];
+    w.n64a = w.n64b = w.nbfa = w.nbfb = w.npart = w.ncount = 0;
+  }
+  nlanes_ = 1;
+  for (auto& sp : sites_) {
+    sp->lane = 0;
+    for (GemmPlan& p : sp->plan)
+      for (OperandPlan& op : p.P) op.lane = 0;
+  }
+}
+
+// Whether the lanes' workspaces beyond one lane's leave room for everything that
+// the handle may still allocate without them: this plan's shared and constant
+// packs, and the owner's reserve.
+bool Engine::lanes_fit() const {
+  size_t need = reserve_ + workspace_bytes();
+  for (const auto& sp : sites_)
+    for (const GemmPlan& p : sp->plan)
+      for (const OperandPlan& op : p.P)
+        if (p.use_tc) need += op.pack_elems * sizeof(__nv_bfloat16);
+  return need <= device_bytes_free();
 }
 
 int Engine::lanes_busy() const {
@@ -1339,20 +1435,9 @@ void Engine::finalize() {
   for (const TableChunk& c : tables_)
     GBCC_CK(cudaMemcpy(c.d, c.host.data(), c.host.size() * sizeof(int64_t), cudaMemcpyHostToDevice));
   tables_.clear();
-  free_workspaces();
-  for (int k = 0; k < nlanes_; ++k) {
-    Lane& w = lane_ws_[k];
-    if (k > 0 && !w.stream) GBCC_CK(cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking));
-    w.w64a = static_cast<double*>(dev_alloc(w.n64a * sizeof(double)));
-    w.w64b = static_cast<double*>(dev_alloc(w.n64b * sizeof(double)));
-    w.wbfa = static_cast<__nv_bfloat16*>(dev_alloc(w.nbfa * sizeof(__nv_bfloat16)));
-    w.wbfb = static_cast<__nv_bfloat16*>(dev_alloc(w.nbfb * sizeof(__nv_bfloat16)));
-    w.wpart = static_cast<double*>(dev_alloc(w.npart * sizeof(double)));
-    w.wcount = static_cast<unsigned*>(dev_alloc(w.ncount * sizeof(unsigned)));
-    GBCC_CK(cudaMemsetAsync(w.wcount, 0, std::max<size_t>(w.ncount, 1) * sizeof(unsigned), stream_));
-    bytes_ += w.ncount * sizeof(unsigned) + (w.n64a + w.n64b + w.npart) * sizeof(double) +
-              (w.nbfa + w.nbfb) * sizeof(__nv_bfloat16);
-  }
+  const int mode = g_lanes_mode.load();
+  if (nlanes_ > 1 && (mode < 0 ? !lanes_fit() : mode == 0)) merge_lanes();
+  alloc_workspaces();
   // packs shared by several contractions of a residual get their own buffer
   for (auto& kv : pack_uses_) {
     if (kv.second.size() < 2) continue;
@@ -1378,6 +1463,7 @@ void Engine::finalize() {
 void Engine::prepack(int precision) {
   const int pi = plan_index(precision);
   if (!planned_) throw Error(GBCC_ERR_STATE, "engine: prepack before PLAN");
+  if (!scratch_) alloc_workspaces();  // given up by release_scratch()
   if (pi == 0 || packed_[pi]) return;
   if (pi == 2 && !emu_) throw Error(GBCC_ERR_STATE, "engine: no FP64_TC plan");
   for (auto& sp : sites_) {
@@ -1400,6 +1486,18 @@ void Engine::prepack(int precision) {
 }
 
 }  // namespace gbcc
+
+extern "C" int gbcc_testing_lanes_mode(int mode) {
+  if (mode < -1 || mode > 1) return GBCC_ERR_INVALID_ARG;
+  gbcc::g_lanes_mode.store(mode);
+  return GBCC_OK;
+}
+
+extern "C" int gbcc_testing_free_bytes(int64_t bytes) {
+  if (bytes < -1) return GBCC_ERR_INVALID_ARG;
+  gbcc::g_free_bytes.store(bytes);
+  return GBCC_OK;
+}
 
 extern "C" int gbcc_testing_fail_site(int64_t site) {
   if (site < -1) return GBCC_ERR_INVALID_ARG;

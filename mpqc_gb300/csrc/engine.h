@@ -211,13 +211,22 @@ class Engine {
   // its own with its own workspaces; lanes start together and EXEC's end waits
   // for all.  mark() is a point after everything enqueued so far in a lane,
   // wait(k, m) makes lane k wait for it; program order must put a mark before
-  // its waits.  With lanes off (set_lanes, or while profiling) everything runs
-  // in program order on the engine's stream.
+  // its waits.  finalize() makes one lane of them where the device is short of
+  // memory (lanes_fit); then, and while profiling, everything runs in program order
+  // on the engine's stream.
   static constexpr int kLanes = 4;
   void lane(int k);
   int mark(int k);
   void wait(int k, int m);
-  void set_lanes(bool on) { lanes_on_ = on; }
+  // bytes that the engine's owner may still allocate beside the plan: lanes leave
+  // them free
+  void set_reserve(size_t bytes) { reserve_ = bytes; }
+  int lanes() const { return nlanes_; }
+  // Gives the workspaces back (false: there are none); prepack() takes them again,
+  // at other addresses, so captured passes are void.
+  bool release_scratch();
+  // bytes of the plan's workspaces, of all lanes
+  size_t workspace_bytes() const;
   // After an EXEC pass that ended in an exception: waits for what its lanes have
   // been given (end() did not join them), so that nothing of it still runs beside
   // what the stream is given next.  Lanes in a capture have nothing running.
@@ -273,10 +282,16 @@ class Engine {
     unsigned* wcount = nullptr;   // finished splits of each tile (gemm_small.cu), zero between launches
   };
   void free_workspaces();
-  bool concurrent() const { return lanes_on_ && nlanes_ > 1 && !profile_; }
+  void alloc_workspaces();
+  bool scratch_ = false;     // the workspaces are allocated
+  static size_t lane_bytes(const Lane& w);
+  Lane merged_lane() const;
+  void merge_lanes();
+  bool lanes_fit() const;
+  bool concurrent() const { return nlanes_ > 1 && !profile_; }
   Lane lane_ws_[kLanes];
   int nlanes_ = 1;           // lanes the plan uses
-  bool lanes_on_ = true;
+  size_t reserve_ = 0;
   int lane_ = 0;             // current lane of the program pass
   cudaStream_t run_ = nullptr;  // stream of the current operation
   Lane* ws_ = lane_ws_;      // workspaces of the current operation
