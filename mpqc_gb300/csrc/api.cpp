@@ -978,12 +978,14 @@ gbcc_status gbcc_residual_ex(gbcc_handle* h, int32_t precision, const double* t1
     if (!t1_ai || !t2_abij || !r1_ai || !r2_abij)
       throw Error(GBCC_ERR_INVALID_ARG, "gbcc_residual: NULL argument");
     h->have_solution = false;
-    copy_in(h->S.t1->d, t1_ai, n1_of(h), h->stream);
     copy_in(h->S.t2->d, t2_abij, n2_of(h), h->stream);
-    // the residual runs behind the check, the results leave only after it
+    // t1 and tau are under way while the check's answer comes back; amplitudes that
+    // it refuses get no residual
     enqueue_pair_check(h);
-    run_residual(h, precision);
+    copy_in(h->S.t1->d, t1_ai, n1_of(h), h->stream);
+    gbcc::launch_make_tau(h->cfg.o, h->cfg.v, h->S.t1->d, h->S.t2->d, h->S.tau->d, h->stream);
     finish_pair_check(h);
+    h->last_launches = 1 + enqueue_residual_program(h, precision);
     copy_out(r1_ai, h->S.r1->d, n1_of(h), h->stream);
     copy_out(r2_abij, h->S.r2->d, n2_of(h), h->stream);
     sync_check(h);
