@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("use_graphs", [0, 2])
 def test_refused_before_the_residual(use_graphs):
     lib = _lib.load()
-    inp = synth.make_inputs(6, 24, 16, seed=2, t1_scale=1e-2)
+    inp = synth.make_inputs(13, 57, 16, seed=2, t1_scale=1e-2)  # packs for the tensor cores
     bad = inp.t2.copy()
     bad[0, 1, 2, 3] += 1.0
     n0, n1 = C.c_int(), C.c_int()
