@@ -110,7 +110,9 @@ int gbcc_testing_diis_coefficients(int32_t n, const double* B, double damping, d
 /* The last pass of r2 (kernels.h, launch_r2_assemble) on host arrays r2u, tmp,
  * g, r2 [v][v][o][o], Bp [v(v+1)/2][o(o+1)/2] and Bm [v(v-1)/2][o(o-1)/2]
  * (either may be NULL), run repeat times from the same r2; *ms (may be NULL):
- * the time of one. */
+ * the time of one.  gbcc_testing_r2_assemble_pair_max: the largest o that runs on
+ * the per-pair kernel with Bp (pairs = 1) and without (0); past it, the tiled one. */
+int gbcc_testing_r2_assemble_pair_max(int pairs);
 int gbcc_testing_r2_assemble(int64_t o, int64_t v, const double* r2u, const double* tmp, const double* g,
                              const double* Bp, const double* Bm, int accumulate, double* r2, int repeat, float* ms);
 

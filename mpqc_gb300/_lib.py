@@ -43,7 +43,7 @@ TESTING_EXPORTS = ("gbcc_testing_gemm", "gbcc_testing_gemm_ex", "gbcc_testing_ge
                    "gbcc_testing_profile_tiles", "gbcc_testing_tc_launches_total", "gbcc_testing_eigh",
                    "gbcc_testing_df_block_rows", "gbcc_testing_reads_in_place",
                    "gbcc_testing_fail_site", "gbcc_testing_lanes_busy", "gbcc_testing_lanes_mode",
-                   "gbcc_testing_free_bytes", "gbcc_testing_lanes")
+                   "gbcc_testing_free_bytes", "gbcc_testing_lanes", "gbcc_testing_r2_assemble_pair_max")
 
 
 class Config(C.Structure):
@@ -164,6 +164,8 @@ def load(path: str | os.PathLike | None = None) -> C.CDLL:
     lib.gbcc_testing_diis_coefficients.argtypes = [C.c_int32, vp, C.c_double, vp, C.POINTER(C.c_int32)]
     lib.gbcc_testing_reads_in_place.restype = C.c_int
     lib.gbcc_testing_reads_in_place.argtypes = [vp, C.c_int64, C.c_int]
+    lib.gbcc_testing_r2_assemble_pair_max.restype = C.c_int
+    lib.gbcc_testing_r2_assemble_pair_max.argtypes = [C.c_int]
     lib.gbcc_testing_lanes_mode.restype = C.c_int
     lib.gbcc_testing_lanes_mode.argtypes = [C.c_int]
     lib.gbcc_testing_free_bytes.restype = C.c_int

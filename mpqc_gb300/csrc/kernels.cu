@@ -1145,17 +1145,26 @@ void launch_pair_unpack(int64_t rows_v, int64_t v, int64_t o, bool ab_pairs, con
     pair_unpack_kernel<true><<<grid_for(rows_v * v, 1), kThreads, 0, st>>>(rows_v, v, o, ab_pairs, Bp, Bm, out);
 }
 
+// A pair's q and, with the ladders' products, its rows of Bp and Bm, in half the
+// shared memory of an SM: two blocks an SM.  That is o <= 69, without the products o <=
+// 85.  Both sides of the line, v = 100: o = 69 0.57 ms, o = 70 (tiled) 0.99; without
+// products o = 85 0.77, o = 86 (tiled) 0.87.
+static int64_t r2_assemble_pair_bytes(int64_t o, bool pairs) { return (2 * o * (o | 1) + (pairs ? o * o : 0)) * 8; }
+
+int64_t r2_assemble_pair_max(bool pairs) {
+  int64_t o = 1;
+  while (r2_assemble_pair_bytes(o + 1, pairs) <= kAssembleSmem) ++o;
+  return o;
+}
+
 void launch_r2_assemble(int64_t o, int64_t v, const double* r2u, const double* tmp, const double* g,
                         const double* Bp, const double* Bm, bool accumulate, double* r2, cudaStream_t st) {
-  // a pair's q, Bp and Bm in half the shared memory of an SM or less (o <= 68): two
-  // blocks an SM.  One side of the line and the other, v = 100: o = 68 0.58 ms,
-  // o = 69 (tiled) 0.57; o = 64 0.47, o = 80 (tiled) 1.11
-  const int64_t bytes = (2 * o * (o | 1) + (Bp ? o * o : 0)) * 8;
   static const bool attr =
       cudaFuncSetAttribute(r2_assemble_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAssembleSmem) ==
           cudaSuccess &&
       cudaFuncSetAttribute(r2_assemble_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAssembleSmem) ==
           cudaSuccess;
+  const int64_t bytes = r2_assemble_pair_bytes(o, Bp != nullptr);
   if (attr && bytes <= kAssembleSmem) {
     const AssembleArgs A{static_cast<int>(o), static_cast<int>(v), r2u, tmp, g, Bp, Bm, r2};
     const int64_t want = (o * o / 4 + 31) / 32 * 32;  // about four elements a thread

@@ -357,7 +357,9 @@ void launch_pair_unpack(int64_t rows_v, int64_t v, int64_t o, bool ab_pairs, con
 
 // r2(a,b,i,j) (+)= q(a,b,i,j) + q(b,a,j,i) + g(a,b,i,j) + unpack(Bp, Bm)(a,b,i,j),
 // q = r2u - 0.5 tmp - tmp(b,a,i,j); Bp null: no unpack, Bm null: no B- part;
-// accumulate: add to r2, else overwrite it
+// accumulate: add to r2, else overwrite it.  r2_assemble_pair_max: the largest o of its
+// per-pair kernel, with the ladders' products or without.
+int64_t r2_assemble_pair_max(bool pairs);
 void launch_r2_assemble(int64_t o, int64_t v, const double* r2u, const double* tmp, const double* g,
                         const double* Bp, const double* Bm, bool accumulate, double* r2, cudaStream_t st);
 

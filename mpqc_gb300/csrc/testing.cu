@@ -286,6 +286,10 @@ extern "C" int gbcc_testing_split(const double* x, int64_t n, int nslices, uint1
   }
 }
 
+extern "C" int gbcc_testing_r2_assemble_pair_max(int pairs) {
+  return static_cast<int>(gbcc::r2_assemble_pair_max(pairs != 0));
+}
+
 extern "C" int gbcc_testing_r2_assemble(int64_t o, int64_t v, const double* r2u, const double* tmp, const double* g,
                                         const double* Bp, const double* Bm, int accumulate, double* r2, int repeat,
                                         float* ms) {
