@@ -260,6 +260,23 @@ def ncu_traffic():
     return None
 
 
+def tc_kernel(p):
+    """The kernel that a profiled split-BF16 contraction ran on, as the tuner chose it."""
+    if p["bn"] == 256 and p["sps"] == 2:
+        return f"gemm_pair_kernel<{2 if p['pairs'] == 3 else 3}>"
+    return f"gemm_tc_kernel<{p['bn']}, 0, {p['sps']}>"
+
+
+def ladder_traffic(p):
+    """(bytes, source) of the ladder launch: the committed capture's where it is of the
+    kernel that ran, else None."""
+    captured = "gemm_tc_kernel<192, 0, 2>"
+    if tc_kernel(p) == captured and (p["M"], p["N"], p["K"]) == (51360, 528, 51360):
+        return ncu_traffic(), (f"dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of this launch on "
+                               f"{captured} (profiles/ladder_gemm_o32_v320.md), not measured in this run")
+    return None, f"not measured: the committed capture is of {captured} at o = 32, v = 320"
+
+
 def ours(args):
     import torch
     ws, rank, local = dist_env()
@@ -363,11 +380,10 @@ def ours(args):
         executed = lp["pairs"] * lp["flops"]
         peak = pk.get("bf16_tflops_sustained") or 1700.0
         ach = executed / (lp["gemm_ms"] * 1e-3) / 1e12
+        traffic, source = ladder_traffic(lp)
         roof = {"bound": "tensor", "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak,
-                "traffic": ncu_traffic(),
-                "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of this launch "
-                                  "(profiles/ladder_gemm_o32_v320.md), not measured in this run",
-                "kernel": "gemm_tc_kernel (particle-particle ladder, G+ tau+ pair products)",
+                "traffic": traffic, "traffic_source": source,
+                "kernel": tc_kernel(lp) + " (particle-particle ladder, G+ tau+ pair products)",
                 "executed_flops_per_launch": executed, "launch_ms": lp["gemm_ms"],
                 "peak_source": "MEASURED_PEAKS.json bf16_tflops_sustained (of measured)"}
     terms = {}
@@ -723,7 +739,8 @@ def gemm_probe(args):
     kernel for --gemm-slices >= 1, plain FP64 for 0); prints one JSON line with
     the kernel time per launch and the executed slice-product TFLOP/s.  The
     launches are what an ncu capture of this command sees
-    (``-k regex:gemm_tc_kernel``)."""
+    (``-k regex:gemm_``: gemm_tc_kernel, with --gemm-sps 2 and bn 256
+    gemm_pair_kernel, FP64-grade gemm_multi_kernel)."""
     import ctypes as C
     from mpqc_gb300 import _lib, build as gb
     gb.build()
@@ -736,7 +753,7 @@ def gemm_probe(args):
     ms = C.c_float()
     sl = args.gemm_slices
     if sl < 0:
-        # FP64-grade: six fixed-point slices, 21 pair products in six class launches
+        # FP64-grade: six fixed-point slices, all 21 pair products in one launch
         st = lib.gbcc_testing_gemm_fp64tc(M, N, K, A.ctypes.data, B.ctypes.data, Cm.ctypes.data, args.gemm_bn,
                                           args.gemm_ksplit, args.gemm_cta2, args.gemm_repeat, C.byref(ms))
     else:
