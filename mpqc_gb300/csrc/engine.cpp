@@ -510,8 +510,10 @@ void Engine::merge_lanes() {
 
 // Whether the lanes' workspaces beyond one lane's leave room for everything that
 // the handle may still allocate without them: this plan's shared and constant
-// packs, and the owner's reserve.
+// packs, and the owner's reserve.  (Up to 32 MB the device is not asked: that takes
+// 0.3 ms, an eighth of a small handle's set-up.)
 bool Engine::lanes_fit() const {
+  if (g_free_bytes.load() < 0 && workspace_bytes() - lane_bytes(merged_lane()) <= size_t{32} << 20) return true;
   size_t need = reserve_ + workspace_bytes();
   for (const auto& sp : sites_)
     for (const GemmPlan& p : sp->plan)
@@ -1262,7 +1264,7 @@ void Engine::contract(const Ix& c, double beta, double alpha, const std::vector<
       p.slices = slices;
       p.emu = emu;
       // the ladder and ring contractions take the faster 192/256-wide tiles
-      // (not FP64_TC: its chunk sums need the float-float fold of tiles up to 128)
+      // (FP64_TC has its own kernel and tile: gemm_multi_bn)
       const bool wide = !emu && (cls == kClassLadder || cls == kClassRing);
       int bns[4];
       int nbn = 1;

@@ -17,8 +17,8 @@
 // their FP32 register sums as in gemm_tc.cu's tiles of 192 and 256; bounded
 // waits and teardown likewise.
 //
-// 9500^3, two slices: 2.88 ms, 1.79 PFLOP/s of slice products (128 x 192 tiles on one CTA:
-// 3.36 ms; 18145 x 1275 x 9000: 0.77 against 0.88 ms).
+// 9500^3, two slices, in bands of 8 tiles: 2.84 ms, 1.81 PFLOP/s of slice products
+// (128 x 192 tiles on one CTA: 3.71 ms; 18145 x 1275 x 9000: 0.765 against 0.934 ms).
 #include <algorithm>
 
 #include "fp_bits.cuh"
@@ -381,7 +381,7 @@ bool launch(const GemmTcArgs& g, cudaStream_t st) {
 bool launch_gemm_pair(const GemmTcArgs& g, cudaStream_t st) {
   // whole panels of two or three slices, every pair p + q below the slice count
   const int sl = g.a_slices;
-  if ((sl != 2 && sl != 3) || g.b_slices != sl || g.npairs != sl * (sl + 1) / 2 || g.a_row0 || g.b_row0 ||
+  if ((sl != 2 && sl != 3) || g.b_slices != sl || g.npairs != sl * (sl + 1) / 2 ||
       g.chunk < 1 || g.skip_stage1)
     return false;
   for (int q = 0; q < g.npairs; ++q)

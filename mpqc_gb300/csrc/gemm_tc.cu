@@ -85,9 +85,10 @@ struct TcCfg {
   static constexpr int kThreads = 32 * (kEpiWarp0 + kEpiWarps);
   // staging tile per epilogue warp: (hi, lo) float pairs with the float-float
   // fold (BN <= 128), single floats at BN = 192 (room for a fifth stage, or two
-  // stages of both slices), doubles at BN = 256.  The BN = 256 kernel spills
-  // and keeps its spills in L1: enlarging its shared memory (a fourth stage)
-  // measured 1.14 -> 0.88 PFLOP/s, so it keeps three stages.
+  // stages of both slices).  BN = 256 stages floats too, in the room of doubles: that
+  // leaves three pipeline stages.  With a fourth, taken from the L1 that holds its
+  // register spills, its earlier epilogue ran at 0.88 instead of 1.14 PFLOP/s; the
+  // present one spills less and was not measured with four.
   static constexpr uint32_t kStgElem = BN == 192 ? 4u : 8u;
   static constexpr uint32_t kStgBytes = kEpiWarps * 32 * kStgLd * kStgElem;
   // as many stages as fit in 227 KB next to the staging tile and barriers (one
@@ -204,9 +205,7 @@ __global__ void __launch_bounds__(TcCfg<BN, CTA2, SPS>::kThreads, 1)
       prefetch_tmap(&tmB);
     }
     __syncwarp();
-    // first panel row of the operands (a window of a larger panel); rows
-    // past the panel's end load as zeros, rows past M or N are not stored
-    const int a_row0 = static_cast<int>(g.a_row0), b_row0 = static_cast<int>(g.b_row0);
+    // rows past a panel's end load as zeros, rows past M or N are not stored
     const uint32_t sA0 = smem_u32(sA), sB0 = smem_u32(sB);
     uint32_t gi = 0;  // stage-use counter across tiles
     bool ok = true;
@@ -230,23 +229,23 @@ __global__ void __launch_bounds__(TcCfg<BN, CTA2, SPS>::kThreads, 1)
           // the leader's full barrier counts the bytes of both CTAs
           const uint32_t bar = full0 + static_cast<uint32_t>(s) * 8u;
           if (leader) mbar_expect_tx(lead, &full[s], 2 * Cfg::kStageBytes);
-          tma_load_3d_pair(lead, &tmA, bar, dA, 0, m0 + a_row0, g.pa[pr] * kblocks + kb);
-          tma_load_3d_pair(lead, &tmB, bar, dB, 0, nb0 + b_row0, g.pb[pr] * kblocks + kb);
+          tma_load_3d_pair(lead, &tmA, bar, dA, 0, m0, g.pa[pr] * kblocks + kb);
+          tma_load_3d_pair(lead, &tmB, bar, dB, 0, nb0, g.pb[pr] * kblocks + kb);
         } else if constexpr (SPS == 1) {
           // test hook (gbcc_testing_gemm_timeout): leave one stage unloaded,
           // so that its consumer's bounded wait runs out
           if (g.skip_stage1 == 0 || static_cast<int64_t>(gi) + 1 != g.skip_stage1) {
             mbar_expect_tx(lead, &full[s], Cfg::kStageBytes);
-            tma_load_3d(lead, &tmA, &full[s], dA, 0, m0 + a_row0, g.pa[pr] * kblocks + kb);
-            tma_load_3d(lead, &tmB, &full[s], dB, 0, nb0 + b_row0, g.pb[pr] * kblocks + kb);
+            tma_load_3d(lead, &tmA, &full[s], dA, 0, m0, g.pa[pr] * kblocks + kb);
+            tma_load_3d(lead, &tmB, &full[s], dB, 0, nb0, g.pb[pr] * kblocks + kb);
           }
         } else {
           // every slice of A and B of this k-block
           mbar_expect_tx(lead, &full[s], Cfg::kStageBytes);
 #pragma unroll
           for (int j = 0; j < SPS; ++j) {
-            tma_load_3d(lead, &tmA, &full[s], dA + j * Cfg::kABytes, 0, m0 + a_row0, j * kblocks + kb);
-            tma_load_3d(lead, &tmB, &full[s], dB + j * Cfg::kBBytes, 0, nb0 + b_row0, j * kblocks + kb);
+            tma_load_3d(lead, &tmA, &full[s], dA + j * Cfg::kABytes, 0, m0, j * kblocks + kb);
+            tma_load_3d(lead, &tmB, &full[s], dB + j * Cfg::kBBytes, 0, nb0, j * kblocks + kb);
           }
         }
         if (SPS > 1 || ++pr == g.npairs) {
@@ -723,8 +722,6 @@ bool launch_gemm_tc(const GemmTcArgs& g, cudaStream_t st) {
     return false;
   if (g.Mpad > (1LL << 31) - 1 || g.Npad > (1LL << 31) - 1 || g.Kpad > (1LL << 31) - 1) return false;
   if ((g.a_rows && g.a_rows < g.Mpad) || (g.b_rows && g.b_rows < g.Npad)) return false;
-  if (g.a_row0 < 0 || g.b_row0 < 0 || g.a_row0 + g.Mpad > (1LL << 31) - 1 || g.b_row0 + g.Npad > (1LL << 31) - 1)
-    return false;
   if ((g.Npad / g.bn) * (g.Mpad / BM) * (g.ksplit > 1 ? g.ksplit : 1) > (1LL << 31) - 1) return false;
   if (g.ksplit > 1 && (!g.partial || g.kb_per_split < 1 ||
                        static_cast<int64_t>(g.ksplit - 1) * g.kb_per_split >= g.Kpad / BK))

@@ -96,24 +96,10 @@ struct GatherArgs {
 // I_p 2^(E - 8(p+1)) exactly in BF16 (at most 8 significant bits).  Every
 // product of slices p of A and q of B with p + q = w is then an integer
 // multiple of 2^(E_A + E_B - 8(w + 2)) of magnitude at most 2^14 of it, so
-// FP32 sums of up to 2^10 of them stay within 2^24 units and are exact: one
-// TMEM chunk (8 (k-block, pair) steps, 512 products) and the FP32 register
-// sum of two chunks before each float-float fold.
+// FP32 sums of up to 2^10 of them stay within 2^24 units and are exact: the
+// length of a TMEM accumulation (gemm_multi.cu).
 constexpr int kFixedBits = 8;
 constexpr int kFixedSlices = 6;   // 47 bits below the row's leading power of two
-constexpr int kFixedChunk = 8;    // (k-block, pair) steps per TMEM accumulation: 512 products
-constexpr int kFixedFold = 2;     // chunks summed in FP32 registers before the float-float fold
-// The pairs (p, w - p), both below n, of weight class w; returns their number.
-inline int fixed_class_pairs(int n, int w, int* pa, int* pb) {
-  int k = 0;
-  for (int p = 0; p < n; ++p)
-    if (w - p >= 0 && w - p < n) {
-      pa[k] = p;
-      pb[k] = w - p;
-      ++k;
-    }
-  return k;
-}
 
 inline void gather_set_c4(GatherTerm& T, const int64_t* hca, int64_t n) {
   bool ok = reinterpret_cast<uintptr_t>(T.a) % 16 == 0;
@@ -240,9 +226,6 @@ struct GemmTcArgs {
   // (CTAs working at the same time then share fewer, wider operand panels in
   // L2); 0 or 1: N fastest over whole rows of tiles
   int group;
-  // first row of A / B within their panels (a window of a larger panel:
-  // rows past the panel's end load as zeros; 0 for whole panels)
-  int64_t a_row0, b_row0;
   // test hooks: the pipeline barriers' wait limit in ns (0: 2 s), and 1 +
   // the stage (counted over a CTA's stage uses; one pair per stage) whose
   // loads the producer leaves out (0: none -- the value-initialised default)
@@ -474,9 +457,9 @@ struct SolveParams {
 };
 // zero the state for a solve (mixed: start in the mixed phase)
 void launch_solve_init(SolveState* s, int mixed, cudaStream_t st);
-// one thread: E, error, convergence test, phase switch, DIIS bookkeeping,
-// and the conditions of the loop, the update and the residual precision
-// the energy terms, then the iteration's decision in the same launch
+// the energy terms, then in the same launch, on one thread: E, error, convergence
+// test, phase switch, DIIS bookkeeping, and the conditions of the loop, the update
+// and the residual precision
 void launch_energy_decide(const EnergyTermsArgs& e, const SolveParams& p, cudaStream_t st);
 // nanosecond timestamp (globaltimer) of the current iteration's residual:
 // base[2 (iter - 1) + which]

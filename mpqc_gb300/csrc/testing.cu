@@ -478,6 +478,27 @@ extern "C" int gbcc_testing_fixed_split(const double* x, int64_t rows, int64_t c
   return status;
 }
 
+namespace {
+
+// FP64-grade products class by class on gemm_tc_kernel, for comparison (the library
+// runs gemm_multi_kernel): (k-block, pair) steps per TMEM accumulation, 512
+// products, and accumulations summed in FP32 registers before a float-float fold
+constexpr int kFixedChunk = 8;
+constexpr int kFixedFold = 2;
+// the pairs (p, w - p), both below n, of weight class w; returns their number
+int fixed_class_pairs(int n, int w, int* pa, int* pb) {
+  int k = 0;
+  for (int p = 0; p < n; ++p)
+    if (w - p >= 0 && w - p < n) {
+      pa[k] = p;
+      pb[k] = w - p;
+      ++k;
+    }
+  return k;
+}
+
+}  // namespace
+
 extern "C" int gbcc_testing_gemm_fp64tc(int64_t M, int64_t N, int64_t K, const double* A, const double* B,
                                         double* Cout, int bn_req, int ksplit, int cta2, int repeat, float* ms) {
   using namespace gbcc;

@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("bn", [32, 64])
-@pytest.mark.parametrize("M,N,K,ksplit", [(5, 70, 16161, 1), (130, 66, 65536, 1), (1, 1, 32000, 1),
+@pytest.mark.parametrize("M,N,K,ksplit", [(300, 200, 2000, 1), (64, 300, 4096, 4), (5, 70, 16161, 1), (130, 66, 65536, 1), (1, 1, 32000, 1),
                                           (129, 65, 32001, 1), (33, 31, 262144, 1), (8, 40, 400000, 3)])
 def test_long_sums_of_one_sign_are_exact(gbcc_lib, M, N, K, ksplit, bn):
     # 17- and 15-bit integers: sums of at most 400000 products stay below 2^51
