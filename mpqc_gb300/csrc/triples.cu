@@ -21,7 +21,7 @@
 // columns a.  Each pair is one product over 2 K (gemm_multi.cu), written once
 // to its own array, in its own order; the energy kernel adds the three as it
 // reads them.  (Six read-modify-write passes of W through scattered offsets, one
-// per term and pair i, j, took 112 ms at o = 20, v = 76; this takes 17 ms.)  A
+// per term and pair i, j, took 113 ms at o = 20, v = 76; this takes 17.5 ms.)  A
 // batch is as many triplets as keep the three arrays in about 96 MB, most of
 // L2.  The energy kernel takes 8 x 8 x 8 blocks of a <= b <= c: all six
 // orderings of a set {a, b, c} are read once and give all six permuted W
@@ -552,7 +552,7 @@ __device__ __forceinline__ int tile_at(int x, int y) { return x * kB + (x ^ y); 
 // pair, all asynchronous, run under the terms of this one.  Every cube of
 // ordering m is read at F[m], the same six offsets for all three arrays and all
 // pairs.  Nine triplets at v = 76: 58 -> 44 us against blocks of one pair each with
-// one stage ((T) at o = 20, v = 76: 20.4 -> 17.1 ms).
+// one stage ((T) at o = 20, v = 76: 20.4 -> 17.1 ms, before the sums above).
 template <typename R>
 __global__ void __launch_bounds__(kEnergyThreads, 1) triples_blocks_kernel(EnergyArgs g) {
   extern __shared__ double smem_d[];
