@@ -316,9 +316,13 @@ std::pair<double, double> energy_error(gbcc_handle* h, gbcc::EnergyTermsArgs e) 
 void ensure_diis(gbcc_handle* h) {
   const int nd = h->cfg.n_diis;
   if (h->ndiis_alloc == nd) return;
-  for (void* p : {(void*)h->x1, (void*)h->x2, (void*)h->e1, (void*)h->e2, (void*)h->Bmat,
-                  (void*)h->coef, (void*)h->d_nskip})
+  // every pointer is cleared before the first allocation: one that fails leaves
+  // none to freed memory behind
+  auto drop = [](auto*& p) {
     gbcc::dev_free(p);
+    p = nullptr;
+  };
+  drop(h->x1), drop(h->x2), drop(h->e1), drop(h->e2), drop(h->Bmat), drop(h->coef), drop(h->d_nskip);
   const size_t n1 = static_cast<size_t>(n1_of(h)), n2 = static_cast<size_t>(n2_of(h));
   h->x1 = static_cast<double*>(gbcc::dev_alloc(nd * n1 * sizeof(double)));
   h->e1 = static_cast<double*>(gbcc::dev_alloc(nd * n1 * sizeof(double)));
