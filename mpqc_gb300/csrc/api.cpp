@@ -113,6 +113,21 @@ gbcc_status guarded(gbcc_handle* h, F&& f) {
   }
 }
 
+void drop_graphs(gbcc_handle* h);
+
+// fn, and where it runs out of device memory, fn again without the residual's
+// workspaces, which hold nothing between calls (the next residual takes them again).
+template <class F>
+void with_scratch(gbcc_handle* h, F&& fn) {
+  try {
+    fn();
+  } catch (const Error& e) {
+    if (e.status != GBCC_ERR_OOM || !h->eng->release_scratch()) throw;
+    drop_graphs(h);
+    fn();
+  }
+}
+
 // The handle's tensors, on the first input call.  An allocation failure part
 // way leaves them incomplete: the handle then refuses every call but
 // gbcc_destroy (GBCC_ERR_STATE).
@@ -232,6 +247,18 @@ int hi_prec(const gbcc_handle* h) {
 // whether the handle's plan includes the FP64_TC contractions
 bool uses_fp64_tc(const gbcc_handle* h) { return hi_prec(h) == GBCC_PREC_FP64_TC; }
 
+// The constant packs (and workspaces) of a precision.  Where those of a precision
+// that the handle's plan left no room for run out of memory, its lanes make room.
+void prepack(gbcc_handle* h, int precision) {
+  try {
+    h->eng->prepack(precision);
+  } catch (const Error& e) {
+    if (e.status != GBCC_ERR_OOM || !h->eng->one_lane()) throw;
+    drop_graphs(h);
+    h->eng->prepack(precision);
+  }
+}
+
 // One EXEC pass of the residual program; if it fails midway, nothing of it is
 // still running when the exception leaves.
 void exec_residual(gbcc_handle* h, int precision) {
@@ -250,7 +277,7 @@ void exec_residual(gbcc_handle* h, int precision) {
 // fixed pointers, sizes and tensor maps once the plan is finalised); later
 // evaluations replay it.  Returns the number of kernels it enqueued.
 int enqueue_residual_program(gbcc_handle* h, int precision) {
-  h->eng->prepack(precision);  // once per plan; no workspace changes
+  prepack(h, precision);  // once per plan
   auto direct = [&]() {
     exec_residual(h, precision);
     return h->eng->kernel_launches();
@@ -336,7 +363,7 @@ void ensure_diis(gbcc_handle* h) {
 
 // The residual program of one precision as a (not instantiated) graph.
 cudaGraph_t capture_residual_graph(gbcc_handle* h, int precision) {
-  h->eng->prepack(precision);
+  prepack(h, precision);
   cudaGraph_t g = nullptr;
   GBCC_CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   try {
@@ -570,15 +597,12 @@ void check_pair_symmetric(gbcc_handle* h) {
   finish_pair_check(h);
 }
 
-// What later calls on the handle may allocate: a calibration's residuals, the DIIS
-// vectors and seeds of a solve, (ab|cd) for a refill, and (T)'s operands and sums.
+// What later calls on the handle allocate beside the residual's workspaces: a
+// calibration's residuals, the DIIS vectors and the seeds of a solve.  (A refill's
+// (ab|cd) and (T) can have the workspaces: with_scratch.)
 size_t later_bytes(const gbcc_handle* h) {
   const size_t n = static_cast<size_t>(n1_of(h) + n2_of(h)) * sizeof(double);
-  size_t need = n;
-  if (!h->x1) need += 2 * static_cast<size_t>(h->cfg.n_diis) * n;
-  if (!h->seed1) need += n;
-  if (h->S.Gabcd && !h->S.Gabcd->d) need += static_cast<size_t>(h->S.Gabcd->size()) * sizeof(double);
-  return need + gbcc::triples_bytes(h->cfg.o, h->cfg.v);
+  return n + (h->x1 ? 0 : 2 * static_cast<size_t>(h->cfg.n_diis) * n) + (h->seed1 ? 0 : n);
 }
 
 void plan_residual(gbcc_handle* h) {
@@ -587,6 +611,7 @@ void plan_residual(gbcc_handle* h) {
   h->eng->set_slices(h->slices_used[0], h->slices_used[1], h->slices_used[2]);
   h->eng->set_frozen({h->S.t1, h->S.t2, h->S.tau});
   h->eng->set_emulation(uses_fp64_tc(h));
+  h->eng->set_mixed(h->cfg.precision == GBCC_PREC_MIXED);
   h->eng->set_reserve(later_bytes(h));
   h->eng->begin(gbcc::Mode::kPlan, GBCC_PREC_FP64);
   gbcc::residual_program(*h->eng, h->S);
@@ -854,7 +879,7 @@ gbcc_status gbcc_set_inputs(gbcc_handle* h, const gbcc_inputs* in) {
     copy_in(S.Giajb->d, in->Giajb, o * v * o * v, h->stream);
     copy_in(S.Gijka->d, in->Gijka, o * o * o * v, h->stream);
     copy_in(S.Giabc->d, in->Giabc, o * v * v * v, h->stream);
-    h->eng->acquire(*S.Gabcd);
+    with_scratch(h, [&] { h->eng->acquire(*S.Gabcd); });
     copy_in(S.Gabcd->d, in->Gabcd, v * v * v * v, h->stream);
     commit_inputs(h);
     return GBCC_OK;
@@ -941,7 +966,7 @@ gbcc_status gbcc_device_inputs(gbcc_handle* h, gbcc_inputs* out) {
     if (h->S.naux > 0 || h->S.nao > 0)
       throw Error(GBCC_ERR_STATE, "gbcc_device_inputs: the handle holds density-fitted or integral-direct inputs");
     gbcc::CcsdTensors& S = h->S;
-    h->eng->acquire(*S.Gabcd);  // given back by the previous commit
+    with_scratch(h, [&] { h->eng->acquire(*S.Gabcd); });  // given back by the previous commit
     GBCC_CK(cudaStreamSynchronize(h->stream));  // zero-initialisation done
     out->eps_o = S.eps_o->d;
     out->eps_v = S.eps_v->d;
@@ -1273,14 +1298,7 @@ gbcc_status gbcc_triples(gbcc_handle* h, int32_t precision, const double* t1_ai,
     in.Giabc = S.Giabc->d;
     in.eps_o = S.eps_o->d;
     in.eps_v = S.eps_v->d;
-    try {
-      *e_t = gbcc::triples_energy(in, precision, h->stream, h->d_err);
-    } catch (const Error& e) {
-      // short of memory: the residual's workspaces hold nothing between calls
-      if (e.status != GBCC_ERR_OOM || !h->eng->release_scratch()) throw;
-      drop_graphs(h);
-      *e_t = gbcc::triples_energy(in, precision, h->stream, h->d_err);
-    }
+    with_scratch(h, [&] { *e_t = gbcc::triples_energy(in, precision, h->stream, h->d_err); });
     sync_check(h);
     return GBCC_OK;
   });

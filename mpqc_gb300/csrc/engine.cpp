@@ -424,6 +424,13 @@ void Engine::alloc_workspaces() {
   scratch_ = true;
 }
 
+bool Engine::one_lane() {
+  if (nlanes_ <= 1) return false;
+  release_scratch();
+  merge_lanes();
+  return true;
+}
+
 bool Engine::release_scratch() {
   if (!scratch_ || workspace_bytes() == 0) return false;
   abandon();
@@ -508,17 +515,19 @@ void Engine::merge_lanes() {
   }
 }
 
-// Whether the lanes' workspaces beyond one lane's leave room for everything that
-// the handle may still allocate without them: this plan's shared and constant
-// packs, and the owner's reserve.  (Up to 32 MB the device is not asked: that takes
+// Whether the lanes' workspaces beyond one lane's leave room for what the handle may
+// still allocate beside them: this plan's shared and constant packs in the precisions
+// it runs, and the owner's reserve.  (Up to 32 MB the device is not asked: that takes
 // 0.3 ms, an eighth of a small handle's set-up.)
 bool Engine::lanes_fit() const {
   if (g_free_bytes.load() < 0 && workspace_bytes() - lane_bytes(merged_lane()) <= size_t{32} << 20) return true;
   size_t need = reserve_ + workspace_bytes();
   for (const auto& sp : sites_)
-    for (const GemmPlan& p : sp->plan)
-      for (const OperandPlan& op : p.P)
-        if (p.use_tc) need += op.pack_elems * sizeof(__nv_bfloat16);
+    for (int pm = mixed_ ? 1 : 2; pm < 3; ++pm)
+      for (const OperandPlan& op : sp->plan[pm].P)
+        if (sp->plan[pm].use_tc && op.constant) need += op.pack_elems * sizeof(__nv_bfloat16);
+  for (const auto& kv : pack_uses_)
+    if (kv.second.size() > 1) need += kv.second.front()->pack_elems * sizeof(__nv_bfloat16);
   return need <= device_bytes_free();
 }
 

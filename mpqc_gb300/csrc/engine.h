@@ -218,9 +218,14 @@ class Engine {
   void lane(int k);
   int mark(int k);
   void wait(int k, int m);
-  // bytes that the engine's owner may still allocate beside the plan: lanes leave
-  // them free
+  // bytes that the engine's owner may still allocate beside the plan and its
+  // workspaces: lanes leave them free
   void set_reserve(size_t bytes) { reserve_ = bytes; }
+  // whether the mixed plan is run, and its packs are to be left room for
+  void set_mixed(bool on) { mixed_ = on; }
+  // makes one lane of a plan's lanes between passes (false: there is one); prepack()
+  // takes its workspace, and captured passes are void
+  bool one_lane();
   int lanes() const { return nlanes_; }
   // Gives the workspaces back (false: there are none); prepack() takes them again,
   // at other addresses, so captured passes are void.
@@ -309,6 +314,7 @@ class Engine {
   int chunk_lo_ = 24;
   bool profile_ = false;
   bool emu_ = false;
+  bool mixed_ = false;
   bool trial_ = false;
   bool packed_[3] = {false, false, false};
   std::unordered_set<const Tensor*> frozen_;

@@ -845,15 +845,6 @@ double triples_tc(const TriplesInputs& in, int precision, cudaStream_t st, int* 
 
 }  // namespace
 
-size_t triples_bytes(int64_t o, int64_t v) {
-  const size_t rows = static_cast<size_t>(2 * o * v * v + 2 * o * o * v), v3 = static_cast<size_t>(v) * v * v;
-  const size_t K = static_cast<size_t>(v + o + 63) / 64 * 64;
-  // six slices of the panels (FP64: 8 bytes, and 40 of offsets a row), the sums
-  const size_t panels = rows * (12 * K + 40);
-  const size_t sums = std::max(3 * v3 * 8, std::min<size_t>(static_cast<size_t>(o) * v3 * 8, size_t{8} << 30));
-  return panels + sums + static_cast<size_t>(o) * o * v * v * 8 + (size_t{64} << 20);
-}
-
 double triples_energy(const TriplesInputs& in, int precision, cudaStream_t st, int* err) {
   if (precision != GBCC_PREC_FP64) return triples_tc(in, precision, st, err);
   Triples t(in, st);

@@ -26,7 +26,4 @@ struct TriplesInputs {
 // Synchronises the stream; throws gbcc::Error.
 double triples_energy(const TriplesInputs& in, int precision, cudaStream_t st, int* err);
 
-// The most device memory that takes, in any precision (an upper bound).
-size_t triples_bytes(int64_t o, int64_t v);
-
 }  // namespace gbcc

@@ -107,3 +107,31 @@ def test_triples_take_the_workspaces_when_memory_is_short(hooks):
             assert ex.value.status == GBCC_ERR_OOM
             got = s.residual(t1, t2)
             assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
+
+
+def test_refill_takes_the_workspaces_when_memory_is_short(hooks):
+    inp = synth.make_inputs(5, 19, 20, seed=4, t1_scale=1e-2)
+    with Solver(5, 19, precision="mixed", slices=(2, 2, 2), autotune=False) as s:
+        s.set_inputs(inp.eps_o, inp.eps_v, **ints_dict(inp))
+        ref = s.residual(inp.t1, inp.t2)
+        assert hooks.gbcc_testing_fail_alloc(0, None) == 0  # (ab|cd), the refill's first allocation
+        s.set_inputs(inp.eps_o, inp.eps_v, **ints_dict(inp))
+        got = s.residual(inp.t1, inp.t2)
+    assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
+
+
+def test_packs_of_another_precision_take_the_lanes_when_memory_is_short(hooks):
+    s, t1, t2 = make("standard", 13, 57, precision="fp64", use_graphs=1)
+    with s:
+        ref64 = s.residual(t1, t2)
+        ref = s.residual(t1, t2, precision="mixed")
+        assert lanes_of(s)[0] == 4
+    s, t1, t2 = make("standard", 13, 57, precision="fp64", use_graphs=1)
+    with s:
+        s.residual(t1, t2)
+        assert hooks.gbcc_testing_fail_alloc(1, None) == 0  # the second pack of the mixed plan
+        got = s.residual(t1, t2, precision="mixed")
+        assert lanes_of(s)[0] == 1
+        assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
+        got = s.residual(t1, t2)
+        assert np.array_equal(got[0], ref64[0]) and np.array_equal(got[1], ref64[1])
